@@ -103,7 +103,8 @@ typedef struct {
     double origin[3]; /* coordinates of point (0,0,0) */
     int dims[3];      /* nx, ny, nz */
     int64_t fluid_count; /* output */
-    int64_t ray_tests;   /* output: ray-triangle tests performed */
+    int64_t ray_tests;   /* output: (point, candidate triangle) tests decided: a column's points share
+                          * most of them */
 } lbm_vox_desc;
 
 /* tri12: ntri rows of x1 y1 z1 x2 y2 z2 x3 y3 z3 nx ny nz (the STL's own facet

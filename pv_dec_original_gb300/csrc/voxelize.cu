@@ -11,17 +11,26 @@
 //   parity -> Fluid        ComplexGeometry.cpp:1041-1048
 //
 // GB300 design: the reference tests every point against every triangle
-// (O(N*T)).  Here each lattice column gets a candidate list of the triangles
-// whose xy extent, widened by a per-triangle margin, contains the column's
-// ray; a triangle outside that widened extent provably fails the
-// point-in-triangle test for every point of the column (the margin is ~1e8
-// times the worst-case rounding of that test), so dropping it changes no
-// count.  Triangles that can never pass (zero area, or a computed normal
-// with |n_z| < 1e-16, which the reference rejects outright) are dropped;
-// ill-conditioned ones go to a global list tested by every point.
-// Threads run (column, k) with k fastest, so the 32 lanes of a warp walk the
-// same candidate list in lock step and its triangles are broadcast loads.
-#include <vector>
+// (O(N*T)).  Here a triangle meets only the lattice columns its xy extent,
+// widened by a per-triangle margin, contains: a triangle outside that
+// widened extent provably fails the point-in-triangle test for every point
+// of the column (the margin is ~1e8 times the worst-case rounding of that
+// test), so dropping it changes no count.  Triangles that can never pass
+// (zero area, or a computed normal with |n_z| < 1e-16, which the reference
+// rejects outright) are dropped; ill-conditioned ones go to a global list
+// tested by every point.
+// All points of a column share the ray's x and y, so a (column, triangle)
+// pair is decided once for the whole column: whether the line lies inside
+// the triangle does not depend on k but for rounding, and the crossing
+// counts for the k below the height where the line meets the facet plane.
+// Both decisions carry a bound of ~300 times the worst rounding of the
+// reference's tests; what lies within it (a line through an edge or a
+// vertex, a point on the facet) is left to the reference's own FP64 test of
+// that (point, triangle).  The pair flips the parity of a range of k: two
+// bits of a difference bit field, whose running XOR along k is the mask.
+// (70,040 triangles on a 56 x 54 x 509 lattice: 0.06 ms on the device,
+// where one FP64 test per point and candidate took 12.3 ms at GB300's two
+// FP64 multiply-adds a cycle and SM.)
 #include <cmath>
 #include <algorithm>
 
@@ -126,84 +135,302 @@ __device__ double cull_margin(const double* T, double zspan) {
     return m;
 }
 
-struct TriBox {
-    double x0, x1, y0, y1;
+// What every kernel of a call needs.
+struct VoxParams {
+    double bb[6];
+    double org[3];
+    double s;
+    double zspan;     // of cull_margin
+    double span;      // bound of every coordinate difference of the tests
+    double dz;        // ray length of an unadjusted ray
+    double zabs;      // bound of |pz|, |ez|
+    int nx, ny, nz;
+    int kadj[2];      // the k whose ray ends are moved off the bounding box (-1: none)
+    int exact_only;   // rays the column decisions do not describe: every pair is tested point by point
+    int64_t ncol;
+    int64_t ntri;
+    int64_t cap;      // entries of the pair list
 };
 
-__global__ void tri_prep(const double* __restrict__ tri, int64_t ntri, double zspan, TriBox* __restrict__ box,
-                         uint8_t* __restrict__ status) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntri) return;
-    const double* T = tri + 12 * t;
-    double m = cull_margin(T, zspan);
-    TriBox b;
-    b.x0 = fmin(fmin(T[0], T[3]), T[6]) - m;
-    b.x1 = fmax(fmax(T[0], T[3]), T[6]) + m;
-    b.y0 = fmin(fmin(T[1], T[4]), T[7]) - m;
-    b.y1 = fmax(fmax(T[1], T[4]), T[7]) + m;
-    box[t] = b;
-    status[t] = m < 0.0 ? 0 : (m > 1e29 ? 2 : 1);
+// Counters of one call.
+struct VoxCounters {
+    unsigned long long fluid, pairs;
+    unsigned long long npair;  // pairs left to k_exact_pairs (may exceed the list)
+    unsigned long long nglob, nwide;
+};
+
+__device__ __forceinline__ double column_x(const VoxParams& P, int i) {
+    double x = P.org[0] + i * P.s;
+    if (x == P.bb[0]) x += 0.02;
+    if (x == P.bb[1]) x -= 0.02;
+    return x;
+}
+__device__ __forceinline__ double column_y(const VoxParams& P, int j) {
+    double y = P.org[1] + j * P.s;
+    if (y == P.bb[2]) y += 0.02;
+    if (y == P.bb[3]) y -= 0.02;
+    return y;
 }
 
-// pass 0: count per column; pass 1: fill lists.
-template <int PASS>
-__global__ void tri_bin(int64_t ntri, const TriBox* __restrict__ box, const uint8_t* __restrict__ status,
-                        const double* __restrict__ colx, const double* __restrict__ coly, int nx, int ny,
-                        double ox, double oy, double s, int64_t* __restrict__ count, int32_t* __restrict__ list) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntri || status[t] != 1) return;
-    TriBox b = box[t];
-    // clamp in FP64 before converting: margins can be far outside int range
-    const double fi0 = fmax(floor((b.x0 - ox) / s) - 1.0, 0.0), fi1 = fmin(ceil((b.x1 - ox) / s) + 1.0, nx - 1.0);
-    const double fj0 = fmax(floor((b.y0 - oy) / s) - 1.0, 0.0), fj1 = fmin(ceil((b.y1 - oy) / s) + 1.0, ny - 1.0);
-    if (!(fi0 <= fi1) || !(fj0 <= fj1)) return;
-    const int i0 = (int)fi0, i1 = (int)fi1, j0 = (int)fj0, j1 = (int)fj1;
-    for (int j = j0; j <= j1; ++j) {
-        double yy = coly[j];
-        if (yy < b.y0 || yy > b.y1) continue;
-        for (int i = i0; i <= i1; ++i) {
-            double xx = colx[i];
-            if (xx < b.x0 || xx > b.x1) continue;
-            int64_t c = (int64_t)j * nx + i;
-            if (PASS == 0) {
-                atomicAdd(reinterpret_cast<unsigned long long*>(count + c), 1ull);
-            } else {
-                unsigned long long slot = atomicAdd(reinterpret_cast<unsigned long long*>(count + c), 1ull);
-                list[slot] = (int32_t)t;
+// Difference bit field [k / 32][column]: point (c, k) is fluid when the XOR
+// of bits 0 .. k of its column is 1.
+__device__ __forceinline__ void flip(uint32_t* __restrict__ bits, const VoxParams& P, int64_t c, int k) {
+    if (k < P.nz) atomicXor(bits + (int64_t)(k >> 5) * P.ncol + c, 1u << (k & 31));
+}
+__device__ __forceinline__ void flip_range(uint32_t* __restrict__ bits, const VoxParams& P, int64_t c, int k0, int k1) {
+    flip(bits, P, c, k0);
+    flip(bits, P, c, k1 + 1);
+}
+
+__device__ __forceinline__ bool exact_hit(const VoxParams& P, const double* T, int i, int j, int k) {
+    return ray_hits(point_ray(P.bb, P.org, P.s, i, j, k), T) != 0;
+}
+
+// One triangle's FP64 constants for the column decisions, besides its 12 numbers.
+struct TriConst {
+    double nX, nY, nZ, inv_nZ;          // computed normal
+    double uX, uY, uZ, vX, vY, vZ;      // edges
+    double uu, uv, vv, inv_D;
+    double E;                           // bound of the barycentric coordinates' rounding; < 0: decide nothing
+    double inv_fz;                      // 1 / facet normal z
+};
+
+__device__ __forceinline__ TriConst tri_const(const VoxParams& P, const double* T) {
+    TriConst c;
+    c.uX = T[3] - T[0]; c.uY = T[4] - T[1]; c.uZ = T[5] - T[2];
+    c.vX = T[6] - T[0]; c.vY = T[7] - T[1]; c.vZ = T[8] - T[2];
+    c.nX = c.uY * c.vZ - c.uZ * c.vY;
+    c.nY = c.uZ * c.vX - c.uX * c.vZ;
+    c.nZ = c.uX * c.vY - c.uY * c.vX;
+    c.inv_nZ = 1.0 / c.nZ;
+    c.uu = c.uX * c.uX + c.uY * c.uY + c.uZ * c.uZ;
+    c.uv = c.uX * c.vX + c.uY * c.vY + c.uZ * c.vZ;
+    c.vv = c.vX * c.vX + c.vY * c.vY + c.vZ * c.vZ;
+    c.inv_D = 1.0 / (c.uv * c.uv - c.uu * c.vv);
+    const double n2 = c.nX * c.nX + c.nY * c.nY + c.nZ * c.nZ;
+    const double L2 = fmax(c.uu, c.vv);  // squared edge scale (the third edge is at most twice as long)
+    // The barycentric coordinates' rounding: an error eps * span in w moves
+    // the point on the computed plane by eps span L^2 / |nZ| along z, and
+    // that by a factor L / |n| in the coordinates; with shape = L^2 / |n|
+    // that is eps shape^2 (|n| / |nZ|) (span / L), times a small count of
+    // operations (< 30); 1e-12 is 9000 eps.
+    const double L = sqrt(L2);
+    c.E = 4e-12 * (L2 * L2 / n2) * (sqrt(n2) * fabs(c.inv_nZ)) * (1.0 + P.span / L);
+    c.inv_fz = 1.0 / T[11];
+    const double den = fabs(P.dz * T[11]);  // the reference rejects |den| < 1e-16
+    if (!(c.E < 1e-2) || !(den > 2e-16) || !isfinite(c.inv_fz) || P.exact_only) c.E = -1.0;
+    return c;
+}
+
+// Column (i, j) against triangle T: flips the column's parity where the ray
+// of point k crosses T.  A pair that no bound decides goes to the pair list,
+// tested point by point by k_exact_pairs.
+__device__ __forceinline__ void column_pair(const VoxParams& P, const TriConst& t, const double* T, int32_t tri,
+                                            int i, int j, double px, double py, uint32_t* __restrict__ bits,
+                                            int2* __restrict__ list, VoxCounters* __restrict__ cnt) {
+    const int64_t c = (int64_t)j * P.nx + i;
+    bool undecided = t.E < 0.0;
+    if (!undecided) {
+        const double wX = px - T[0], wY = py - T[1];
+        const double wZ = -(t.nX * wX + t.nY * wY) * t.inv_nZ;
+        const double wu = wX * t.uX + wY * t.uY + wZ * t.uZ;
+        const double wv = wX * t.vX + wY * t.vY + wZ * t.vZ;
+        const double sb = (t.uv * wv - t.vv * wu) * t.inv_D;
+        const double tb = (t.uv * wu - t.uu * wv) * t.inv_D;
+        if (sb < -t.E || tb < -t.E || sb + tb > 1.0 + t.E) return;  // outside for every k
+        undecided = !(sb > t.E && tb > t.E && sb + tb < 1.0 - t.E);
+    }
+    if (!undecided) {
+        // 0 <= t <= 1 of the ray parameter: z* - dz <= pz(k) <= z*
+        const double ax = (T[0] - px) * T[9], ay = (T[1] - py) * T[10];
+        const double zs = T[2] + (ax + ay) * t.inv_fz;
+        const double inv_s = 1.0 / P.s;
+        const double p0 = P.org[2] + 0.5 * P.s;
+        const double kU = (zs - p0) * inv_s, kL = (zs - P.dz - p0) * inv_s;
+        const double tol = (1e-12 * ((fabs(ax) + fabs(ay)) * fabs(t.inv_fz) + fabs(T[2]) + P.zabs)) * inv_s +
+                           1e-12 * (fabs(kU) + fabs(kL) + P.nz);
+        if (tol < 0.25) {
+            // clamped: beyond the lattice only the side matters
+            const double hiU = fmin(fmax(kU, -4.0), P.nz + 4.0), hiL = fmin(fmax(kL, -4.0), P.nz + 4.0);
+            const int aU = (int)ceil(hiU - tol), aL = (int)floor(hiL + tol);
+            const bool ambU = (double)aU <= hiU + tol, ambL = (double)aL >= hiL - tol;
+            const int k0 = max(aL + 1, 0), k1 = min(aU - 1, P.nz - 1);
+            if (k0 <= k1) flip_range(bits, P, c, k0, k1);
+            // the k on a bound and the k whose ray is moved: the reference's own test
+            const int special[4] = {ambU ? aU : -1, ambL ? aL : -1, P.kadj[0], P.kadj[1]};
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const int k = special[m];
+                if (k < 0 || k >= P.nz) continue;
+                bool seen = false;
+                for (int n = 0; n < m; ++n) seen |= special[n] == k;
+                if (seen) continue;
+                if (exact_hit(P, T, i, j, k) != (k >= k0 && k <= k1)) flip_range(bits, P, c, k, k);
             }
+            return;
+        }
+    }
+    const unsigned long long slot = atomicAdd(&cnt->npair, 1ull);
+    if (slot < (unsigned long long)P.cap) list[slot] = make_int2(tri, (int)c);  // else: a second run with room for all
+}
+
+// A triangle's columns: the lattice range of its widened xy extent.
+struct TriExtent {
+    double x0, x1, y0, y1;
+    int i0, i1, j0, j1;
+    int kind;  // 0: never counts, 1: columns i0..i1, j0..j1, 2: global list
+};
+
+__device__ __forceinline__ TriExtent tri_extent(const VoxParams& P, const double* T) {
+    TriExtent e{};
+    e.i1 = e.j1 = -1;
+    const double m = cull_margin(T, P.zspan);
+    e.kind = m < 0.0 ? 0 : (m > 1e29 ? 2 : 1);
+    if (e.kind != 1) return e;
+    e.x0 = fmin(fmin(T[0], T[3]), T[6]) - m;
+    e.x1 = fmax(fmax(T[0], T[3]), T[6]) + m;
+    e.y0 = fmin(fmin(T[1], T[4]), T[7]) - m;
+    e.y1 = fmax(fmax(T[1], T[4]), T[7]) + m;
+    // clamp in FP64 before converting: margins can be far outside int range
+    const double fi0 = fmax(floor((e.x0 - P.org[0]) / P.s) - 1.0, 0.0);
+    const double fi1 = fmin(ceil((e.x1 - P.org[0]) / P.s) + 1.0, P.nx - 1.0);
+    const double fj0 = fmax(floor((e.y0 - P.org[1]) / P.s) - 1.0, 0.0);
+    const double fj1 = fmin(ceil((e.y1 - P.org[1]) / P.s) + 1.0, P.ny - 1.0);
+    if (fi0 <= fi1 && fj0 <= fj1) {
+        e.i0 = (int)fi0; e.i1 = (int)fi1; e.j0 = (int)fj0; e.j1 = (int)fj1;
+    }
+    return e;
+}
+
+__device__ __forceinline__ void add_pairs(unsigned pairs, VoxCounters* __restrict__ cnt) {
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&cnt->pairs, (unsigned long long)pairs);
+}
+
+// One thread a triangle: classification and, for extents of up to
+// kWideColumns columns (a mesh about as fine as the lattice), its columns;
+// wider ones go to the wide list.
+constexpr int kWideColumns = 32;
+__global__ void __launch_bounds__(128) k_tri_columns(const VoxParams P, const double* __restrict__ tri,
+                                                     uint32_t* __restrict__ bits, int2* __restrict__ list,
+                                                     int32_t* __restrict__ glob, int32_t* __restrict__ wide,
+                                                     VoxCounters* __restrict__ cnt) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned pairs = 0;
+    if (t < P.ntri) {
+        const double* T = tri + 12 * t;
+        const TriExtent e = tri_extent(P, T);
+        const int64_t n = (int64_t)(e.i1 - e.i0 + 1) * (e.j1 - e.j0 + 1);
+        if (e.kind == 2) {
+            glob[atomicAdd(&cnt->nglob, 1ull)] = (int32_t)t;
+        } else if (n > kWideColumns) {
+            wide[atomicAdd(&cnt->nwide, 1ull)] = (int32_t)t;
+        } else if (n > 0) {
+            TriConst k;
+            bool have = false;
+            for (int j = e.j0; j <= e.j1; ++j) {
+                const double yy = column_y(P, j);
+                if (yy < e.y0 || yy > e.y1) continue;
+                for (int i = e.i0; i <= e.i1; ++i) {
+                    const double xx = column_x(P, i);
+                    if (xx < e.x0 || xx > e.x1) continue;
+                    if (!have) { k = tri_const(P, T); have = true; }
+                    ++pairs;
+                    column_pair(P, k, T, (int32_t)t, i, j, xx, yy, bits, list, cnt);
+                }
+            }
+        }
+    }
+    add_pairs(pairs, cnt);
+}
+
+// The wide list: one thread a column, a grid row a triangle (one thread
+// walked the 576 columns of a cap's facet in 1 ms, one after another).
+__global__ void __launch_bounds__(128) k_wide_columns(const VoxParams P, const double* __restrict__ tri,
+                                                      uint32_t* __restrict__ bits, int2* __restrict__ list,
+                                                      const int32_t* __restrict__ wide,
+                                                      VoxCounters* __restrict__ cnt) {
+    const unsigned long long nwide = cnt->nwide;
+    unsigned pairs = 0;
+    for (unsigned long long w = blockIdx.y; w < nwide; w += gridDim.y) {
+        const int32_t t = wide[w];
+        const double* T = tri + 12 * (int64_t)t;
+        const TriExtent e = tri_extent(P, T);
+        const int nc = e.i1 - e.i0 + 1;
+        const int64_t n = (int64_t)nc * (e.j1 - e.j0 + 1);
+        int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+        if (c >= n) continue;
+        const TriConst k = tri_const(P, T);
+        for (; c < n; c += (int64_t)gridDim.x * blockDim.x) {
+            const int i = e.i0 + (int)(c % nc), j = e.j0 + (int)(c / nc);
+            const double xx = column_x(P, i), yy = column_y(P, j);
+            if (xx < e.x0 || xx > e.x1 || yy < e.y0 || yy > e.y1) continue;
+            ++pairs;
+            column_pair(P, k, T, t, i, j, xx, yy, bits, list, cnt);
+        }
+    }
+    add_pairs(pairs, cnt);
+}
+
+// The pairs no bound decided: one warp a pair, the reference's test for
+// every k (32 consecutive k a pass: their results are one word of the field).
+__global__ void __launch_bounds__(128) k_exact_pairs(const VoxParams P, const double* __restrict__ tri,
+                                                     uint32_t* __restrict__ bits, const int2* __restrict__ list,
+                                                     const VoxCounters* __restrict__ cnt) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long n = min(cnt->npair, (unsigned long long)P.cap);
+    const int nw = (P.nz + 31) / 32;
+    const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
+    for (unsigned long long e = (unsigned long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; e < n * nw;
+         e += warps) {
+        const int2 p = list[e / nw];
+        const int kw = (int)(e % nw), k = kw * 32 + lane;
+        const double* T = tri + 12 * (int64_t)p.x;
+        const bool hit = k < P.nz && exact_hit(P, T, p.y % P.nx, p.y / P.nx, k);
+        const uint32_t h = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0 && h) {
+            uint32_t* w = bits + (int64_t)kw * P.ncol + p.y;
+            const uint32_t d = h ^ (h << 1);
+            if (d) atomicXor(w, d);
+            if ((h >> 31) && kw + 1 < nw) atomicXor(w + P.ncol, 1u);
         }
     }
 }
 
-struct RayParams {
-    double bb[6];
-    double org[3];
-    double s;
-    int nx, ny, nz;
-    int kchunks;
-};
-
-__global__ void __launch_bounds__(128) ray_count(RayParams P, const double* __restrict__ tri,
-                                                 const int64_t* __restrict__ off, const int32_t* __restrict__ list,
-                                                 const int32_t* __restrict__ glob, int64_t nglob,
-                                                 uint8_t* __restrict__ mask, unsigned long long* __restrict__ fluid) {
-    const int64_t c = blockIdx.x / P.kchunks;
-    const int k = (int)(blockIdx.x % P.kchunks) * blockDim.x + threadIdx.x;
-    const int i = (int)(c % P.nx), j = (int)(c / P.nx);
-    int count = 0;
-    const bool live = k < P.nz;
-    if (live) {
-        Ray r = point_ray(P.bb, P.org, P.s, i, j, k);
-        const int64_t b = off[c], e = off[c + 1];
-        for (int64_t q = b; q < e; ++q) count += ray_hits(r, tri + 12 * (int64_t)__ldg(list + q));
-        for (int64_t q = 0; q < nglob; ++q) count += ray_hits(r, tri + 12 * (int64_t)__ldg(glob + q));
-        uint8_t v = (count % 2 == 1) ? 1 : 0;
-        mask[((int64_t)k * P.ny + j) * P.nx + i] = v;
-        count = v;
+// The field's running XOR into the mask: thread (column, word of 32 k), the
+// parity below the word from the population counts of the words below it;
+// the triangles of the global list are tested here point by point.
+__global__ void __launch_bounds__(128) k_mask(const VoxParams P, const double* __restrict__ tri,
+                                              const uint32_t* __restrict__ bits, const int32_t* __restrict__ glob,
+                                              uint8_t* __restrict__ mask, VoxCounters* __restrict__ cnt) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned fluid = 0;
+    uint32_t below = 0;  // XOR of the words below kw
+    int w = 0;
+    for (int kw = blockIdx.y; c < P.ncol && kw < (P.nz + 31) / 32; kw += gridDim.y) {
+        for (; w < kw; ++w) below ^= bits[(int64_t)w * P.ncol + c];
+        uint32_t v = bits[(int64_t)kw * P.ncol + c];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) v ^= v << d;
+        if (__popc(below) & 1) v = ~v;
+        const int kn = min(32, P.nz - kw * 32);
+        const unsigned long long ng = cnt->nglob;
+        if (ng) {
+            const int i = (int)(c % P.nx), j = (int)(c / P.nx);
+            for (int b = 0; b < kn; ++b) {
+                const Ray r = point_ray(P.bb, P.org, P.s, i, j, kw * 32 + b);
+                uint32_t h = 0;
+                for (unsigned long long q = 0; q < ng; ++q) h ^= (uint32_t)ray_hits(r, tri + 12 * (int64_t)glob[q]);
+                v ^= h << b;
+            }
+        }
+        if (kn < 32) v &= (1u << kn) - 1u;
+        fluid += __popc(v);
+        uint8_t* m = mask + (int64_t)kw * 32 * P.ncol + c;
+        for (int b = 0; b < kn; ++b) m[b * P.ncol] = (uint8_t)((v >> b) & 1u);
     }
-    // block total of fluid points
-    unsigned v = __reduce_add_sync(0xffffffffu, (unsigned)count);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(fluid, (unsigned long long)v);
+    fluid = __reduce_add_sync(0xffffffffu, fluid);
+    if ((threadIdx.x & 31) == 0 && fluid) atomicAdd(&cnt->fluid, (unsigned long long)fluid);
 }
 
 #define VOX_CHECK(call)                                                        \
@@ -220,91 +447,84 @@ __global__ void __launch_bounds__(128) ray_count(RayParams P, const double* __re
 cudaError_t voxelize_device(const double* d_tri, int64_t ntri, const double bbox[6], const double origin[3],
                             double spacing, const int dims[3], uint8_t* d_mask, VoxResult* res, cudaStream_t st,
                             std::string* err) {
-    const int nx = dims[0], ny = dims[1], nz = dims[2];
-    const int64_t ncol = (int64_t)nx * ny;
-    // column ray coordinates, exactly as point_ray computes them
-    std::vector<double> colx(nx), coly(ny);
-    for (int i = 0; i < nx; ++i) colx[i] = point_ray(bbox, origin, spacing, i, 0, 0).px;
-    for (int j = 0; j < ny; ++j) coly[j] = point_ray(bbox, origin, spacing, 0, j, 0).py;
-    const double zspan = (bbox[5] - bbox[4]) + 1.0 + spacing;
-
-    TriBox* d_box = nullptr;
-    uint8_t* d_status = nullptr;
-    double *d_colx = nullptr, *d_coly = nullptr;
-    int64_t *d_cnt = nullptr, *d_off = nullptr;
-    int32_t *d_list = nullptr, *d_glob = nullptr;
-    unsigned long long* d_fluid = nullptr;
-    const int64_t tri_alloc = ntri > 0 ? ntri : 1;
-    VOX_CHECK(cudaMallocAsync(&d_box, sizeof(TriBox) * tri_alloc, st));
-    VOX_CHECK(cudaMallocAsync(&d_status, tri_alloc, st));
-    VOX_CHECK(cudaMallocAsync(&d_colx, sizeof(double) * nx, st));
-    VOX_CHECK(cudaMallocAsync(&d_coly, sizeof(double) * ny, st));
-    VOX_CHECK(cudaMallocAsync(&d_cnt, sizeof(int64_t) * (ncol + 1), st));
-    VOX_CHECK(cudaMallocAsync(&d_off, sizeof(int64_t) * (ncol + 1), st));
-    VOX_CHECK(cudaMallocAsync(&d_fluid, sizeof(unsigned long long), st));
-    VOX_CHECK(cudaMemcpyAsync(d_colx, colx.data(), sizeof(double) * nx, cudaMemcpyHostToDevice, st));
-    VOX_CHECK(cudaMemcpyAsync(d_coly, coly.data(), sizeof(double) * ny, cudaMemcpyHostToDevice, st));
-    VOX_CHECK(cudaMemsetAsync(d_cnt, 0, sizeof(int64_t) * (ncol + 1), st));
-    VOX_CHECK(cudaMemsetAsync(d_fluid, 0, sizeof(unsigned long long), st));
-
-    const unsigned tb = 256, tg = (unsigned)ceil_div(tri_alloc, tb);
-    if (ntri > 0) tri_prep<<<tg, tb, 0, st>>>(d_tri, ntri, zspan, d_box, d_status);
-    VOX_CHECK(cudaGetLastError());
-
-    // global list (ill-conditioned triangles) assembled on the host
-    std::vector<uint8_t> status(ntri);
-    if (ntri > 0) VOX_CHECK(cudaMemcpyAsync(status.data(), d_status, ntri, cudaMemcpyDeviceToHost, st));
-    VOX_CHECK(cudaStreamSynchronize(st));
-    std::vector<int32_t> glob;
-    for (int64_t t = 0; t < ntri; ++t)
-        if (status[t] == 2) glob.push_back((int32_t)t);
-    VOX_CHECK(cudaMallocAsync(&d_glob, sizeof(int32_t) * (glob.size() + 1), st));
-    if (!glob.empty())
-        VOX_CHECK(cudaMemcpyAsync(d_glob, glob.data(), sizeof(int32_t) * glob.size(), cudaMemcpyHostToDevice, st));
-
-    if (ntri > 0)
-        tri_bin<0><<<tg, tb, 0, st>>>(ntri, d_box, d_status, d_colx, d_coly, nx, ny, origin[0], origin[1], spacing,
-                                      d_cnt, nullptr);
-    VOX_CHECK(cudaGetLastError());
-    int64_t total = 0;
-    VOX_CHECK(exclusive_scan_i64(d_cnt, d_off, ncol + 1, &total, st));
-    VOX_CHECK(cudaMallocAsync(&d_list, sizeof(int32_t) * (total + 1), st));
-    VOX_CHECK(cudaMemcpyAsync(d_cnt, d_off, sizeof(int64_t) * (ncol + 1), cudaMemcpyDeviceToDevice, st));
-    if (ntri > 0)
-        tri_bin<1><<<tg, tb, 0, st>>>(ntri, d_box, d_status, d_colx, d_coly, nx, ny, origin[0], origin[1], spacing,
-                                      d_cnt, d_list);
-    VOX_CHECK(cudaGetLastError());
-
-    RayParams P;
+    VoxParams P{};
     for (int q = 0; q < 6; ++q) P.bb[q] = bbox[q];
     for (int q = 0; q < 3; ++q) P.org[q] = origin[q];
     P.s = spacing;
-    P.nx = nx; P.ny = ny; P.nz = nz;
-    P.kchunks = (int)ceil_div(nz, 128);
-    const int64_t nblocks = ncol * P.kchunks;
-    if (nblocks > 0x7fffffffLL) {
+    P.nx = dims[0]; P.ny = dims[1]; P.nz = dims[2];
+    P.ncol = (int64_t)P.nx * P.ny;
+    P.ntri = ntri;
+    if (P.ncol > 0x7fffffffLL || ntri > 0x7fffffffLL) {
         if (err) *err = "lattice too large for the voxelizer grid";
         return cudaErrorInvalidValue;
     }
-    if (nblocks > 0)
-        ray_count<<<(unsigned)nblocks, 128, 0, st>>>(P, d_tri, d_off, d_list, d_glob, (int64_t)glob.size(), d_mask,
-                                                     d_fluid);
-    VOX_CHECK(cudaGetLastError());
-    unsigned long long fluid = 0;
-    VOX_CHECK(cudaMemcpyAsync(&fluid, d_fluid, sizeof(fluid), cudaMemcpyDeviceToHost, st));
-    VOX_CHECK(cudaStreamSynchronize(st));
-    res->fluid = (int64_t)fluid;
-    res->tests = (total + (int64_t)glob.size() * ncol) * nz;
-    cudaFreeAsync(d_box, st);
-    cudaFreeAsync(d_status, st);
-    cudaFreeAsync(d_colx, st);
-    cudaFreeAsync(d_coly, st);
-    cudaFreeAsync(d_cnt, st);
-    cudaFreeAsync(d_off, st);
-    cudaFreeAsync(d_list, st);
-    cudaFreeAsync(d_glob, st);
-    cudaFreeAsync(d_fluid, st);
-    return cudaStreamSynchronize(st);
+    P.zspan = (bbox[5] - bbox[4]) + 1.0 + spacing;
+    // bounds of the coordinates a test meets
+    double far = 0.0;
+    for (int q = 0; q < 6; ++q) far = std::fmax(far, std::fabs(bbox[q]));
+    for (int q = 0; q < 3; ++q)
+        far = std::fmax(far, std::fmax(std::fabs(origin[q]), std::fabs(origin[q] + dims[q] * spacing)));
+    P.dz = (bbox[5] - bbox[4]) + 0.1 - 0.5 * spacing;
+    P.zabs = far + std::fabs(bbox[5] - bbox[4]) + spacing + 1.0;
+    P.span = 4.0 * P.zabs;
+    // the k whose ray start or end lies on the bounding box (point_ray moves
+    // it): at most one each on an ordinary lattice
+    P.kadj[0] = P.kadj[1] = -1;
+    P.exact_only = !(P.dz > 1e-6 * P.zabs) || !std::isfinite(P.span);
+    double last = -INFINITY;
+    int nstart = 0, nend = 0;
+    for (int k = 0; k < P.nz; ++k) {
+        const double z = origin[2] + k * spacing;
+        const double pz = z + spacing / 2, ez = z + (bbox[5] - bbox[4]) + 0.1;
+        if (pz == bbox[4]) { P.kadj[0] = k; ++nstart; }
+        if (ez == bbox[5]) { P.kadj[1] = k; ++nend; }
+        if (!(pz > last)) P.exact_only = 1;
+        last = pz;
+    }
+    if (nstart > 1 || nend > 1) P.exact_only = 1;
+
+    const int nw = (int)ceil_div(P.nz, 32);
+    const int64_t tri_alloc = ntri > 0 ? ntri : 1;
+    VoxCounters got{};
+    // one run of the kernels with room for `cap` undecided pairs, scratch in
+    // one allocation: counters, bit field, pair, global and wide lists
+    auto run = [&](int64_t cap) -> cudaError_t {
+        P.cap = cap;
+        const size_t b_cnt = 256, b_bits = sizeof(uint32_t) * (size_t)nw * P.ncol;
+        const size_t o_list = (b_cnt + b_bits + 255) / 256 * 256;
+        const size_t o_glob = (o_list + sizeof(int2) * (size_t)cap + 255) / 256 * 256;
+        unsigned char* base = nullptr;
+        VOX_CHECK(cudaMallocAsync(&base, o_glob + 2 * sizeof(int32_t) * (size_t)tri_alloc, st));
+        VoxCounters* cnt = reinterpret_cast<VoxCounters*>(base);
+        uint32_t* bits = reinterpret_cast<uint32_t*>(base + b_cnt);
+        int2* list = reinterpret_cast<int2*>(base + o_list);
+        int32_t* glob = reinterpret_cast<int32_t*>(base + o_glob);
+        int32_t* wide = glob + tri_alloc;
+        auto body = [&]() -> cudaError_t {
+            VOX_CHECK(cudaMemsetAsync(base, 0, b_cnt + b_bits, st));
+            if (ntri > 0) {
+                k_tri_columns<<<(unsigned)ceil_div(ntri, 128), 128, 0, st>>>(P, d_tri, bits, list, glob, wide, cnt);
+                k_wide_columns<<<dim3(16, 152), 128, 0, st>>>(P, d_tri, bits, list, wide, cnt);
+                k_exact_pairs<<<608, 128, 0, st>>>(P, d_tri, bits, list, cnt);
+                VOX_CHECK(cudaGetLastError());
+            }
+            k_mask<<<dim3((unsigned)ceil_div(P.ncol, 128), (unsigned)std::min(nw, 4096)), 128, 0, st>>>(P, d_tri, bits, glob, d_mask,
+                                                                                        cnt);
+            VOX_CHECK(cudaGetLastError());
+            VOX_CHECK(cudaMemcpyAsync(&got, cnt, sizeof(got), cudaMemcpyDeviceToHost, st));
+            VOX_CHECK(cudaStreamSynchronize(st));
+            return cudaSuccess;
+        };
+        const cudaError_t e = body();
+        cudaFreeAsync(base, st);
+        return e;
+    };
+    cudaError_t e = run(std::max<int64_t>(4 * tri_alloc, 65536));
+    if (e == cudaSuccess && got.npair > (unsigned long long)P.cap) e = run((int64_t)got.npair);
+    if (e != cudaSuccess) return e;
+    res->fluid = (int64_t)got.fluid;
+    res->tests = (int64_t)(got.pairs + got.nglob * (unsigned long long)P.ncol) * P.nz;
+    return cudaSuccess;
 }
 
 }  // namespace lbm
