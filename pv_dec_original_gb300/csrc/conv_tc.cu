@@ -342,175 +342,206 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
 
 // ---------------------------------------------------------------------------
 // Weight gradient dW[o][t][c] += sum over output voxels m of
-// dY[m][o] X[src(m, t)][c] (stride 1 or 2) on tcgen05.  GEMM rows are the
-// 27 ci (tap, input channel) pairs R = t ci + c in tiles of 128 (M), the
-// columns the co output channels (N), and K = 16 output voxels of one x-row
-// an MMA (Wo % 16 == 0).  Per 16-voxel slice the CTA stages, with cp.async,
-// the im2col rows of its tiles -- for every (tap, 8-channel group) the 16
-// voxels' source values, zero where the tap falls outside the grid -- and
-// dY of the 16 voxels, both MN-major: a core matrix is 8 voxels x 8
-// channels, 128 contiguous bytes; the next 8 rows (channels) lie 256 bytes
-// on, the next 8 voxels 128.  Two stages: the copies of slice k + 1 overlap
-// the MMAs of slice k (an mbarrier per stage, every wait bounded).  The
-// tiles of a CTA accumulate in tensor memory over its share of the slices
-// (CTAs along y take different tiles); the epilogue adds them to dW with
-// FP32 atomics.
-constexpr int kTileBytes = 128 * 32;  // one 128-row x 16-voxel BF16 tile
+// dY[m][o] X[src(m, t)][c] (kernel size 3, stride 1 or 2, or kernel size 1).
+// A contraction over the voxels with few rows and columns (co x ci of 16 to
+// 64) for each of 27 taps.  On tcgen05 it needs either an im2col operand --
+// 27 copies of X through shared memory, which is what bounded the kernel
+// before this one (864 16-byte cp.async per 16 voxels: 1.46 ms on the
+// 16-channel layer at 256 x 128 x 128) -- or shifted views of one staged
+// tile as 128 matrix rows a constant stride apart, of which 30% are
+// products that count, in more accumulators than tensor memory has columns.
+// Warp-level MMAs take any 8 voxel rows as an operand, so all taps read one
+// staged tile: per 16 voxels one ldmatrix of dY and one per tap of X, the
+// sums in registers.
+//
+// A CTA walks output tiles of TZ x TY x TX voxels, NS of them in flight:
+// per tile a tensor copy of dY (COB channels) and of the input voxels its
+// taps read (16 channels), zero-filled outside the grids (the padding, and
+// ragged tiles, add nothing), swizzled so that the 8 rows of an ldmatrix
+// phase lie in different banks at stride 1 for any tap.  Warps are NG tap
+// groups (TPW taps each) x KG groups of voxel rows; D = dY^T X with
+// m16n8k16 (M = 16 output channels, N = 8 input channels, K = 16 voxels of
+// an x-run).  Bound by shared memory: an ldmatrix.x4 (4 cycles) per two MMAs
+// of 2 cycles at 16 channels, per four at 32.  256 x 128 x 128: 16 -> 16
+// 162 us (1122 before), 32 -> 16 316 us (2493), stride-2 16 -> 32 63 us
+// (153), 1x1x1 61 us (411); 128 x 64 x 64, 32 -> 32: 92 us (327).
+// grid.y walks the (co / COB) x (ci / 16) channel blocks.  Every
+// FLUSH tiles the KG groups add their sums in turn to the CTA's in shared
+// memory: an MMA drops bits of its accumulator, so that chains of 216 MMAs
+// left dW 2.4e-6 from the kernel before, further off FP64 than it (7e-7);
+// with chains of 64 it is not.
+// Each CTA adds its block to dW with FP32 atomics.
+template <int KS_, int S_, int COB_>
+struct WGeo {
+    static constexpr int KS = KS_, S = S_, COB = COB_;
+    static constexpr int TAPS = KS * KS * KS;
+    // tile and warps: the input tile (with its halo) of NS stages fills the
+    // shared memory; 9 taps a warp at COB 16 (72 sums a thread), 3 at COB 32
+    static constexpr int TZ = S == 2 ? 2 : 4, TY = S == 2 ? 4 : 8, TX = (S == 1 && COB == 16) ? 32 : 16;
+    static constexpr int XD = S * (TZ - 1) + KS, XH = S * (TY - 1) + KS, XW = S * (TX - 1) + KS;
+    static constexpr int TPW = KS == 1 ? 1 : (COB == 16 ? 9 : 3);
+    static constexpr int NG = TAPS / TPW;
+    static constexpr int KG = KS == 1 ? 12 : (COB == 16 ? 4 : 2);
+    static constexpr int THREADS = 32 * NG * KG;
+    static constexpr int KSTEPS = TZ * TY * TX / 16;
+    static constexpr int XBYTES = XD * XH * XW * 32, YBYTES = TZ * TY * TX * COB * 2;
+    static constexpr int XPAD = (XBYTES + 1023) / 1024 * 1024, STAGE = XPAD + (YBYTES + 1023) / 1024 * 1024;
+    // tiles between flushes of a thread's sums: chains of at most 64 MMAs
+    static constexpr int FLUSH = 64 * KG / KSTEPS > 1 ? 64 * KG / KSTEPS : 1;
+    // sums [o][tap][16], rows 8 floats apart modulo the 32 banks
+    static constexpr int ROW = TAPS * 16 % 32 == 16 ? TAPS * 16 + 8 : TAPS * 16 + 24;
+    static constexpr int SUMS = COB * ROW * 4;
+    static constexpr int NS = 3 * STAGE + SUMS <= 220 * 1024 ? 3 : 2;
+    static constexpr int SMEM = NS * STAGE + SUMS + 1024;  // stages from a 1024-byte boundary
+    static_assert(SMEM <= 227 * 1024, "shared memory");
+};
 
-__host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n) {
-    return idesc_bf16(m, n) | (1u << 15) | (1u << 16);  // A and B MN-major
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
 }
 
-template <int CO>
-__global__ void __launch_bounds__(kThreads) k_conv3_wgrad_tc(const bf16* __restrict__ x, const bf16* __restrict__ dy,
-                                                             float* __restrict__ dw, int Di, int Hi, int Wi, int Do,
-                                                             int Ho, int Wo, int ci, int S, int tpg, int ncols,
-                                                             int slices_per_cta, int nslices) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int RT = (27 * ci + 127) / 128;
-    const int tile0 = blockIdx.y * tpg;
-    const int ntiles = min(tpg, RT - tile0);
-    const int stage_bytes = tpg * kTileBytes + CO * 32;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * stage_bytes);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
+__device__ __forceinline__ void mma_m16n8k16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Byte offset of 16-byte chunk k of voxel v in a staged tile of 16 / 32
+// channels: the tensor copy's 32- / 64-byte swizzle.
+__device__ __forceinline__ uint32_t chunk16(uint32_t v, uint32_t k) { return (v << 5) | ((k << 4) ^ ((v & 4u) << 2)); }
+__device__ __forceinline__ uint32_t chunk32(uint32_t v, uint32_t k) { return (v << 6) | ((k << 4) ^ ((v & 6u) << 3)); }
+
+template <class G>
+__global__ void __launch_bounds__(G::THREADS, 1) k_conv_wgrad_tiles(const __grid_constant__ CUtensorMap xmap,
+                                                                   const __grid_constant__ CUtensorMap ymap,
+                                                                   float* __restrict__ dw, int Do, int Ho, int Wo,
+                                                                   int ci, int ntiles) {
+    constexpr int S = G::S, KS = G::KS, COB = G::COB, NS = G::NS, MT = COB / 16;
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t full[NS];
+    unsigned char* smem = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
+    const uint32_t base = saddr(smem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int s_begin = blockIdx.x * slices_per_cta;
-    const int s_end = min(nslices, s_begin + slices_per_cta);
+    const int tg = warp % G::NG, kg = warp / G::NG;
+    const int cb = ci / 16, c0 = (blockIdx.y % cb) * 16, o0 = (blockIdx.y / cb) * COB;
+    const int nbx = (Wo + G::TX - 1) / G::TX, nby = (Ho + G::TY - 1) / G::TY;
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tslot)),
-                     "r"(ncols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        mbar_init(saddr(bar), 1);
-        mbar_init(saddr(bar + 1), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tslot;
-    const uint32_t smem_a = saddr(smem);
-    const int xs = Wo / 16;  // slices per output row
-
-    // one slice's copies into stage b
-    auto stage = [&](int sl, int b) {
-        const uint32_t a_base = smem_a + b * stage_bytes, b_base = a_base + tpg * kTileBytes;
-        const int row = sl / xs, ox0 = (sl - row * xs) * 16;
-        const int oy = row % Ho, oz = row / Ho;
-        const int64_t m0 = ((int64_t)oz * Ho + oy) * Wo + ox0;
-        for (int i = tid; i < (CO / 8) * 16; i += kThreads) {
-            const int og = i >> 4, v = i & 15;
-            cp_async16(b_base + og * 256 + v * 16, dy + (m0 + v) * CO + og * 8, true);
-        }
-        for (int i = tid; i < ntiles * 256; i += kThreads) {
-            const int lg = i >> 4, v = i & 15;
-            const int R = (tile0 * 16 + lg) * 8;  // first row of this 8-row group
-            const int t = R / ci, cg = (R - t * ci) >> 3;
-            const int tz = t / 9, ty = (t / 3) % 3, tx = t % 3;
-            const int ix = S * (ox0 + v) + tx - 1, iy = S * oy + ty - 1, iz = S * oz + tz - 1;
-            const bool in = t < 27 && ix >= 0 && iy >= 0 && iz >= 0 && ix < Wi && iy < Hi && iz < Di;
-            const bf16* src = in ? x + (((int64_t)iz * Hi + iy) * Wi + ix) * ci + cg * 8 : x;
-            cp_async16(a_base + lg * 256 + v * 16, src, in);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    auto issue = [&](int tile, int s) {
+        const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
+        const uint32_t bar = saddr(full + s), dst = base + s * G::STAGE;
+        mbar_expect_tx(bar, (uint32_t)(G::XBYTES + G::YBYTES));
+        tma_load4(dst, &xmap, c0, S * bx * G::TX - KS / 2, S * by * G::TY - KS / 2, S * bz * G::TZ - KS / 2, bar);
+        tma_load4(dst + G::XPAD, &ymap, o0, bx * G::TX, by * G::TY, bz * G::TZ, bar);
     };
 
-    constexpr uint32_t IDESC = idesc_bf16_mn(128, CO);
+    if (tid == 0) {
+        for (int s = 0; s < NS; ++s) mbar_init(saddr(full + s), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const int first = blockIdx.x, step = gridDim.x;
+    int issued = 0;  // thread 0: tiles issued
+    if (tid == 0)
+        for (; issued < NS - 1 && first + issued * step < ntiles; ++issued) issue(first + issued * step, issued);
+
+    float acc[G::TPW][MT][2][4];
+#pragma unroll
+    for (int t = 0; t < G::TPW; ++t)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[t][m][0][k] = acc[t][m][1][k] = 0.f;
+
+    // this lane's voxel of the K = 16 and its 16-byte chunk in an ldmatrix.x4:
+    // (voxels 0-7, 0-7, 8-15, 8-15) x (channels 0-7, 8-15, 0-7, 8-15)
+    const uint32_t lv = ((lane >> 4) << 3) | (lane & 7), lc = (lane >> 3) & 1;
+    const int tz = KS == 1 ? 0 : (G::TPW == 9 ? tg : tg / 3), ty0 = G::TPW == 3 ? tg % 3 : 0;
+    const uint32_t tapv = (uint32_t)((tz * G::XH + ty0) * G::XW);
+    float* sum = reinterpret_cast<float*>(smem + NS * G::STAGE);
+    const int g = lane >> 2, q = lane & 3;
+    bool summed = false;
+    auto flush = [&]() {
+        for (int r = 0; r < G::KG; ++r) {
+            if (kg == r) {
+#pragma unroll
+                for (int t = 0; t < G::TPW; ++t)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+#pragma unroll
+                        for (int n = 0; n < 2; ++n)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                float2* p = reinterpret_cast<float2*>(sum + (16 * m + g + 8 * h) * G::ROW +
+                                                                      (tg * G::TPW + t) * 16 + 8 * n + 2 * q);
+                                float2 v = make_float2(acc[t][m][n][2 * h], acc[t][m][n][2 * h + 1]);
+                                if (summed || r > 0) {
+                                    const float2 w = *p;
+                                    v.x += w.x;
+                                    v.y += w.y;
+                                }
+                                *p = v;
+                                acc[t][m][n][2 * h] = acc[t][m][n][2 * h + 1] = 0.f;
+                            }
+            }
+            __syncthreads();
+        }
+        summed = true;
+    };
     bool ok = true;
-    uint32_t uses[2] = {0u, 0u};
-    if (s_begin < s_end) stage(s_begin, 0);
-    int sl = s_begin;
-    for (; sl < s_end && ok; ++sl) {
-        const int b = (sl - s_begin) & 1;
-        if (sl + 1 < s_end) {
-            // the other stage is free once the MMAs of the previous slice are done
-            if (sl > s_begin) ok = mbar_wait(saddr(bar + (b ^ 1)), (uses[b ^ 1] - 1) & 1);
-            ok = __syncthreads_and(ok);
-            if (!ok) break;
-            stage(sl + 1, b ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    int it = 0;
+    for (int tile = first; tile < ntiles; tile += step, ++it) {
+        const int s = it % NS;
+        if (tid == 0 && first + issued * step < ntiles) {
+            // the stage's previous tile was read before the barrier that ended its pass
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue(first + issued * step, issued % NS);
+            ++issued;
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a_base = smem_a + b * stage_bytes, b_base = a_base + tpg * kTileBytes;
-            const uint64_t bd = smem_desc(b_base, 128, 256);
-            for (int j = 0; j < ntiles; ++j)
-                mma_bf16(tmem + (uint32_t)(j * CO), smem_desc(a_base + j * kTileBytes, 128, 256), bd, IDESC,
-                         sl > s_begin ? 1u : 0u);
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             saddr(bar + b))
-                         : "memory");
-        }
-        ++uses[b];
-    }
-    // the MMAs of the last slice (each stage's last use) are done
-    if (ok && s_end > s_begin) {
-        const int bl = (s_end - 1 - s_begin) & 1;
-        ok = mbar_wait(saddr(bar + bl), (uses[bl] - 1) & 1);
-    }
-    ok = __syncthreads_and(ok);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok && s_end > s_begin) {
-        for (int j = 0; j < ntiles; ++j) {
-            const int R = (tile0 + j) * 128 + 32 * warp + lane;
-            const int t = R / ci, c = R - t * ci;
+        ok = mbar_wait(saddr(full + s), (uint32_t)((it / NS) & 1));
+        ok = __syncthreads_and(ok);
+        if (!ok) break;
+        const uint32_t xs = base + s * G::STAGE, ys = xs + G::XPAD;
+        for (int ks = kg; ks < G::KSTEPS; ks += G::KG) {
+            constexpr int RUNS = G::TX / 16;
+            const int row = ks / RUNS, x = (ks % RUNS) * 16, z = row / G::TY, y = row % G::TY;
+            const uint32_t dv = (uint32_t)(row * G::TX + x) + lv;
+            uint32_t a[MT][4];
 #pragma unroll
-            for (int c16 = 0; c16 < CO / 16; ++c16) {
-                float v[16];
-                tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(j * CO + c16 * 16), v);
-                if (t < 27) {
+            for (int m = 0; m < MT; ++m)
+                ldmatrix4_trans(a[m], ys + (COB == 16 ? chunk16(dv, lc) : chunk32(dv, 2 * m + lc)));
+            const uint32_t xv = (uint32_t)((S * z * G::XH + S * y) * G::XW + S * x) + S * lv + tapv;
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) atomicAdd(dw + ((int64_t)(c16 * 16 + k) * 27 + t) * ci + c, v[k]);
+            for (int t = 0; t < G::TPW; ++t) {
+                uint32_t b[4];
+                ldmatrix4_trans(b, xs + chunk16(xv + (uint32_t)((t / 3) * G::XW + t % 3), lc));
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    mma_m16n8k16(acc[t][m][0], a[m], b[0], b[2]);
+                    mma_m16n8k16(acc[t][m][1], a[m], b[1], b[3]);
                 }
             }
         }
-    } else if (!ok) {
-        // a wait gave up: record it, wait (bounded) for both stages' MMAs, release the tensor memory
-        if (tid == 0) atomicOr(&g_conv_tc_flags, 1u);
-        for (int b = 0; b < 2; ++b)
-            if (uses[b]) mbar_wait(saddr(bar + b), (uses[b] - 1) & 1);
+        __syncthreads();
+        if ((it + 1) % G::FLUSH == 0) flush();
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
-}
-
-template <int CO>
-cudaError_t launch_wgrad_co(const bf16* x, const bf16* dy, float* dw, int Di, int Hi, int Wi, int ci, int S,
-                            cudaStream_t st) {
-    const int Do = (Di - 1) / S + 1, Ho = (Hi - 1) / S + 1, Wo = (Wi - 1) / S + 1;
-    const int RT = (27 * ci + 127) / 128;
-    const int tpg_max = 256 / CO;  // tensor-memory columns of a CTA <= 256
-    const int groups = (RT + tpg_max - 1) / tpg_max;
-    const int tpg = (RT + groups - 1) / groups;
-    int ncols = 32;
-    while (ncols < tpg * CO) ncols *= 2;
-    const int nslices = (int)((int64_t)Do * Ho * Wo / 16);
-    const int want = 4 * 152 / groups > 1 ? 4 * 152 / groups : 1;
-    const int spc = (nslices + want - 1) / want;
-    const int nx = (nslices + spc - 1) / spc;
-    // shared memory: two stages, two mbarriers and the tensor-memory slot,
-    // padded so that at most 512 / ncols CTAs reside on an SM (their
-    // tensor memory then always fits)
-    const int actual = 2 * (tpg * kTileBytes + CO * 32) + 32;
-    const int per_sm = 512 / ncols;
-    int bytes = 233472 / (per_sm + 1) + 1024;
-    if (bytes < actual) bytes = actual;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_conv3_wgrad_tc<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    k_conv3_wgrad_tc<CO><<<dim3((unsigned)nx, (unsigned)groups), kThreads, bytes, st>>>(
-        x, dy, dw, Di, Hi, Wi, Do, Ho, Wo, ci, S, tpg, ncols, spc, nslices);
-    return cudaGetLastError();
+    if (!ok) {
+        // a copy did not land in time: record it and wait (bounded) for those in flight
+        if (tid == 0) {
+            atomicOr(&g_conv_tc_flags, 2u);
+            for (int k = it; k < issued; ++k) mbar_wait(saddr(full + k % NS), (uint32_t)((k / NS) & 1));
+        }
+        __syncthreads();
+        return;
+    }
+    flush();
+    for (int e = tid; e < G::TAPS * COB * 16; e += G::THREADS) {
+        const int c = e & 15, t = (e >> 4) % G::TAPS, o = (e >> 4) / G::TAPS;
+        atomicAdd(dw + ((int64_t)(o0 + o) * G::TAPS + t) * ci + c0 + c, sum[o * G::ROW + t * 16 + c]);
+    }
 }
 
 // Wt [ci][t][co] = W [co][26 - t][ci]: the input gradient of a stride-1
@@ -560,6 +591,42 @@ cudaError_t input_map(CUtensorMap* map, const bf16* x, int Di, int Hi, int Wi, i
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// Tensor map of a channels-last BF16 tensor [D][H][W][C] with box
+// (bd, bh, bw, bc), bc = 16 or 32 channels, its 32- / 64-byte rows swizzled,
+// zero fill outside.
+cudaError_t tile_map(CUtensorMap* map, const bf16* x, int D, int H, int W, int C, int bd, int bh, int bw, int bc) {
+    EncodeTiled f = encode_tiled();
+    if (!f) return cudaErrorNotSupported;
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
+    const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
+    const cuuint32_t box[4] = {(cuuint32_t)bc, (cuuint32_t)bw, (cuuint32_t)bh, (cuuint32_t)bd};
+    const cuuint32_t estride[4] = {1, 1, 1, 1};
+    const CUresult r = f(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), dims, strides, box, estride,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, bc == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <class G>
+cudaError_t launch_wgrad(const bf16* x, const bf16* dy, float* dw, int Di, int Hi, int Wi, int ci, int co,
+                         cudaStream_t st) {
+    const int Do = (Di - 1) / G::S + 1, Ho = (Hi - 1) / G::S + 1, Wo = (Wi - 1) / G::S + 1;
+    CUtensorMap xm, ym;
+    cudaError_t e = tile_map(&xm, x, Di, Hi, Wi, ci, G::XD, G::XH, G::XW, 16);
+    if (e == cudaSuccess) e = tile_map(&ym, dy, Do, Ho, Wo, co, G::TZ, G::TY, G::TX, G::COB);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_conv_wgrad_tiles<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+    if (e != cudaSuccess) return e;
+    const int64_t tiles = lbm::ceil_div(Do, G::TZ) * lbm::ceil_div(Ho, G::TY) * lbm::ceil_div(Wo, G::TX);
+    const int roles = co / G::COB * (ci / 16);
+    // one CTA an SM over all channel blocks, each with about the same number of tiles
+    const int64_t want = 152 / roles > 1 ? 152 / roles : 1;
+    const int64_t per = lbm::ceil_div(tiles, want);
+    k_conv_wgrad_tiles<G><<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)roles), G::THREADS, G::SMEM, st>>>(
+        xm, ym, dw, Do, Ho, Wo, ci, (int)tiles);
+    return cudaGetLastError();
 }
 
 template <int S, int CO>
@@ -623,23 +690,24 @@ cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, 
                        : launch_s<1>(x, D, H, W, ci, w, bias, co, relu, y, y32, st);
 }
 
-bool conv3_wgrad_tc_applies(int D, int H, int W, int ci, int co, int stride) {
+bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride) {
     const bool ch = (ci == 16 || ci == 32 || ci == 64) && (co == 16 || co == 32 || co == 64);
-    if (!ch || D <= 0 || H <= 0 || W <= 0 || (stride != 1 && stride != 2)) return false;
-    const int64_t Wo = (W - 1) / stride + 1;
-    const int64_t vox = (int64_t)((D - 1) / stride + 1) * ((H - 1) / stride + 1) * Wo;
-    return Wo % 16 == 0 && vox / 16 < ((int64_t)1 << 31);
+    return ch && D > 0 && H > 0 && W > 0 && ((ks == 3 && (stride == 1 || stride == 2)) || (ks == 1 && stride == 1)) &&
+           (int64_t)D * H * W < ((int64_t)1 << 31);
 }
 
-cudaError_t conv3_wgrad_tc(const void* x, int D, int H, int W, int ci, const void* dy, int co, int stride, float* dw,
-                           cudaStream_t st) {
+cudaError_t conv_wgrad_tiles(const void* x, int D, int H, int W, int ci, const void* dy, int co, int ks, int stride,
+                             float* dw, cudaStream_t st) {
     const bf16* xb = static_cast<const bf16*>(x);
     const bf16* db = static_cast<const bf16*>(dy);
-    switch (co) {
-        case 16: return launch_wgrad_co<16>(xb, db, dw, D, H, W, ci, stride, st);
-        case 32: return launch_wgrad_co<32>(xb, db, dw, D, H, W, ci, stride, st);
-        default: return launch_wgrad_co<64>(xb, db, dw, D, H, W, ci, stride, st);
-    }
+    if (ks == 1)
+        return co == 16 ? launch_wgrad<WGeo<1, 1, 16>>(xb, db, dw, D, H, W, ci, co, st)
+                        : launch_wgrad<WGeo<1, 1, 32>>(xb, db, dw, D, H, W, ci, co, st);
+    if (stride == 1)
+        return co == 16 ? launch_wgrad<WGeo<3, 1, 16>>(xb, db, dw, D, H, W, ci, co, st)
+                        : launch_wgrad<WGeo<3, 1, 32>>(xb, db, dw, D, H, W, ci, co, st);
+    return co == 16 ? launch_wgrad<WGeo<3, 2, 16>>(xb, db, dw, D, H, W, ci, co, st)
+                    : launch_wgrad<WGeo<3, 2, 32>>(xb, db, dw, D, H, W, ci, co, st);
 }
 
 cudaError_t conv3_flip_transpose(const void* w, void* wt, int co, int ci, cudaStream_t st) {

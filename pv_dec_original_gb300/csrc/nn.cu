@@ -6,9 +6,9 @@
 // Activations are BF16, channels-last (voxel-major, channel counts padded to
 // multiples of 16); weights are BF16 [co][tap][ci] with an FP32 master copy
 // for Adam; every product accumulates in FP32 on the tensor cores.  The
-// 3x3x3 forward convolutions, stride-1 input gradients and weight
-// gradients run on tcgen05 where the grid tiles (conv_tc.cu); the kernels
-// here (mma.sync m16n8k16 BF16) take the rest and the comparison engine
+// 3x3x3 forward convolutions and stride-1 input gradients run on tcgen05
+// where the grid tiles, the weight gradients on staged tiles (conv_tc.cu);
+// the kernels here (mma.sync m16n8k16 BF16) take the rest and the comparison engine
 // (lbm_nn_set_conv_engine).  A convolution is an implicit GEMM:
 //   forward      rows = output voxels, cols = output channels, K = taps x ci
 //   input grad   rows = input voxels,  cols = input channels,  K = taps x co
@@ -696,7 +696,7 @@ std::atomic<int> g_engine{LBM_NN_ENGINE_AUTO};
 
 // 3x3x3 on shapes the tensor-core kernels tile (conv_tc.cu): the forward
 // convolution at stride 1 or 2, the input gradient at stride 1 (the weight
-// gradient: conv3_wgrad_tc_applies).
+// gradient: conv_wgrad_tiles_applies).
 bool use_tc(const Conv& g) {
     return g_engine.load() == LBM_NN_ENGINE_AUTO && g.ks == 3 &&
            lbm::conv3_tc_applies(g.D, g.H, g.W, g.ci, g.co, g.stride);
@@ -833,9 +833,9 @@ lbm_status lbm_nn_conv3d_bwd(const void* x, const int dims_in[3], int ci, const 
             e = launch_gemm<1>(ci, static_cast<const bf16*>(dy), static_cast<const bf16*>(w_t), nullptr,
                                static_cast<bf16*>(dx), nullptr, g, rows_in, co, 0, st);
     }
-    if (e == cudaSuccess && dw && g.ks == 3 && g_engine.load() == LBM_NN_ENGINE_AUTO && aligned16(x) &&
-        aligned16(dy) && lbm::conv3_wgrad_tc_applies(g.D, g.H, g.W, ci, co, g.stride)) {
-        e = lbm::conv3_wgrad_tc(x, g.D, g.H, g.W, ci, dy, co, g.stride, dw, st);
+    if (e == cudaSuccess && dw && g_engine.load() == LBM_NN_ENGINE_AUTO &&
+        lbm::conv_wgrad_tiles_applies(g.D, g.H, g.W, ci, co, g.ks, g.stride)) {
+        e = lbm::conv_wgrad_tiles(x, g.D, g.H, g.W, ci, dy, co, g.ks, g.stride, dw, st);
     } else if (e == cudaSuccess && dw) {
         const bf16* xb = static_cast<const bf16*>(x);
         const bf16* dyb = static_cast<const bf16*>(dy);
