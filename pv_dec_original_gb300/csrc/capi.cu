@@ -563,17 +563,32 @@ bool read_stl(const char* path, std::vector<double>& out) {
 }
 
 void reference_bbox(const double* t, int64_t ntri, double spacing, double* bb, int* dims) {
-    double mnx = INFINITY, mny = INFINITY, mnz = INFINITY, mxx = -INFINITY, mxy = -INFINITY, mxz = -INFINITY;
-    for (int64_t k = 0; k < ntri; ++k) {
-        const double* r = t + 12 * k;
+    // four running extremes a side, merged at the end: one chain of minima
+    // over 70k triangles took 0.3 ms
+    constexpr int U = 4;
+    double lo[U][3], hi[U][3];
+    for (int u = 0; u < U; ++u)
+        for (int a = 0; a < 3; ++a) { lo[u][a] = INFINITY; hi[u][a] = -INFINITY; }
+    auto take = [&](int u, const double* r) {
         // the y and z extremes ignore the third vertex (ComplexGeometry.cpp:147-151)
-        mnx = std::min(std::min(std::min(mnx, r[0]), r[3]), r[6]);
-        mny = std::min(std::min(mny, r[1]), r[4]);
-        mnz = std::min(std::min(mnz, r[2]), r[5]);
-        mxx = std::max(std::max(std::max(mxx, r[0]), r[3]), r[6]);
-        mxy = std::max(std::max(mxy, r[1]), r[4]);
-        mxz = std::max(std::max(mxz, r[2]), r[5]);
-    }
+        // (a NaN loses every comparison in this order)
+        lo[u][0] = std::min(std::min(std::min(lo[u][0], r[0]), r[3]), r[6]);
+        hi[u][0] = std::max(std::max(std::max(hi[u][0], r[0]), r[3]), r[6]);
+        for (int a = 1; a < 3; ++a) {
+            lo[u][a] = std::min(std::min(lo[u][a], r[a]), r[3 + a]);
+            hi[u][a] = std::max(std::max(hi[u][a], r[a]), r[3 + a]);
+        }
+    };
+    int64_t k = 0;
+    for (; k + U <= ntri; k += U)
+        for (int u = 0; u < U; ++u) take(u, t + 12 * (k + u));
+    for (; k < ntri; ++k) take(0, t + 12 * k);
+    for (int u = 1; u < U; ++u)
+        for (int a = 0; a < 3; ++a) {
+            lo[0][a] = std::min(lo[0][a], lo[u][a]);
+            hi[0][a] = std::max(hi[0][a], hi[u][a]);
+        }
+    const double mnx = lo[0][0], mny = lo[0][1], mnz = lo[0][2], mxx = hi[0][0], mxy = hi[0][1], mxz = hi[0][2];
     bb[0] = mnx; bb[1] = mxx; bb[2] = mny; bb[3] = mxy; bb[4] = mnz; bb[5] = mxz;
     dims[0] = (int)std::ceil((mxx - mnx) / spacing) + 1;
     dims[1] = (int)std::ceil((mxy - mny) / spacing) + 1;
@@ -786,31 +801,13 @@ lbm_status lbm_voxelize(const double* tri12, int64_t ntri, lbm_vox_desc* desc, u
     const int nx = desc->dims[0], ny = desc->dims[1], nz = desc->dims[2];
     if (nx <= 0 || ny <= 0 || nz <= 0) return fail(nullptr, LBM_ERR_ARG, "empty lattice");
     if (!mask_out) return LBM_OK;
-    const int64_t npts = (int64_t)nx * ny * nz;
     cudaStream_t st = nullptr;
-    double* d_tri = nullptr;
-    uint8_t* d_mask = nullptr;
     std::string err;
-    auto cleanup = [&]() {
-        if (d_tri) cudaFree(d_tri);
-        if (d_mask) cudaFree(d_mask);
-        if (st) cudaStreamDestroy(st);
-    };
-    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&d_tri, sizeof(double) * 12 * (ntri > 0 ? ntri : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&d_mask, npts);
-    if (e == cudaSuccess && ntri > 0)
-        e = cudaMemcpyAsync(d_tri, tri12, sizeof(double) * 12 * ntri, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_mask, 0, npts, st);
     VoxResult res{};
-    if (e == cudaSuccess) {
-        e = voxelize_device(d_tri, ntri, desc->bbox, desc->origin, desc->spacing, desc->dims, d_mask, &res, st, &err);
-    } else {
-        err = cudaGetErrorString(e);
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(mask_out, d_mask, npts, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cleanup();
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = voxelize_device(tri12, ntri, desc->bbox, desc->origin, desc->spacing, desc->dims, mask_out, &res, st, &err);
+    if (st) cudaStreamDestroy(st);
     if (e != cudaSuccess)
         return fail(nullptr, e == cudaErrorMemoryAllocation ? LBM_ERR_ALLOC : LBM_ERR_CUDA,
                     "voxelize: " + (err.empty() ? std::string(cudaGetErrorString(e)) : err));

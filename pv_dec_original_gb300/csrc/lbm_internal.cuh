@@ -208,8 +208,9 @@ struct VoxResult {
     int64_t fluid;
     int64_t tests;
 };
-cudaError_t voxelize_device(const double* d_tri, int64_t ntri, const double bbox[6], const double origin[3],
-                            double spacing, const int dims[3], uint8_t* d_mask, VoxResult* res, cudaStream_t s,
+// Host triangles to the host mask (nx * ny * nz bytes), waiting for both copies.
+cudaError_t voxelize_device(const double* tri, int64_t ntri, const double bbox[6], const double origin[3],
+                            double spacing, const int dims[3], uint8_t* mask, VoxResult* res, cudaStream_t s,
                             std::string* err);
 
 // Exclusive scan of int64 counts (scan.cu); returns the total.

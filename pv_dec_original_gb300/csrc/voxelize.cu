@@ -28,9 +28,10 @@
 // vertex, a point on the facet) is left to the reference's own FP64 test of
 // that (point, triangle).  The pair flips the parity of a range of k: two
 // bits of a difference bit field, whose running XOR along k is the mask.
-// (70,040 triangles on a 56 x 54 x 509 lattice: 0.06 ms on the device,
+// (70,040 triangles on a 56 x 54 x 509 lattice: 0.19 ms in these kernels,
 // where one FP64 test per point and candidate took 12.3 ms at GB300's two
-// FP64 multiply-adds a cycle and SM.)
+// FP64 multiply-adds a cycle and SM; k_tri_columns is bound by its ~400 FP64
+// operations a triangle.)
 #include <cmath>
 #include <algorithm>
 
@@ -139,7 +140,7 @@ __device__ double cull_margin(const double* T, double zspan) {
 struct VoxParams {
     double bb[6];
     double org[3];
-    double s;
+    double s, inv_s;
     double zspan;     // of cull_margin
     double span;      // bound of every coordinate difference of the tests
     double dz;        // ray length of an unadjusted ray
@@ -195,6 +196,22 @@ struct TriConst {
     double inv_fz;                      // 1 / facet normal z
 };
 
+// Bound of the rounding of the barycentric coordinates, as the reference
+// computes them, for any point of a column: an error eps * span in w moves
+// the point on the computed plane by eps span L^2 / |nZ| along z, and that
+// by a factor L / |n| in the coordinates; with shape = L^2 / |n| that is
+// eps shape^2 (|n| / |nZ|) (span / L), times a small count of operations
+// (< 30); 4e-12 is 36,000 eps.  L2: the larger squared edge at vertex 1
+// (the third edge is at most twice as long); n2, nZ: the computed normal.
+// In FP32 where nothing can underflow: the bound needs no digits (GB300's
+// FP64 rate is 1/64 of FP32's).
+__device__ __forceinline__ double barycentric_bound(const VoxParams& P, double L2, double n2, double nZ) {
+    const float l2 = (float)L2, m2 = (float)n2;
+    if (!(l2 > 1e-8f && l2 < 1e8f && m2 > 1e-20f))
+        return 4e-12 * (L2 / n2 * L2) * (sqrt(n2) / fabs(nZ)) * (1.0 + P.span / sqrt(L2));
+    return 4e-12f * (l2 * l2 / m2) * (sqrtf(m2) / fabsf((float)nZ)) * (1.0f + (float)P.span * rsqrtf(l2));
+}
+
 __device__ __forceinline__ TriConst tri_const(const VoxParams& P, const double* T) {
     TriConst c;
     c.uX = T[3] - T[0]; c.uY = T[4] - T[1]; c.uZ = T[5] - T[2];
@@ -208,17 +225,10 @@ __device__ __forceinline__ TriConst tri_const(const VoxParams& P, const double* 
     c.vv = c.vX * c.vX + c.vY * c.vY + c.vZ * c.vZ;
     c.inv_D = 1.0 / (c.uv * c.uv - c.uu * c.vv);
     const double n2 = c.nX * c.nX + c.nY * c.nY + c.nZ * c.nZ;
-    const double L2 = fmax(c.uu, c.vv);  // squared edge scale (the third edge is at most twice as long)
-    // The barycentric coordinates' rounding: an error eps * span in w moves
-    // the point on the computed plane by eps span L^2 / |nZ| along z, and
-    // that by a factor L / |n| in the coordinates; with shape = L^2 / |n|
-    // that is eps shape^2 (|n| / |nZ|) (span / L), times a small count of
-    // operations (< 30); 1e-12 is 9000 eps.
-    const double L = sqrt(L2);
-    c.E = 4e-12 * (L2 * L2 / n2) * (sqrt(n2) * fabs(c.inv_nZ)) * (1.0 + P.span / L);
+    c.E = barycentric_bound(P, fmax(c.uu, c.vv), n2, c.nZ);
     c.inv_fz = 1.0 / T[11];
     const double den = fabs(P.dz * T[11]);  // the reference rejects |den| < 1e-16
-    if (!(c.E < 1e-2) || !(den > 2e-16) || !isfinite(c.inv_fz) || P.exact_only) c.E = -1.0;
+    if (!isfinite(c.E) || !(den > 2e-16) || !isfinite(c.inv_fz) || P.exact_only) c.E = -1.0;
     return c;
 }
 
@@ -244,7 +254,7 @@ __device__ __forceinline__ void column_pair(const VoxParams& P, const TriConst& 
         // 0 <= t <= 1 of the ray parameter: z* - dz <= pz(k) <= z*
         const double ax = (T[0] - px) * T[9], ay = (T[1] - py) * T[10];
         const double zs = T[2] + (ax + ay) * t.inv_fz;
-        const double inv_s = 1.0 / P.s;
+        const double inv_s = P.inv_s;
         const double p0 = P.org[2] + 0.5 * P.s;
         const double kU = (zs - p0) * inv_s, kL = (zs - P.dz - p0) * inv_s;
         const double tol = (1e-12 * ((fabs(ax) + fabs(ay)) * fabs(t.inv_fz) + fabs(T[2]) + P.zabs)) * inv_s +
@@ -274,12 +284,28 @@ __device__ __forceinline__ void column_pair(const VoxParams& P, const TriConst& 
     if (slot < (unsigned long long)P.cap) list[slot] = make_int2(tri, (int)c);  // else: a second run with room for all
 }
 
-// A triangle's columns: the lattice range of its widened xy extent.
+// A triangle's columns: the lattice range of its xy extent widened by the
+// distance within which rounding can matter.  A point d outside an edge has
+// a barycentric coordinate at least d / (2 L) outside [0, 1] (no height of
+// the triangle exceeds 2 L), so beyond 4 L E no test passes.  `pairs` counts
+// the columns of cull_margin's wider extent: the tests this replaces.
 struct TriExtent {
     double x0, x1, y0, y1;
     int i0, i1, j0, j1;
     int kind;  // 0: never counts, 1: columns i0..i1, j0..j1, 2: global list
+    unsigned pairs;
 };
+
+// Lattice indices whose column coordinate may lie in [a, b] (one more on
+// either side: the coordinates' rounding).
+__device__ __forceinline__ bool index_range(double a, double b, double org, double inv_s, int n, int& k0, int& k1) {
+    // clamp in FP64 before converting: margins can be far outside int range
+    const double f0 = fmax(floor((a - org) * inv_s) - 1.0, 0.0), f1 = fmin(ceil((b - org) * inv_s) + 1.0, n - 1.0);
+    if (!(f0 <= f1)) return false;
+    k0 = (int)f0;
+    k1 = (int)f1;
+    return true;
+}
 
 __device__ __forceinline__ TriExtent tri_extent(const VoxParams& P, const double* T) {
     TriExtent e{};
@@ -287,44 +313,70 @@ __device__ __forceinline__ TriExtent tri_extent(const VoxParams& P, const double
     const double m = cull_margin(T, P.zspan);
     e.kind = m < 0.0 ? 0 : (m > 1e29 ? 2 : 1);
     if (e.kind != 1) return e;
-    e.x0 = fmin(fmin(T[0], T[3]), T[6]) - m;
-    e.x1 = fmax(fmax(T[0], T[3]), T[6]) + m;
-    e.y0 = fmin(fmin(T[1], T[4]), T[7]) - m;
-    e.y1 = fmax(fmax(T[1], T[4]), T[7]) + m;
-    // clamp in FP64 before converting: margins can be far outside int range
-    const double fi0 = fmax(floor((e.x0 - P.org[0]) / P.s) - 1.0, 0.0);
-    const double fi1 = fmin(ceil((e.x1 - P.org[0]) / P.s) + 1.0, P.nx - 1.0);
-    const double fj0 = fmax(floor((e.y0 - P.org[1]) / P.s) - 1.0, 0.0);
-    const double fj1 = fmin(ceil((e.y1 - P.org[1]) / P.s) + 1.0, P.ny - 1.0);
-    if (fi0 <= fi1 && fj0 <= fj1) {
-        e.i0 = (int)fi0; e.i1 = (int)fi1; e.j0 = (int)fj0; e.j1 = (int)fj1;
+    const double xl = fmin(fmin(T[0], T[3]), T[6]), xh = fmax(fmax(T[0], T[3]), T[6]);
+    const double yl = fmin(fmin(T[1], T[4]), T[7]), yh = fmax(fmax(T[1], T[4]), T[7]);
+    if (!index_range(xl - m, xh + m, P.org[0], P.inv_s, P.nx, e.i0, e.i1) ||
+        !index_range(yl - m, yh + m, P.org[1], P.inv_s, P.ny, e.j0, e.j1)) {
+        e.i0 = e.j0 = 0;
+        e.i1 = e.j1 = -1;
+        return e;
+    }
+    unsigned ni = 0, nj = 0;
+    for (int i = e.i0; i <= e.i1; ++i) {
+        const double x = column_x(P, i);
+        ni += x >= xl - m && x <= xh + m;
+    }
+    for (int j = e.j0; j <= e.j1; ++j) {
+        const double y = column_y(P, j);
+        nj += y >= yl - m && y <= yh + m;
+    }
+    e.pairs = ni * nj;
+    const double uX = T[3] - T[0], uY = T[4] - T[1], uZ = T[5] - T[2];
+    const double vX = T[6] - T[0], vY = T[7] - T[1], vZ = T[8] - T[2];
+    const double nX = uY * vZ - uZ * vY, nY = uZ * vX - uX * vZ, nZ = uX * vY - uY * vX;
+    const double L2 = fmax(uX * uX + uY * uY + uZ * uZ, vX * vX + vY * vY + vZ * vZ);
+    const double t = 4.0 * (double)sqrtf((float)L2) * barycentric_bound(P, L2, nX * nX + nY * nY + nZ * nZ, nZ);
+    const double w = t < m ? t : m;  // (a NaN or infinite bound keeps m)
+    e.x0 = xl - w; e.x1 = xh + w;
+    e.y0 = yl - w; e.y1 = yh + w;
+    if (!index_range(e.x0, e.x1, P.org[0], P.inv_s, P.nx, e.i0, e.i1) ||
+        !index_range(e.y0, e.y1, P.org[1], P.inv_s, P.ny, e.j0, e.j1)) {
+        e.i0 = e.j0 = 0;
+        e.i1 = e.j1 = -1;
     }
     return e;
 }
 
-__device__ __forceinline__ void add_pairs(unsigned pairs, VoxCounters* __restrict__ cnt) {
-    pairs = __reduce_add_sync(0xffffffffu, pairs);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&cnt->pairs, (unsigned long long)pairs);
+__device__ __forceinline__ void add_pairs(unsigned long long pairs, VoxCounters* __restrict__ cnt) {
+    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_down_sync(0xffffffffu, pairs, o);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&cnt->pairs, pairs);
 }
 
 // One thread a triangle: classification and, for extents of up to
 // kWideColumns columns (a mesh about as fine as the lattice), its columns;
 // wider ones go to the wide list.
 constexpr int kWideColumns = 32;
-__global__ void __launch_bounds__(128) k_tri_columns(const VoxParams P, const double* __restrict__ tri,
+struct WideTri {
+    TriExtent e;
+    int32_t tri;
+};
+__global__ void __launch_bounds__(128, 4) k_tri_columns(const VoxParams P, const double* __restrict__ tri,
                                                      uint32_t* __restrict__ bits, int2* __restrict__ list,
-                                                     int32_t* __restrict__ glob, int32_t* __restrict__ wide,
-                                                     VoxCounters* __restrict__ cnt) {
+                                                     int32_t* __restrict__ glob, WideTri* __restrict__ wide,
+                                                        VoxCounters* __restrict__ cnt) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned pairs = 0;
+    unsigned long long pairs = 0;
     if (t < P.ntri) {
         const double* T = tri + 12 * t;
         const TriExtent e = tri_extent(P, T);
+        pairs = e.pairs;
         const int64_t n = (int64_t)(e.i1 - e.i0 + 1) * (e.j1 - e.j0 + 1);
         if (e.kind == 2) {
             glob[atomicAdd(&cnt->nglob, 1ull)] = (int32_t)t;
         } else if (n > kWideColumns) {
-            wide[atomicAdd(&cnt->nwide, 1ull)] = (int32_t)t;
+            const unsigned long long w = atomicAdd(&cnt->nwide, 1ull);
+            wide[w].e = e;
+            wide[w].tri = (int32_t)t;
         } else if (n > 0) {
             TriConst k;
             bool have = false;
@@ -335,7 +387,6 @@ __global__ void __launch_bounds__(128) k_tri_columns(const VoxParams P, const do
                     const double xx = column_x(P, i);
                     if (xx < e.x0 || xx > e.x1) continue;
                     if (!have) { k = tri_const(P, T); have = true; }
-                    ++pairs;
                     column_pair(P, k, T, (int32_t)t, i, j, xx, yy, bits, list, cnt);
                 }
             }
@@ -348,28 +399,25 @@ __global__ void __launch_bounds__(128) k_tri_columns(const VoxParams P, const do
 // walked the 576 columns of a cap's facet in 1 ms, one after another).
 __global__ void __launch_bounds__(128) k_wide_columns(const VoxParams P, const double* __restrict__ tri,
                                                       uint32_t* __restrict__ bits, int2* __restrict__ list,
-                                                      const int32_t* __restrict__ wide,
+                                                      const WideTri* __restrict__ wide,
                                                       VoxCounters* __restrict__ cnt) {
     const unsigned long long nwide = cnt->nwide;
-    unsigned pairs = 0;
     for (unsigned long long w = blockIdx.y; w < nwide; w += gridDim.y) {
-        const int32_t t = wide[w];
-        const double* T = tri + 12 * (int64_t)t;
-        const TriExtent e = tri_extent(P, T);
+        const TriExtent e = wide[w].e;
         const int nc = e.i1 - e.i0 + 1;
         const int64_t n = (int64_t)nc * (e.j1 - e.j0 + 1);
         int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (c >= n) continue;
+        const int32_t t = wide[w].tri;
+        const double* T = tri + 12 * (int64_t)t;
         const TriConst k = tri_const(P, T);
         for (; c < n; c += (int64_t)gridDim.x * blockDim.x) {
             const int i = e.i0 + (int)(c % nc), j = e.j0 + (int)(c / nc);
             const double xx = column_x(P, i), yy = column_y(P, j);
             if (xx < e.x0 || xx > e.x1 || yy < e.y0 || yy > e.y1) continue;
-            ++pairs;
             column_pair(P, k, T, t, i, j, xx, yy, bits, list, cnt);
         }
     }
-    add_pairs(pairs, cnt);
 }
 
 // The pairs no bound decided: one warp a pair, the reference's test for
@@ -444,13 +492,14 @@ __global__ void __launch_bounds__(128) k_mask(const VoxParams P, const double* _
 
 }  // namespace
 
-cudaError_t voxelize_device(const double* d_tri, int64_t ntri, const double bbox[6], const double origin[3],
-                            double spacing, const int dims[3], uint8_t* d_mask, VoxResult* res, cudaStream_t st,
+cudaError_t voxelize_device(const double* tri, int64_t ntri, const double bbox[6], const double origin[3],
+                            double spacing, const int dims[3], uint8_t* mask, VoxResult* res, cudaStream_t st,
                             std::string* err) {
     VoxParams P{};
     for (int q = 0; q < 6; ++q) P.bb[q] = bbox[q];
     for (int q = 0; q < 3; ++q) P.org[q] = origin[q];
     P.s = spacing;
+    P.inv_s = 1.0 / spacing;
     P.nx = dims[0]; P.ny = dims[1]; P.nz = dims[2];
     P.ncol = (int64_t)P.nx * P.ny;
     P.ntri = ntri;
@@ -486,32 +535,47 @@ cudaError_t voxelize_device(const double* d_tri, int64_t ntri, const double bbox
     const int nw = (int)ceil_div(P.nz, 32);
     const int64_t tri_alloc = ntri > 0 ? ntri : 1;
     VoxCounters got{};
-    // one run of the kernels with room for `cap` undecided pairs, scratch in
-    // one allocation: counters, bit field, pair, global and wide lists
+    // one run with room for `cap` undecided pairs; triangles, mask, counters,
+    // bit field, pair, global and wide lists in one allocation
     auto run = [&](int64_t cap) -> cudaError_t {
         P.cap = cap;
-        const size_t b_cnt = 256, b_bits = sizeof(uint32_t) * (size_t)nw * P.ncol;
-        const size_t o_list = (b_cnt + b_bits + 255) / 256 * 256;
-        const size_t o_glob = (o_list + sizeof(int2) * (size_t)cap + 255) / 256 * 256;
+        const int64_t npts = P.ncol * P.nz;
+        size_t at = 0;
+        auto place = [&](size_t bytes) {
+            const size_t o = at;
+            at = (at + bytes + 255) / 256 * 256;
+            return o;
+        };
+        const size_t o_cnt = place(sizeof(VoxCounters)), b_bits = sizeof(uint32_t) * (size_t)nw * P.ncol;
+        const size_t o_bits = place(b_bits), o_list = place(sizeof(int2) * (size_t)cap);
+        const size_t o_glob = place(sizeof(int32_t) * tri_alloc), o_wide = place(sizeof(WideTri) * tri_alloc);
+        const size_t o_tri = place(sizeof(double) * 12 * tri_alloc), o_mask = place((size_t)npts);
         unsigned char* base = nullptr;
-        VOX_CHECK(cudaMallocAsync(&base, o_glob + 2 * sizeof(int32_t) * (size_t)tri_alloc, st));
-        VoxCounters* cnt = reinterpret_cast<VoxCounters*>(base);
-        uint32_t* bits = reinterpret_cast<uint32_t*>(base + b_cnt);
+        VOX_CHECK(cudaMallocAsync(&base, at, st));
+        VoxCounters* cnt = reinterpret_cast<VoxCounters*>(base + o_cnt);
+        uint32_t* bits = reinterpret_cast<uint32_t*>(base + o_bits);
         int2* list = reinterpret_cast<int2*>(base + o_list);
         int32_t* glob = reinterpret_cast<int32_t*>(base + o_glob);
-        int32_t* wide = glob + tri_alloc;
+        WideTri* wide = reinterpret_cast<WideTri*>(base + o_wide);
+        double* d_tri = reinterpret_cast<double*>(base + o_tri);
+        uint8_t* d_mask = base + o_mask;
         auto body = [&]() -> cudaError_t {
-            VOX_CHECK(cudaMemsetAsync(base, 0, b_cnt + b_bits, st));
+            VOX_CHECK(cudaMemsetAsync(base, 0, o_bits + b_bits, st));
             if (ntri > 0) {
+                VOX_CHECK(cudaMemcpyAsync(d_tri, tri, sizeof(double) * 12 * ntri, cudaMemcpyHostToDevice, st));
                 k_tri_columns<<<(unsigned)ceil_div(ntri, 128), 128, 0, st>>>(P, d_tri, bits, list, glob, wide, cnt);
-                k_wide_columns<<<dim3(16, 152), 128, 0, st>>>(P, d_tri, bits, list, wide, cnt);
+                k_wide_columns<<<dim3(8, 304), 128, 0, st>>>(P, d_tri, bits, list, wide, cnt);
                 k_exact_pairs<<<608, 128, 0, st>>>(P, d_tri, bits, list, cnt);
                 VOX_CHECK(cudaGetLastError());
             }
-            k_mask<<<dim3((unsigned)ceil_div(P.ncol, 128), (unsigned)std::min(nw, 4096)), 128, 0, st>>>(P, d_tri, bits, glob, d_mask,
-                                                                                        cnt);
+            k_mask<<<dim3((unsigned)ceil_div(P.ncol, 128), (unsigned)std::min(nw, 4096)), 128, 0, st>>>(
+                P, d_tri, bits, glob, d_mask, cnt);
             VOX_CHECK(cudaGetLastError());
+            // the caller's pages are touched while the kernels run: a copy
+            // into pages the process has never written ran at 1.1 GB/s
+            for (int64_t k = 0; k < npts; k += 4096) reinterpret_cast<volatile uint8_t*>(mask)[k] = 0;
             VOX_CHECK(cudaMemcpyAsync(&got, cnt, sizeof(got), cudaMemcpyDeviceToHost, st));
+            VOX_CHECK(cudaMemcpyAsync(mask, d_mask, (size_t)npts, cudaMemcpyDeviceToHost, st));
             VOX_CHECK(cudaStreamSynchronize(st));
             return cudaSuccess;
         };
