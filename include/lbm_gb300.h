@@ -333,7 +333,7 @@ lbm_status lbm_preset_flags(lbm_handle* h, unsigned flags);
 
 /* Launch-shape variants of the step kernel: one node per thread with
  * (block size, minimum resident blocks per SM) = (128,12) (128,10) (128,8)
- * (256,3) (256,1); variant 5, the tiled kernel (bulk copies stage each
+ * (256,3) (256,1), the last (64,8) in FP64; variant 5, the tiled kernel (bulk copies stage each
  * 256-node tile's sources in shared memory; physics mode, FP32 / FP16 /
  * BF16; elsewhere it runs variant 0, or 4 for FP64); variants 6 (128,10)
  * and 7 (128,12), the compact kernel (32 bytes of node metadata per warp of

@@ -52,7 +52,7 @@ struct lbm_handle {
     bool has_state = false;
     void* buf[2] = {nullptr, nullptr};
     int cur = 0;
-    void* stale = nullptr;
+    void* stale[2] = {nullptr, nullptr};  // parity: post-boundary f of the boundary list; stale[cur] of the last step
     void* nw_prev = nullptr;
     double *nw_n = nullptr, *nw_wss = nullptr, *nw_acc = nullptr, *nw_accm = nullptr;
     float *nw_nf = nullptr, *nw_wssf = nullptr;  // FP32-arithmetic formats
@@ -238,13 +238,13 @@ void free_geometry(lbm_handle* h) {
     void* ptrs[] = {g.cls, g.sp_pt, g.sp_miss, g.sp_cls, g.sp_nw, g.sp_bc, g.bcidx, g.sp_prof, g.nw_pt, g.act_word,
                     g.sp_of_act, h->bct, h->sp_flux,
                     g.act_idx, g.act_pt,
-                    h->buf[0], h->buf[1], h->stale, h->nw_prev, h->nw_n, h->nw_wss, h->nw_acc, h->nw_accm,
+                    h->buf[0], h->buf[1], h->stale[0], h->stale[1], h->nw_prev, h->nw_n, h->nw_wss, h->nw_acc, h->nw_accm,
                     h->partials, h->sums, h->out_f, h->macro, h->seg_delta, h->nw_nf, h->nw_wssf, h->nw_accf, h->tile_plan,
                     h->nw_ring, h->nw_out, h->sp_q, h->nw_fields, h->seg_abs, h->warp_block};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     g = GeometryLists();
-    h->buf[0] = h->buf[1] = h->stale = h->nw_prev = nullptr;
+    h->buf[0] = h->buf[1] = h->stale[0] = h->stale[1] = h->nw_prev = nullptr;
     h->nw_n = h->nw_wss = h->nw_acc = h->nw_accm = h->partials = h->sums = h->out_f = h->macro = nullptr;
     h->seg_delta = nullptr;
     h->nseg = 0;
@@ -291,7 +291,10 @@ StepParams make_params(lbm_handle* h, int kind) {
     p.sp_cls = h->g.sp_cls;
     p.sp_nw = h->g.sp_nw;
     p.sp_prof = h->g.sp_prof;
-    p.stale = h->stale;
+    // a step reads the last step's and writes the other; the prologue (after
+    // which cur is 1) writes stale[1]; a read-out reads the last step's
+    p.stale_in = h->stale[h->cur];
+    p.stale = kind == 1 ? h->stale[1] : h->stale[1 - h->cur];
     p.nnw = h->g.nnw;
     p.nw_n = h->nw_n;
     p.nw_wss = h->nw_wss;
@@ -325,6 +328,7 @@ StepParams make_params(lbm_handle* h, int kind) {
     p.sp_q = h->d.mode == LBM_PHYSICS ? h->sp_q : nullptr;
     p.flags = h->flags;
     p.act_idx = h->g.act_idx;
+    p.nw_pt = h->g.nw_pt;
     p.partials = h->partials;
     return p;
 }
@@ -943,7 +947,7 @@ lbm_status lbm_set_geometry(lbm_handle* h, const uint8_t* mask, const int dims[3
     CK(h, cudaMemsetAsync(h->buf[0], 0, es * Q * h->stride, h->st));
     CK(h, cudaMemsetAsync(h->buf[1], 0, es * Q * h->stride, h->st));
     if (h->d.mode == LBM_PARITY) {
-        CK(h, dalloc(h, &h->stale, rs * Q * (h->g.nsp + 1)));
+        for (void*& b : h->stale) CK(h, dalloc(h, &b, rs * Q * (h->g.nsp + 1)));
         CK(h, dalloc(h, &h->nw_prev, rs * 4 * (h->g.nnw + 1)));
     }
     CK(h, dalloc(h, &h->nw_n, sizeof(double) * 3 * (h->g.nnw + 1)));
@@ -1723,7 +1727,8 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* best, float* ms_per
         {h->nw_accf, sizeof(float2) * 4 * (h->g.nnw + 1), nullptr},
         {h->nw_wssf, sizeof(float) * (h->g.nnw + 1), nullptr},
         {h->nw_ring, sizeof(float) * kRingSlots * 4 * (h->g.nnw + 1), nullptr}};
-    if (h->stale) items.push_back({h->stale, rs * h->d.Q * (h->g.nsp + 1), nullptr});
+    for (void* b : h->stale)
+        if (b) items.push_back({b, rs * h->d.Q * (h->g.nsp + 1), nullptr});
     if (h->nw_prev) items.push_back({h->nw_prev, rs * 4 * (h->g.nnw + 1), nullptr});
     auto release = [&]() {
         for (Item& it : items)

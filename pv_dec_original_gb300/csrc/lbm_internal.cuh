@@ -96,7 +96,11 @@ struct StepParams {
     const int32_t* sp_bc;     // boundary-condition rule of a boundary-list entry (-1: none)
     double* sp_flux;          // read-out: momentum along the rule's face axis, per entry
     const float* sp_q;        // physics: wall distance of each missing link, [Q][nsp] (null: half-way bounce-back)
-    void* stale;              // parity: previous post-boundary f, [q][nsp] in the arithmetic type
+    // parity: post-boundary f of the boundary list, [q][nsp] in the arithmetic
+    // type: the previous step's, and this step's (another buffer: the FP64
+    // stress blocks read stale_in while the nodes' threads write stale)
+    const void* stale_in;
+    void* stale;
     // next-to-wall accumulators
     int64_t nnw;
     const double* nw_n;       // [3][nnw]
@@ -114,7 +118,8 @@ struct StepParams {
     const float* nw_nf;       // [3][nw_stride]
     int64_t nw_stride;        // plane stride of nw_nf (nnw + 1 rounded up to 4)
     float* nw_ring;           // float4 [kRingSlots][nnw]: step s in slot s % kRingSlots
-    int64_t fold_blocks;      // leading blocks of a step launch that fold the ring (set by the launcher)
+    int64_t fold_blocks;      // leading blocks of a step launch that fold the ring, or (FP64) compute the
+                              // next-to-wall stress (set by the launcher)
     int pdl_early;            // step launch: let the next launch begin at block start (else at block end)
     float2* nw_accf;          // [4][nnw]
     void* nw_prev;            // parity: rho, ux, uy, uz of the previous collision, [4][nnw]
@@ -146,7 +151,8 @@ struct StepParams {
     double* out_f;            // [a*Q + q] FP64, or null
     double* out_rho;          // rho per node (FP64 moments of the full f), or null
     double* out_u;            // u per node, 3 per node, or null
-    const int32_t* act_idx;   // per point active index (readout only)
+    const int32_t* act_idx;   // per point active index
+    const int64_t* nw_pt;     // point of a next-to-wall node (FP64 stress)
     double* partials;         // per block: mass - nact, mom3
 };
 

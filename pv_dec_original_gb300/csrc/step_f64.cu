@@ -62,7 +62,7 @@ __global__ void k_warm(const float* __restrict__ rho, const float* __restrict__ 
     const double r = rho[a];
     const double ux = u[3 * a], uy = u[3 * a + 1], uz = u[3 * a + 2];
     double e[Q];
-    feq_all<Q, double, false>(e, r, ux, uy, uz);
+    feq_all<Q>(e, r, ux, uy, uz);
     if (regularized) {
         const int64_t n = act_pt[a];
         const int idx[3] = {(int)(n % nx), (int)((n / nx) % ny), (int)(n / ((int64_t)nx * ny))};

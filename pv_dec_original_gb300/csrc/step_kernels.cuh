@@ -64,6 +64,42 @@ __device__ __forceinline__ void momentum(const R (&f)[Q], R& px, R& py, R& pz) {
     }
 }
 
+// x / d, y / d and z / d, rounded as three divisions round them, from one
+// reciprocal: with h = RN(1 / d), q = RN(x h) is within an ulp or so of x / d
+// and RN(q + h RN(x - q d)), the remainder by a fused multiply-add, is the
+// correctly rounded quotient (Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), as long
+// as nothing comes near the exponent range's ends and h is not the one
+// exception, a d with an all-ones mantissa.  Densities and momenta never do;
+// anything else takes the divisions.
+__device__ __forceinline__ bool mid_exponent(double v) {
+    // 2^-500 <= |v| < 2^500, or v == 0
+    const uint32_t h = (uint32_t)__double2hiint(v) & 0x7fffffffu;
+    return (h - (523u << 20) < (1000u << 20)) || ((h | (uint32_t)__double2loint(v)) == 0u);
+}
+
+__device__ __forceinline__ void divide3(double x, double y, double z, double d, double& qx, double& qy, double& qz) {
+    const uint32_t dh = (uint32_t)__double2hiint(d), dl = (uint32_t)__double2loint(d);
+    const bool plain = ((dh & 0x7fffffffu) - (923u << 20) < (200u << 20)) &&
+                       !(dl == 0xffffffffu && (dh & 0xfffffu) == 0xfffffu);
+    if (plain && mid_exponent(x) && mid_exponent(y) && mid_exponent(z)) {
+        const double h = __drcp_rn(d);
+        const double a = x * h, b = y * h, c = z * h;
+        // (a quotient of -0 keeps its sign)
+        auto refine = [&](double q, double v) {
+            const double t = __fma_rn(__fma_rn(-q, d, v), h, q);
+            return __hiloint2double(__double2hiint(t) | (__double2hiint(q) & 0x80000000), __double2loint(t));
+        };
+        qx = refine(a, x);
+        qy = refine(b, y);
+        qz = refine(c, z);
+    } else {
+        qx = x / d;
+        qy = y / d;
+        qz = z / d;
+    }
+}
+
 // Moments.  Full f (FP64): rho = sum f and u = j / rho with three divisions,
 // as the reference rounds them (Simulation.cpp:52-175).  Offsets (FP32):
 // r = rho - 1 = sum d, u = j / (1 + r).  `r` returns rho (full) or rho - 1.
@@ -78,7 +114,7 @@ __device__ __forceinline__ void moments(const R (&f)[Q], R& r, R& ux, R& uy, R& 
         const R inv = __frcp_rn(R(1) + d);
         ux = px * inv; uy = py * inv; uz = pz * inv;
     } else {
-        ux = px / d; uy = py / d; uz = pz / d;
+        divide3(px, py, pz, d, ux, uy, uz);
     }
     r = d;
 }
@@ -95,25 +131,6 @@ __device__ __forceinline__ R feq_q(R r, R ux, R uy, R uz, R usqr) {
         return (R)Lat<Q>::w(q) * r * (R(1.0) + R(3.0) * du + R(4.5) * du * du - R(1.5) * usqr);
     }
 }
-
-template <int Q, typename R, bool OFF, int q = 0>
-__device__ __forceinline__ void relax_all(R (&f)[Q], R r, R ux, R uy, R uz, R usqr, R inv_tau) {
-    if constexpr (q < Q) {
-        const R e = feq_q<Q, q, R, OFF>(r, ux, uy, uz, usqr);
-        f[q] = f[q] + inv_tau * (e - f[q]);
-        relax_all<Q, R, OFF, q + 1>(f, r, ux, uy, uz, usqr, inv_tau);
-    }
-}
-
-template <int Q, typename R, bool OFF, int q = 0>
-__device__ __forceinline__ void feq_all(R (&e)[Q], R r, R ux, R uy, R uz) {
-    if constexpr (q < Q) {
-        const R usqr = ux * ux + uy * uy + uz * uz;
-        e[q] = feq_q<Q, q, R, OFF>(r, ux, uy, uz, usqr);
-        feq_all<Q, R, OFF, q + 1>(e, r, ux, uy, uz);
-    }
-}
-
 
 // ---------------------------------------------------------------------------
 // FP32 arithmetic on offsets, with the lattice constants folded by hand:
@@ -140,6 +157,52 @@ __device__ __forceinline__ R cdot(R x, R y, R z) {
     } else {
         return R(0);
     }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 forms.  GB300 issues two FP64 operations a cycle and SM (a warp's FP64
+// instruction takes 16 cycles), so the FP64 step is bound by their number.
+// These forms give the reference's values bit for bit with fewer of them:
+// products with a component c in {0, +-1} are signed additions (cdot: the
+// same sums, zero terms left out), and a direction pair (q, opp q) shares
+// what depends on c . u up to its sign.
+
+// Equilibrium of every direction, w rho (1 + 3cu + 4.5(cu)^2 - 1.5u^2) in
+// the reference's operation order (Simulation.cpp:183-197); u15 = 1.5 u^2.
+template <int Q, int q = 0>
+__device__ __forceinline__ void feq_pairs(double (&e)[Q], double r, double ux, double uy, double uz, double u15) {
+    if constexpr (q < Q) {
+        constexpr int o = Lat<Q>::opp(q);
+        const double wr = Lat<Q>::w(q) * r;
+        if constexpr (q == Lat<Q>::REST) {
+            e[q] = wr * (1.0 - u15);
+        } else if constexpr (q < o) {
+            const double du = cdot<Q, q, double>(ux, uy, uz);
+            const double t = 3.0 * du, s = (4.5 * du) * du;
+            e[q] = wr * (((1.0 + t) + s) - u15);
+            e[o] = wr * (((1.0 - t) + s) - u15);
+        }
+        feq_pairs<Q, q + 1>(e, r, ux, uy, uz, u15);
+    }
+}
+
+template <int Q>
+__device__ __forceinline__ void feq_all(double (&e)[Q], double r, double ux, double uy, double uz) {
+    feq_pairs<Q>(e, r, ux, uy, uz, 1.5 * (ux * ux + uy * uy + uz * uz));
+}
+
+// BGK collision: f + (feq - f) / tau (Simulation.cpp:199-205).
+template <int Q>
+__device__ __forceinline__ void relax_all(double (&f)[Q], double r, double ux, double uy, double uz, double inv_tau) {
+    double e[Q];
+    feq_all<Q>(e, r, ux, uy, uz);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) f[q] = f[q] + inv_tau * (e[q] - f[q]);
+}
+
+// v == 0.0 (either sign) without the FP64 pipe.
+__device__ __forceinline__ bool is_zero_bits(double v) {
+    return ((uint32_t)__double2loint(v) | ((uint32_t)__double2hiint(v) << 1)) == 0u;
 }
 
 // Sums of a pair relaxation: the even parts (one per pair) and, per axis,
@@ -546,45 +609,74 @@ __device__ __forceinline__ int bc_axis(const BCDev& b) {
 // ---------------------------------------------------------------------------
 // Wall shear stress.
 
-// Reference form (Simulation.cpp:880-898): literal loop nest, FP64.
-template <int Q>
-__device__ __forceinline__ void wss_reference(const double (&f)[Q], const double (&feq)[Q], const double n[3],
-                                              double C, double tau_i[3]) {
-    for (int i = 0; i < 3; ++i) {
-        double sum_alpha = 0.0;
-#pragma unroll
-        for (int al = 0; al < Q; ++al) {
-            const double c[3] = {(double)Lat<Q>::cx(al), (double)Lat<Q>::cy(al), (double)Lat<Q>::cz(al)};
-            double sum_k = 0.0;
-            for (int k = 0; k < 3; ++k) sum_k += c[k] * n[k] * n[i];
-            double sum_j = 0.0;
-            for (int j = 0; j < 3; ++j) sum_j += c[j] * n[j] * (c[i] - sum_k);
-            double f_ne = f[al] - feq[al];
-            sum_alpha += f_ne * sum_j;
+// sum_j c_j n_j (c_i - sum_k c_k n_k n_i) of component i for every direction
+// pair (it is the same for q and opp q); n_k n_i = P0, P1, P2.
+template <int Q, int i, int q = 0>
+__device__ __forceinline__ void wss_weights(double (&w)[Q], const double (&n)[3], double P0, double P1, double P2) {
+    if constexpr (q < Q) {
+        constexpr int o = Lat<Q>::opp(q);
+        if constexpr (q < o) {
+            const double d = (double)lat_c<Q>(q, i) - cdot<Q, q, double>(P0, P1, P2);
+            w[q] = w[o] = cdot<Q, q, double>(n[0] * d, n[1] * d, n[2] * d);
         }
-        tau_i[i] = C * sum_alpha;
+        wss_weights<Q, i, q + 1>(w, n, P0, P1, P2);
     }
 }
 
-// Same quantity, factored: tau_i = C sum_a f_ne (c.n)(c_i - (c.n) n_i), with
-// the equilibrium of moments (r, u) evaluated inside the loop.
-template <int Q, typename R, bool OFF>
-__device__ __forceinline__ void wss_fast(const R (&f)[Q], R r, R ux, R uy, R uz, const R n[3], R C, R tau_i[3]) {
-    const R usqr = ux * ux + uy * uy + uz * uz;
-    R a0 = R(0), a1 = R(0), a2 = R(0);
+template <int Q, int i>
+__device__ __forceinline__ double wss_component(const double (&ne)[Q], const double (&n)[3], double C) {
+    double w[Q];
+    wss_weights<Q, i>(w, n, n[0] * n[i], n[1] * n[i], n[2] * n[i]);
+    double s = 0.0;
 #pragma unroll
-    for (int al = 0; al < Q; ++al) {
-        const R cx = (R)Lat<Q>::cx(al), cy = (R)Lat<Q>::cy(al), cz = (R)Lat<Q>::cz(al);
-        const R du = ux * cx + uy * cy + uz * cz;
-        const R e = OFF ? (R)Lat<Q>::w(al) * (r + (R(1) + r) * (R(3.0) * du + R(4.5) * du * du - R(1.5) * usqr))
-                        : (R)Lat<Q>::w(al) * r * (R(1.0) + R(3.0) * du + R(4.5) * du * du - R(1.5) * usqr);
-        const R cn = cx * n[0] + cy * n[1] + cz * n[2];
-        const R k = (f[al] - e) * cn;
-        a0 += k * (cx - cn * n[0]);
-        a1 += k * (cy - cn * n[1]);
-        a2 += k * (cz - cn * n[2]);
-    }
-    tau_i[0] = C * a0; tau_i[1] = C * a1; tau_i[2] = C * a2;
+    for (int al = 0; al < Q; ++al)
+        if (al != Lat<Q>::REST) s += ne[al] * w[al];
+    return C * s;
+}
+
+// Reference form (Simulation.cpp:880-898), FP64: the sum over the directions
+// in the reference's order with its factors (wss_weights), ne = f - feq.
+template <int Q>
+__device__ __forceinline__ void wss_reference(const double (&ne)[Q], const double (&n)[3], double C,
+                                              double (&tau_i)[3]) {
+    tau_i[0] = wss_component<Q, 0>(ne, n, C);
+    tau_i[1] = wss_component<Q, 1>(ne, n, C);
+    tau_i[2] = wss_component<Q, 2>(ne, n, C);
+}
+
+// Same quantity, factored (FP64 physics mode): Pi = sum ne c c from the pair
+// sums of ne, tau = C (Pi n - (n.Pi n) n).
+template <int Q>
+__device__ __forceinline__ void wss_fast(const double (&ne)[Q], const double (&n)[3], double C, double (&tau_i)[3]) {
+    double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    second_moments<Q, 0, double>(ne, m);
+    const double px = m[0] * n[0] + m[3] * n[1] + m[4] * n[2];
+    const double py = m[3] * n[0] + m[1] * n[1] + m[5] * n[2];
+    const double pz = m[4] * n[0] + m[5] * n[1] + m[2] * n[2];
+    const double nn = px * n[0] + py * n[1] + pz * n[2];
+    tau_i[0] = C * (px - nn * n[0]);
+    tau_i[1] = C * (py - nn * n[1]);
+    tau_i[2] = C * (pz - nn * n[2]);
+}
+
+// FP64 wall shear stress of next-to-wall node nw from its post-boundary f;
+// (r, u): the moments the equilibrium is taken at.
+template <int Q, int MODE>
+__device__ __forceinline__ void wss_f64(const StepParams& P, int64_t nw, const double (&f)[Q], double r, double ux,
+                                        double uy, double uz) {
+    const double n[3] = {P.nw_n[nw], P.nw_n[P.nnw + nw], P.nw_n[2 * P.nnw + nw]};
+    double ne[Q], t[3];
+    feq_all<Q>(ne, r, ux, uy, uz);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) ne[q] = f[q] - ne[q];
+    if constexpr (MODE == MODE_PARITY) wss_reference<Q>(ne, n, P.wss_C, t);
+    else wss_fast<Q>(ne, n, P.wss_phys, t);
+    const double W = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+    P.nw_wss[nw] = W;
+    P.nw_acc[nw] += t[0];
+    P.nw_acc[P.nnw + nw] += t[1];
+    P.nw_acc[2 * P.nnw + nw] += t[2];
+    P.nw_accm[nw] += W;
 }
 
 // Compensated accumulation in two floats (Neumaier): acc.x carries the sum,
@@ -665,7 +757,8 @@ __device__ __forceinline__ double full_value(R v, int q) {
 // f* == 0.0 in the arithmetic's own representation.
 template <int Q, typename R, bool OFF>
 __device__ __forceinline__ bool is_exact_zero(R v, int q) {
-    return OFF ? (v == -(R)Lat<Q>::w(q)) : (v == R(0));
+    if constexpr (OFF) return v == -(R)Lat<Q>::w(q);
+    else return is_zero_bits(v);
 }
 
 // ---------------------------------------------------------------------------
@@ -688,7 +781,9 @@ __device__ __forceinline__ bool word_nw(uint64_t w) { return (w >> 63) & 1ull; }
 // After the pull: boundary rules, wall shear stress, collision and store
 // (or the read-out sums) of node a with post-stream populations g.  nr and
 // slot: the next-to-wall normal and stress-ring slot (FP32 formats).
-template <int Q, typename S, int MODE, int KIND, bool WIDE>
+// STRESS false: the FP64 flat step, whose stress is computed by blocks of
+// next-to-wall nodes (stress_blocks_work).
+template <int Q, typename S, int MODE, int KIND, bool WIDE, bool STRESS = true>
 __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a, const uint64_t word,
                                             const int64_t s, const bool lng, const int c, const uint32_t miss,
                                             typename Store<S>::real (&g)[Q], const float (&nr)[3], const int slot,
@@ -714,7 +809,7 @@ __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a
     int nw = -1;  // next-to-wall index: boundary-list entries below nnw
     if (lng) {
         // ---- boundary-list node: history, boundary rules
-        R* __restrict__ stale = static_cast<R*>(P.stale);
+        const R* __restrict__ stale = static_cast<const R*>(P.stale_in);
         if constexpr (MODE == MODE_PARITY) {
             if (parity_readout) {
                 // the boundary list keeps the exact post-boundary f of the last step
@@ -803,26 +898,14 @@ __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a
         float jx = 0.f, jy = 0.f, jz = 0.f;  // momentum of g (FP32 offsets: the collision invariants)
         if constexpr (OFF && !SC) momentum<Q, float>(g, jx, jy, jz);
         R* __restrict__ prev = static_cast<R*>(P.nw_prev);
-        if (KIND == KIND_STEP && nw >= 0) {
+        if (STRESS && KIND == KIND_STEP && nw >= 0) {
             if constexpr (!OFF) {
-                // FP64: the reference's arithmetic
-                double t[3];
-                const double nn[3] = {P.nw_n[nw], P.nw_n[P.nnw + nw], P.nw_n[2 * P.nnw + nw]};
-                if constexpr (MODE == MODE_PARITY) {
-                    // equilibrium of the previous collision (time-lagged, as the reference)
-                    double e[Q];
-                    feq_all<Q, double, false>(e, prev[nw], prev[P.nnw + nw], prev[2 * P.nnw + nw],
-                                              prev[3 * P.nnw + nw]);
-                    wss_reference<Q>(g, e, nn, P.wss_C, t);
-                } else {
-                    wss_fast<Q, double, false>(g, r, ux, uy, uz, nn, P.wss_phys, t);
-                }
-                const double W = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
-                P.nw_wss[nw] = W;
-                P.nw_acc[nw] += t[0];
-                P.nw_acc[P.nnw + nw] += t[1];
-                P.nw_acc[2 * P.nnw + nw] += t[2];
-                P.nw_accm[nw] += W;
+                // FP64: the reference's arithmetic; parity: equilibrium of the
+                // previous collision (time-lagged, as the reference)
+                if constexpr (MODE == MODE_PARITY)
+                    wss_f64<Q, MODE>(P, nw, g, prev[nw], prev[P.nnw + nw], prev[2 * P.nnw + nw], prev[3 * P.nnw + nw]);
+                else
+                    wss_f64<Q, MODE>(P, nw, g, r, ux, uy, uz);
             } else {
                 // FP32 arithmetic end to end
                 float t[4];
@@ -849,7 +932,7 @@ __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a
                 R* __restrict__ stale = static_cast<R*>(P.stale);
 #pragma unroll
                 for (int q = 0; q < Q; ++q) stale[q * P.nsp + s] = g[q];
-                if (nw >= 0) {
+                if ((STRESS || KIND != KIND_STEP) && nw >= 0) {
                     // moments of this step's collision, for the next step's lagged stress
                     prev[nw] = r; prev[P.nnw + nw] = ux; prev[2 * P.nnw + nw] = uy; prev[3 * P.nnw + nw] = uz;
                 }
@@ -887,7 +970,7 @@ __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a
             relax_pairs<Q>(g, A, B, ux, uy, uz, om, om1, ps);
             close_invariants<Q>(g, ps, om1, r, jx, jy, jz);
         } else {
-            relax_all<Q, R, OFF>(g, r, ux, uy, uz, ux * ux + uy * uy + uz * uz, (R)P.inv_tau);
+            relax_all<Q>(g, r, ux, uy, uz, P.inv_tau);
         }
         if (!(fabsf((float)r) < 1e30f)) atomicOr(P.flags, FLAG_NONFINITE);
         S* __restrict__ fout_a = fout + ai;
@@ -1023,13 +1106,58 @@ __device__ __forceinline__ void pull_node(const StepParams& P, const int64_t a, 
 
 // One node's update: pull, boundary rules, wall shear stress, collision and
 // store (or the read-out sums).
-template <int Q, typename S, int MODE, int KIND, bool WIDE, bool WALLS = false, bool CG = false>
+template <int Q, typename S, int MODE, int KIND, bool WIDE, bool WALLS = false, bool CG = false, bool STRESS = true>
 __device__ __forceinline__ void node_update(const StepParams& P, const int64_t a, const uint64_t word,
                                             const int32_t sp_entry, double (&part)[kPartialStride]) {
     typename Store<S>::real g[Q];
     Pulled pl;
     pull_node<Q, S, MODE, KIND, WIDE, WALLS, CG>(P, a, word, sp_entry, g, pl);
-    node_finish<Q, S, MODE, KIND, WIDE>(P, a, word, pl.s, pl.lng, pl.c, pl.miss, g, pl.nr, pl.slot, part);
+    node_finish<Q, S, MODE, KIND, WIDE, STRESS>(P, a, word, pl.s, pl.lng, pl.c, pl.miss, g, pl.nr, pl.slot, part);
+}
+
+// FP64 wall shear stress off the nodes' own threads (flat launches).
+// 11-40% of a vessel's nodes lie next to the wall, at the ends of its
+// x-runs, so that nearly every warp holds some: in the nodes' threads the
+// stress, more FP64 operations than the rest of the node together, cost
+// every warp.  Leading blocks of the step's own launch do it with full warps
+// instead: they pull the next-to-wall nodes' populations once more (interior
+// fluid nodes: every source is active, no boundary rule) from the input
+// planes, which the launch does not write.  Parity mode: the equilibrium is
+// that of the previous collision, whose moments (`prev`) only these blocks
+// read and replace.  65k nodes, D3Q19, parity: 181 us a step with the
+// reference's sums in the nodes' threads, 68 us with a second launch over
+// the next-to-wall nodes, 52 us with these blocks and the forms above.
+template <int Q, int MODE, bool WIDE>
+__device__ __forceinline__ void stress_blocks_work(const StepParams& P, int64_t block, int bt) {
+    using I = typename std::conditional<WIDE, int64_t, int32_t>::type;
+    const int64_t nw = block * bt + threadIdx.x;
+    if (nw >= P.nnw) return;
+    const int64_t a = P.act_idx[P.nw_pt[nw]];
+    if (!in_bounds(a, P.nact, P.flags)) return;
+    const int64_t seg = word_segment(__ldg(P.act_word + a));
+    if (!in_bounds(seg, P.nseg, P.flags)) return;
+    const int32_t* __restrict__ row = P.seg_delta + seg * kDeltaRow<Q>;
+    const double* __restrict__ fin = static_cast<const double*>(P.fin) + (I)a;
+    double g[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const I off = (I)q * (I)P.stride + (q == Lat<Q>::REST ? 0 : __ldg(row + q));
+        g[q] = in_bounds(a + (int64_t)off, (int64_t)Q * P.stride, P.flags) ? fin[off] : 0.0;
+    }
+    double r, ux, uy, uz;
+    if constexpr (MODE == MODE_PARITY) {
+        const double* __restrict__ stale = static_cast<const double*>(P.stale_in);
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (is_zero_bits(g[q])) g[q] = stale[q * P.nsp + nw];  // an exact zero is not streamed
+        double* __restrict__ prev = static_cast<double*>(P.nw_prev);
+        wss_f64<Q, MODE>(P, nw, g, prev[nw], prev[P.nnw + nw], prev[2 * P.nnw + nw], prev[3 * P.nnw + nw]);
+        moments<Q, double, false>(g, r, ux, uy, uz);
+        prev[nw] = r; prev[P.nnw + nw] = ux; prev[2 * P.nnw + nw] = uy; prev[3 * P.nnw + nw] = uz;
+    } else {
+        moments<Q, double, false>(g, r, ux, uy, uz);
+        wss_f64<Q, MODE>(P, nw, g, r, ux, uy, uz);
+    }
 }
 
 // Programmatic dependent launch: a step kernel is launched with
@@ -1060,12 +1188,14 @@ __global__ void __launch_bounds__(BT, MINB) step_kernel(const StepParams P) {
     int64_t blk = blockIdx.x;
     if constexpr (KIND == KIND_STEP) {
         if (P.pdl_early) pdl_trigger();
-        if constexpr (Store<S>::offset) {
-            // leading blocks: the stress ring's fold (FP32-arithmetic formats)
+        {
+            // leading blocks: the stress ring's fold (FP32-arithmetic
+            // formats), the next-to-wall nodes' stress (FP64)
             if (blk < P.fold_blocks) {
                 pdl_wait();
                 if (blockIdx.x == 0 && threadIdx.x == 0) *P.step_next = *P.step_base + 1;
-                fold_blocks_work(P, blk, BT);
+                if constexpr (Store<S>::offset) fold_blocks_work(P, blk, BT);
+                else stress_blocks_work<Q, MODE, WIDE>(P, blk, BT);
                 if (!P.pdl_early) pdl_trigger();
                 return;
             }
@@ -1095,7 +1225,8 @@ __global__ void __launch_bounds__(BT, MINB) step_kernel(const StepParams P) {
         // block 0 is a node block when there are no fold blocks
         if (blockIdx.x == 0 && threadIdx.x == 0) *P.step_next = *P.step_base + 1;
     }
-    if (a < P.nact) node_update<Q, S, MODE, KIND, WIDE, WALLS>(P, a, word, sp_entry, part);
+    constexpr bool STRESS = Store<S>::offset || KIND != KIND_STEP;
+    if (a < P.nact) node_update<Q, S, MODE, KIND, WIDE, WALLS, false, STRESS>(P, a, word, sp_entry, part);
     if constexpr (KIND == KIND_STEP) {
         if (!P.pdl_early) pdl_trigger();
     }
@@ -1222,6 +1353,14 @@ struct Variant {
 };
 constexpr int kFlatVariants = 5;  // 0..4; 5 = tiled
 constexpr Variant kVariants[kFlatVariants] = {{128, 12}, {128, 10}, {128, 8}, {256, 3}, {256, 1}};
+// Variant 4 in FP64 (its default; 128 registers): the FP64 pipe is shared by the SM's warps,
+// so an SM's time is its number of warps; blocks of two warps spread a small
+// lattice evenly (65k nodes over 152 SMs: 14 warps on the fullest SM, 16
+// with blocks of eight).
+template <typename S, int V>
+constexpr Variant variant_shape() {
+    return V == 4 && std::is_same<S, double>::value ? Variant{64, 8} : kVariants[V];
+}
 
 // A step-kernel launch with programmatic stream serialization (see
 // pdl_trigger / pdl_wait); minb: the kernel's minimum resident blocks per SM.
@@ -1258,14 +1397,14 @@ inline cudaError_t launch_dependent(void (*kern)(const StepParams), int64_t nblo
 
 template <int Q, typename S, int MODE, int V>
 cudaError_t launch_step_variant(const StepParams& p, cudaStream_t st) {
-    constexpr int BT = kVariants[V].bt, MB = kVariants[V].minb;
+    constexpr int BT = variant_shape<S, V>().bt, MB = variant_shape<S, V>().minb;
     const bool narrow = (int64_t)Q * p.stride < ((int64_t)1 << 31);
     const int bt = narrow ? BT : kStepThreads;  // beyond 32-bit offsets: one 64-bit shape for every variant
     constexpr bool PHYS = MODE == MODE_PHYSICS;
     const bool walls = PHYS && p.sp_q != nullptr;  // interpolated bounce-back: one shape, (128, 8)
     const int bw = walls && narrow ? 128 : bt;
     StepParams q = p;
-    q.fold_blocks = Store<S>::offset ? ceil_div(p.nnw, (int64_t)bw * kFoldNodes) : 0;
+    q.fold_blocks = ceil_div(p.nnw, (int64_t)bw * (Store<S>::offset ? kFoldNodes : 1));
     const int64_t nblocks = q.fold_blocks + ceil_div(p.nact, bw);
     if (ceil_div(p.nact, bw) <= 0) return cudaSuccess;
     if (nblocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
