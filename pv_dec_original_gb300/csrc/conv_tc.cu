@@ -1,47 +1,37 @@
 // 3x3x3 convolutions (padding 1, stride 1 or 2) of the warm-start network
 // on the fifth-generation tensor cores: tcgen05.mma with the accumulators in
-// tensor memory.  No reference counterpart (the reference always starts
-// from rest).
+// tensor memory; and the weight gradients.  No reference counterpart (the
+// reference always starts from rest).
 //
-// One CTA (4 warps) computes an output block of 8 (x) x 16 (y) x TZ (z)
-// voxels (TZ = 4 at stride 1, 1 at stride 2) and all co output channels.
-// Per 16-channel chunk of the input it stages the input voxels the block
-// reads (the block plus its one-voxel halo, 10 x 18 x 6 at stride 1;
-// 17 x 33 x 3 at stride 2) with tensor-memory-access copies
-// (cp.async.bulk.tensor, one per channel half and x parity, zero-filled
-// outside the grid: the padding; at stride 2 an element stride of 2 along x
-// picks one parity) completing on an mbarrier, and the chunk of all 27
-// taps' weights with cp.async, in the canonical no-swizzle K-major layout
-// of the MMA operands: core matrices of 8 rows x 16 bytes (8 channels),
-// rows 16 bytes apart.
+// A CTA computes output blocks of 8 (x) x 16 (y) x TZ (z) voxels (TZ = 4 at
+// stride 1, 1 at stride 2) and all co output channels.  Per 16-channel chunk
+// of the input it stages the input voxels the block reads (the block plus
+// its one-voxel halo, 10 x 18 x 6 at stride 1; 17 x 33 x 3 at stride 2),
+// zero outside the grid (the padding), and the chunk of all 27 taps'
+// weights, in the canonical no-swizzle K-major layout of the MMA operands:
+// core matrices of 8 rows x 16 bytes (8 channels), rows 16 bytes apart.
 //   input:   [channel half k (2)][x parity p (S)][z][y][x / S][8 channels]
-//            (a parity plane padded to 128 bytes)
 //   weights: [tap block][co / 8][channel half k][co % 8][8 channels]
-//            (tap block: weight_block)
+//            (stride 1: blocks in weight_block's order)
 // The 128 output voxels of one z plane (8 x by 16 y) are the M = 128 rows
 // of one MMA: row m = 8 y + x.  Output x reads input x = S x + tx - 1, so
 // with the input's x split by parity (stride 2: even and odd columns in
 // separate runs) rows m..m+7 are 8 consecutive staged voxels -- one core
 // matrix -- and the 16 groups of 8 rows are 16 output rows, S input rows
 // apart: the stride-dimension offset.  The two channel halves of the K = 16
-// slice are one staged block apart: the leading-dimension offset.  A tap
+// slice are one staged half apart: the leading-dimension offset.  A tap
 // (tx, ty, tz) is just the descriptor's start address (parity tx mod S,
 // column tx / S, row ty, plane S z + tz): the 27 taps reuse the staged block
-// with no copies.  One elected thread issues the MMAs of a chunk (M = 128,
-// K = 16, BF16 x BF16 -> FP32) into TZ accumulators of co tensor-memory
-// columns each and commits them to an mbarrier; every wait is bounded.  At
-// stride 2: TZ x 27 MMAs of N = co.  At stride 1 the accumulators of the
-// TZ planes are adjacent column ranges and one staged plane feeds up to
-// three output planes (through taps tz = 2, 1, 0), so each (ty, tx) takes
-// one MMA per staged plane with N = 1-3 co: 9 x 6 = 54 MMAs instead of
-// 4 x 27, each reading its A operand once.  The epilogue reads the
-// accumulators with tcgen05.ld (warp w owns tensor-memory lanes 32 w ..
-// 32 w + 31, i.e. rows y = 4 w .. 4 w + 3), adds the bias, applies ReLU and
-// stores BF16 (and FP32 when asked) channels-last.
-//
-// Bound: the A operand (the staged input, 4 KB per MMA) is read from shared
-// memory by every MMA; at co = 16 that operand traffic, not the tensor
-// pipe, sets the rate (see the convolution profile).
+// with no copies.  One thread issues the MMAs of a chunk (M = 128, K = 16,
+// BF16 x BF16 -> FP32) into TZ accumulators of co tensor-memory columns each
+// and commits them to an mbarrier; every wait is bounded.  At stride 2: 27
+// MMAs of N = co.  At stride 1 the accumulators of the TZ planes are adjacent
+// column ranges and one staged plane feeds up to three output planes (through
+// taps tz = 2, 1, 0), so each (ty, tx) takes one MMA per staged plane with
+// N = 1-3 co: 9 x 6 = 54 MMAs instead of 4 x 27, each reading its A operand
+// once.  The epilogue reads the accumulators with tcgen05.ld (warp w owns
+// tensor-memory lanes 32 w .. 32 w + 31, i.e. rows y = 4 w .. 4 w + 3), adds
+// the bias, applies ReLU and stores BF16 (and FP32 when asked) channels-last.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -58,20 +48,15 @@ constexpr int TX = 8, TY = 16;
 constexpr int kThreads = 128;
 constexpr long kWaitLimit = 1L << 20;  // mbarrier polls (each bounded by the hardware's own time limit)
 
-// Staged geometry per stride: output planes per CTA, staged planes, rows,
-// x parities and voxels per parity run.
-template <int S>
-struct Geo {
-    static constexpr int TZ = S == 1 ? 4 : 1;
-    static constexpr int ZB = S * (TZ - 1) + 3;
-    static constexpr int YB = S * (TY - 1) + 3;
-    static constexpr int PAR = S;
-    static constexpr int XH = S == 1 ? TX + 2 : TX + 1;        // stride 2: input x = 2 xh + p, rows 0..16
-    static constexpr int PLANE_RAW = ZB * YB * XH * 16;         // bytes one copy writes (17,280 / 14,256)
+// Staged geometry at stride 2: planes, rows, and voxels per x parity run
+// (input x = 2 xh + p).
+struct Geo2 {
+    static constexpr int ZB = 3, YB = 2 * (TY - 1) + 3, XH = TX + 1;
+    static constexpr int PLANE_RAW = ZB * YB * XH * 16;          // bytes one copy writes
     static constexpr int PLANE = (PLANE_RAW + 127) / 128 * 128;  // copy destinations 128-byte aligned
-    static constexpr int HALF = PAR * PLANE;                     // bytes of one channel half
+    static constexpr int HALF = 2 * PLANE;                       // bytes of one channel half
     static constexpr int TILE = 2 * HALF;
-    static constexpr int TX_BYTES = 2 * PAR * PLANE_RAW;         // bytes the copies of a chunk deliver
+    static constexpr int TX_BYTES = 4 * PLANE_RAW;               // bytes the copies of a chunk deliver
 };
 
 // Set when a bounded wait gave up (read and cleared by conv_tc_status).
@@ -102,16 +87,19 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (long k = 0; k < kWaitLimit; ++k) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
+    for (long k = 0; k < kWaitLimit; ++k)
+        if (mbar_try(bar, parity)) return true;
     return false;
 }
 
@@ -151,37 +139,66 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
-template <int S, int CO>
+// 16 channels (c16) of output voxel vox from their FP32 sums: bias, ReLU, BF16 (and FP32) store.
+template <int CO>
+__device__ __forceinline__ void store16(float (&v)[16], const float* __restrict__ bias, int relu, bf16* __restrict__ y,
+                                        float* __restrict__ y32, int64_t vox, int c16) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        v[k] += bias ? bias[c16 * 16 + k] : 0.f;
+        if (relu) v[k] = fmaxf(v[k], 0.f);
+    }
+    uint4 p[2];
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(p);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+    uint4* dst = reinterpret_cast<uint4*>(y + vox * CO + c16 * 16);
+    dst[0] = p[0];
+    dst[1] = p[1];
+    if (y32) {
+        float4* d32 = reinterpret_cast<float4*>(y32 + vox * CO + c16 * 16);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    }
+}
+
+// Shared-memory block of tap t = 9 tz + 3 ty + tx in the weights staged at
+// stride 1: the three z taps of each (ty, tx) in the order tz = 2, 1, 0, so
+// that one MMA of N = 3 co takes all three: staged plane zz feeds output
+// planes zz - 2, zz - 1, zz through taps tz = 2, 1, 0, and the accumulators
+// of those planes are the adjacent tensor-memory column ranges (z co .. z co
+// + co - 1 for plane z).
+__host__ __device__ constexpr int weight_block(int t) { return ((t / 3) % 3 * 3 + t % 3) * 3 + (2 - t / 9); }
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+template <int CO>
 __host__ __device__ constexpr int smem_bytes() {
-    return Geo<S>::TILE + 27 * CO * 32 + 32;  // input, weights, two mbarriers + tensor-memory address
+    return Geo2::TILE + 27 * CO * 32 + 32;  // input, weights, two mbarriers + tensor-memory address
 }
 
-template <int S, int CO>
+template <int CO>
 __host__ __device__ constexpr uint32_t tmem_cols() {
-    return Geo<S>::TZ * CO < 32 ? 32u : (uint32_t)(Geo<S>::TZ * CO);  // a power of two for CO in {16, 32, 64}
+    return CO < 32 ? 32u : (uint32_t)CO;  // a power of two for CO in {16, 32, 64}
 }
 
-// Shared-memory block of tap t = 9 tz + 3 ty + tx in the staged weights.
-// Stride 1 groups the three z taps of each (ty, tx) in the order tz = 2, 1,
-// 0, so that one MMA of N = 3 co takes all three: staged plane zz feeds
-// output planes zz - 2, zz - 1, zz through taps tz = 2, 1, 0, and the
-// accumulators of those planes are the adjacent tensor-memory column
-// ranges (z co .. z co + co - 1 for plane z).  Stride 2 keeps tap order.
-template <int S>
-__host__ __device__ constexpr int weight_block(int t) {
-    return S == 1 ? ((t / 3) % 3 * 3 + t % 3) * 3 + (2 - t / 9) : t;
-}
-
-// x [Di][Hi][Wi][ci] (read through `map`: the 4-D tensor map of x, box
-// 8 channels x (XH, or 2 XH with element stride 2) x YB x ZB), w [co][27][ci],
-// y [Do][Ho][Wo][co] with Do = Di / S etc.; Do % TZ == 0, Ho % 16 == 0,
-// Wo % 8 == 0 (the launcher checks).
-template <int S, int CO>
-__global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ CUtensorMap map,
-                                                       const bf16* __restrict__ w, const float* __restrict__ bias,
-                                                       bf16* __restrict__ y, float* __restrict__ y32, int Do, int Ho,
-                                                       int Wo, int ci, int relu) {
-    using G = Geo<S>;
+// Stride 2.  x [Di][Hi][Wi][ci] (read through `map`: the 4-D tensor map of x,
+// box 8 channels x 2 XH with element stride 2 x YB x ZB), w [co][27][ci],
+// y [Do][Ho][Wo][co] with Do = Di / 2 etc.; Ho % 16 == 0, Wo % 8 == 0 (the
+// launcher checks).  The input by tensor copies (one per channel half and x
+// parity, element stride 2 along x), the weights by cp.async.
+template <int CO>
+__global__ void __launch_bounds__(kThreads) k_conv3_s2_tc(const __grid_constant__ CUtensorMap map,
+                                                          const bf16* __restrict__ w, const float* __restrict__ bias,
+                                                          bf16* __restrict__ y, float* __restrict__ y32, int Do, int Ho,
+                                                          int Wo, int ci, int relu) {
+    using G = Geo2;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* tile = smem;
     unsigned char* wsm = smem + G::TILE;
@@ -190,9 +207,9 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
     volatile int& copy_failed = *reinterpret_cast<volatile int*>(tslot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nbx = Wo / TX, nby = Ho / TY;
-    const int bx = blockIdx.x % nbx, by = (blockIdx.x / nbx) % nby, bz = blockIdx.x / (nbx * nby);
-    const int x0 = bx * TX, y0 = by * TY, z0 = bz * G::TZ;
-    constexpr uint32_t NCOL = tmem_cols<S, CO>();
+    const int bx = blockIdx.x % nbx, by = (blockIdx.x / nbx) % nby, z0 = blockIdx.x / (nbx * nby);
+    const int x0 = bx * TX, y0 = by * TY;
+    constexpr uint32_t NCOL = tmem_cols<CO>();
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tslot)),
@@ -213,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
 
     const uint32_t tile_a = saddr(tile), w_a = saddr(wsm);
     constexpr uint32_t IDESC = idesc_bf16(128, CO);
-    constexpr uint32_t SBO = S * G::XH * 16;  // S input rows per output row
+    constexpr uint32_t SBO = 2 * G::XH * 16;  // two input rows per output row
     bool ok = true;
     const int chunks = ci / 16;
     int c = 0;
@@ -222,14 +239,14 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
         if (tid == 0) {
             mbar_expect_tx(saddr(bar + 1), (uint32_t)G::TX_BYTES);
             for (int k = 0; k < 2; ++k)
-                for (int p = 0; p < G::PAR; ++p)
-                    tma_load4(tile_a + k * G::HALF + p * G::PLANE, &map, c * 16 + k * 8, S * x0 - 1 + p,
-                              S * y0 - 1, S * z0 - 1, saddr(bar + 1));
+                for (int p = 0; p < 2; ++p)
+                    tma_load4(tile_a + k * G::HALF + p * G::PLANE, &map, c * 16 + k * 8, 2 * x0 - 1 + p, 2 * y0 - 1,
+                              2 * z0 - 1, saddr(bar + 1));
         }
         // the weights of this chunk
         for (int i = tid; i < 27 * CO * 2; i += kThreads) {
             const int k = i & 1, n = (i >> 1) % CO, t = (i >> 1) / CO;
-            cp_async16(w_a + weight_block<S>(t) * (CO * 32) + (n >> 3) * 256 + k * 128 + (n & 7) * 16,
+            cp_async16(w_a + t * (CO * 32) + (n >> 3) * 256 + k * 128 + (n & 7) * 16,
                        w + ((int64_t)n * 27 + t) * ci + c * 16 + k * 8, true);
         }
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
@@ -238,46 +255,13 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
         if (tid == 0) {
             if (mbar_wait(saddr(bar + 1), (uint32_t)(c & 1))) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if constexpr (S == 1) {
-                    // per (ty, tx): one MMA per staged plane zz, into output
-                    // planes lo .. hi - 1 (N = (hi - lo) co) with the taps
-                    // tz = zz - lo .. zz - hi + 1 (weight_block); 54 MMAs
-                    // instead of 108, each reading its A operand once.  The
-                    // first (ty, tx) of the first chunk starts with planes 2
-                    // and 5, whose output ranges (0..2 and 3) cover every
-                    // accumulator once: they initialise it.
-                    static_assert(G::TZ == 4 && G::ZB == 6, "merged z taps: 4 output planes, 6 staged");
-                    constexpr int kOrder[6] = {2, 5, 0, 1, 3, 4};
-                    constexpr uint32_t ID1 = idesc_bf16(128, CO), ID2 = idesc_bf16(128, 2 * CO),
-                                       ID3 = idesc_bf16(128, 3 * CO);
-                    for (int u = 0; u < 9; ++u) {
-                        const int ty = u / 3, tx = u % 3;
-                        for (int j = 0; j < 6; ++j) {
-                            const int zz = kOrder[j];
-                            const int lo = zz > 2 ? zz - 2 : 0, hi = zz + 1 < G::TZ ? zz + 1 : G::TZ;
-                            const int np = hi - lo, b0 = 2 - (zz - lo);
-                            const uint32_t a = tile_a + ((zz * G::YB + ty) * G::XH + tx) * 16;
-                            const uint64_t ad = smem_desc(a, G::HALF, SBO);
-                            const uint64_t bd = smem_desc(w_a + (u * 3 + b0) * (CO * 32), 128, 256);
-                            mma_bf16(tmem + (uint32_t)(lo * CO), ad, bd, np == 3 ? ID3 : (np == 2 ? ID2 : ID1),
-                                     (c > 0 || u > 0 || j >= 2) ? 1u : 0u);
-                        }
-                    }
-                } else {
-                    for (int z = 0; z < G::TZ; ++z) {
-                        for (int t = 0; t < 27; ++t) {
-                            const int tz = t / 9, ty = (t / 3) % 3, tx = t % 3;
-                            const int zz = S * z + tz, p = tx % S, xo = tx / S;
-                            const uint32_t a = tile_a + p * G::PLANE + ((zz * G::YB + ty) * G::XH + xo) * 16;
-                            const uint64_t ad = smem_desc(a, G::HALF, SBO);
-                            const uint64_t bd = smem_desc(w_a + weight_block<S>(t) * (CO * 32), 128, 256);
-                            mma_bf16(tmem + (uint32_t)(z * CO), ad, bd, IDESC, (c > 0 || t > 0) ? 1u : 0u);
-                        }
-                    }
+                for (int t = 0; t < 27; ++t) {
+                    const int tz = t / 9, ty = (t / 3) % 3, tx = t % 3;
+                    const uint32_t a = tile_a + (tx & 1) * G::PLANE + ((tz * G::YB + ty) * G::XH + tx / 2) * 16;
+                    mma_bf16(tmem, smem_desc(a, G::HALF, SBO), smem_desc(w_a + t * (CO * 32), 128, 256), IDESC,
+                             (c > 0 || t > 0) ? 1u : 0u);
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 saddr(bar))
-                             : "memory");
+                tc_commit(saddr(bar));
             } else {
                 copy_failed = 1;
             }
@@ -302,31 +286,12 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
     if (ok) {
         // epilogue: warp w reads lanes 32 w .. 32 w + 31 = rows y = 4 w + lane / 8, x = lane % 8
         const int m = 32 * warp + lane;
-        const int gx = x0 + (m & 7), gy = y0 + (m >> 3);
-        for (int z = 0; z < G::TZ; ++z) {
-            const int64_t vox = ((int64_t)(z0 + z) * Ho + gy) * Wo + gx;
+        const int64_t vox = ((int64_t)z0 * Ho + y0 + (m >> 3)) * Wo + x0 + (m & 7);
 #pragma unroll
-            for (int c16 = 0; c16 < CO / 16; ++c16) {
-                float v[16];
-                tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(z * CO + c16 * 16), v);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    v[k] += bias ? bias[c16 * 16 + k] : 0.f;
-                    if (relu) v[k] = fmaxf(v[k], 0.f);
-                }
-                uint4 p[2];
-                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(p);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) h[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-                uint4* dst = reinterpret_cast<uint4*>(y + vox * CO + c16 * 16);
-                dst[0] = p[0];
-                dst[1] = p[1];
-                if (y32) {
-                    float4* d32 = reinterpret_cast<float4*>(y32 + vox * CO + c16 * 16);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-                }
-            }
+        for (int c16 = 0; c16 < CO / 16; ++c16) {
+            float v[16];
+            tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(c16 * 16), v);
+            store16<CO>(v, bias, relu, y, y32, vox, c16);
         }
     } else if (c > 0) {
         // the wait of chunk c - 1 gave up: record it, wait (bounded) once
@@ -334,6 +299,221 @@ __global__ void __launch_bounds__(kThreads) k_conv3_tc(const __grid_constant__ C
         if (tid == 0) atomicOr(&g_conv_tc_flags, 1u);
         mbar_wait(saddr(bar), (uint32_t)((c - 1) & 1));
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Stride 1 (forward, and the input gradient with flipped weights), any grid.
+// The same block (8 x 16 x 4 outputs), staged layout and MMAs as described
+// at the top, in one persistent CTA an SM whose warps each do one thing:
+//   warps 0-3  epilogue: tensor memory -> bias, ReLU -> global memory
+//   warp 4     one thread issues the MMAs
+//   warps 5-8  producers: the block's input voxels (16 channels) into the
+//              next of NS stages by cp.async, zero outside the grid
+// so the copies of later blocks and the stores of the previous one run
+// beside the current one's MMAs (two sets of accumulators), and the weights
+// are staged once per CTA where they fit (WRES; 64 -> 64 channels: with each
+// stage).  mbarriers hand over the stages (full / empty) and accumulators
+// (tfull / tempty); every wait is bounded, and a role that gives up raises
+// the flag and leaves, whereupon the others' waits run out.
+//
+// What bounds it: an MMA reads its 4 KB of A from shared memory (32 cycles;
+// 54 a chunk) and, from 32 channels on, its N columns.  The kernel before
+// staged with tensor copies, whose 8-channel layout is boxes of 16-byte
+// rows: 2160 a chunk at about 3 cycles each, 7.2k cycles a chunk whatever
+// its MMAs (16 -> 16: 2.4k).  The same bytes by cp.async are 68 warp
+// instructions.
+constexpr int kPipeZ = 4;                                  // output planes of a block
+constexpr int kPipeVox = (kPipeZ + 2) * 18 * 10;           // staged voxels of a block
+constexpr int kPipeHalf = kPipeVox * 16 + 64;              // bytes of an 8-channel half (+64: the halves in different banks)
+constexpr int kPipeTile = 2 * kPipeHalf;
+constexpr int kProducers = 128;
+constexpr int kPipeThreads = 32 * (4 + 1) + kProducers;
+constexpr int kPipeBars = 256;                             // bytes for barriers and the tensor-memory address
+
+template <int CO, bool WRES>
+__host__ __device__ constexpr int pipe_stage() { return kPipeTile + (WRES ? 0 : 27 * CO * 32); }
+
+// The weights [co][27][ci] of 16-channel chunk c into dst: tap blocks of CO
+// rows in weight_block's order, canonical K-major core matrices.
+template <int CO>
+__device__ __forceinline__ void stage_weights(uint32_t dst, const bf16* __restrict__ w, int ci, int c, int tid, int n) {
+    for (int i = tid; i < 27 * CO * 2; i += n) {
+        const int k = i & 1, o = (i >> 1) % CO, t = (i >> 1) / CO;
+        cp_async16(dst + weight_block(t) * (CO * 32) + (o >> 3) * 256 + k * 128 + (o & 7) * 16,
+                   w + ((int64_t)o * 27 + t) * ci + c * 16 + k * 8, true);
+    }
+}
+
+template <int CO, bool WRES>
+__global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __restrict__ x, const bf16* __restrict__ w,
+                                                              const float* __restrict__ bias, bf16* __restrict__ y,
+                                                              float* __restrict__ y32, int D, int H, int W, int ci,
+                                                              int relu, int ntiles, int NS) {
+    constexpr int STAGE = pipe_stage<CO, WRES>();
+    constexpr uint32_t ACC = kPipeZ * CO, NCOL = 2 * ACC;  // tensor-memory columns of one / both accumulator sets
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int chunks = ci / 16;
+    // [barriers][weights of all chunks (WRES)][stages]
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);
+    uint64_t* empty = full + 8;
+    uint64_t* tfull = empty + 8;
+    uint64_t* tempty = tfull + 2;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
+    const uint32_t wres = saddr(smem) + kPipeBars, stages = wres + (WRES ? 27 * CO * 32 * chunks : 0);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nbx = (W + TX - 1) / TX, nby = (H + TY - 1) / TY;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tslot)),
+                     "r"(NCOL)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(saddr(full + s), kProducers / 32);
+            mbar_init(saddr(empty + s), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(saddr(tfull + b), 1);
+            mbar_init(saddr(tempty + b), 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (WRES) {
+        for (int c = 0; c < chunks; ++c) stage_weights<CO>(wres + c * 27 * CO * 32, w, ci, c, tid, kPipeThreads);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tslot;
+    bool ok = true;
+
+    if (warp >= 5) {
+        // ---- producers: item = (voxel, 8-channel half); a thread's voxels lie 64 apart
+        const int p = tid - 160;
+        int g = 0;          // chunk count over all blocks
+        int pend = -1;      // the stage written but not yet announced
+        auto announce = [&](int newer, int s) {
+            if (newer) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(saddr(full + s));
+        };
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+            const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
+            for (int c = 0; c < chunks && ok; ++c, ++g) {
+                const int s = g % NS;
+                if (g >= NS && !__all_sync(0xffffffffu, mbar_try(saddr(empty + s), (uint32_t)((g / NS - 1) & 1)))) {
+                    // the stage is not free yet: announce the one before first
+                    if (pend >= 0) announce(0, pend);
+                    pend = -1;
+                    ok = mbar_wait(saddr(empty + s), (uint32_t)((g / NS - 1) & 1));
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                }
+                const uint32_t dst = stages + s * STAGE + (p & 1) * kPipeHalf;
+                int v = p >> 1, vx = v % 10, vy = v / 10, vz = 0;  // v < 64: the first plane
+                int gx = bx * TX - 1 + vx, gy = by * TY - 1 + vy, gz = bz * kPipeZ - 1;
+                const bf16* src = x + c * 16 + (p & 1) * 8;
+                while (v < kPipeVox) {
+                    const bool in = (unsigned)gx < (unsigned)W && (unsigned)gy < (unsigned)H && (unsigned)gz < (unsigned)D;
+                    cp_async16(dst + v * 16, in ? src + (((int64_t)gz * H + gy) * W + gx) * ci : x, in);
+                    v += 64;  // 6 rows and 4 voxels on
+                    vx += 4; gx += 4; vy += 6; gy += 6;
+                    if (vx >= 10) { vx -= 10; gx -= 10; ++vy; ++gy; }
+                    if (vy >= 18) { vy -= 18; gy -= 18; ++vz; ++gz; }
+                }
+                if (!WRES) stage_weights<CO>(stages + s * STAGE + kPipeTile, w, ci, c, p, kProducers);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (pend >= 0) announce(1, pend);
+                pend = s;
+            }
+        }
+        if (pend >= 0) announce(0, pend);
+    } else if (warp == 4) {
+        if (lane == 0) {
+            // per (ty, tx): one MMA per staged plane zz, into output planes
+            // lo .. hi - 1 (N = (hi - lo) co) with the taps tz = zz - lo ..
+            // zz - hi + 1 (weight_block); 54 MMAs, each reading its A operand
+            // once.  The first (ty, tx) of the first chunk starts with planes
+            // 2 and 5, whose output ranges (0..2 and 3) cover every
+            // accumulator once: they initialise it.
+            static_assert(kPipeZ == 4, "merged z taps: 4 output planes, 6 staged");
+            constexpr uint32_t ID[4] = {0, idesc_bf16(128, CO), idesc_bf16(128, 2 * CO), idesc_bf16(128, 3 * CO)};
+            int g = 0, it = 0;
+            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+                const int b = it & 1;
+                if (it >= 2) ok = mbar_wait(saddr(tempty + b), (uint32_t)((it / 2 - 1) & 1));
+                const uint32_t acc = tmem + b * ACC;
+                for (int c = 0; c < chunks && ok; ++c, ++g) {
+                    const int s = g % NS;
+                    ok = mbar_wait(saddr(full + s), (uint32_t)((g / NS) & 1));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t ta = stages + s * STAGE, wa = WRES ? wres + c * 27 * CO * 32 : ta + kPipeTile;
+                    const uint64_t ad0 = smem_desc(ta, kPipeHalf, 160), bd0 = smem_desc(wa, 128, 256);
+#pragma unroll
+                    for (int u = 0; u < 9; ++u) {
+                        const int ty = u / 3, tx = u % 3;
+#pragma unroll
+                        for (int j = 0; j < 6; ++j) {
+                            constexpr int kOrder[6] = {2, 5, 0, 1, 3, 4};
+                            const int zz = kOrder[j];
+                            const int lo = zz > 2 ? zz - 2 : 0, hi = zz + 1 < kPipeZ ? zz + 1 : kPipeZ;
+                            const int b0 = 2 - (zz - lo);
+                            // addresses below 256 KB: the offsets never carry out of the descriptor's address field
+                            mma_bf16(acc + (uint32_t)(lo * CO), ad0 + (uint64_t)((zz * 18 + ty) * 10 + tx),
+                                     bd0 + (uint64_t)((u * 3 + b0) * (CO * 2)), ID[hi - lo],
+                                     (c > 0 || u > 0 || j >= 2) ? 1u : 0u);
+                        }
+                    }
+                    tc_commit(saddr(empty + s));
+                    if (c == chunks - 1) tc_commit(saddr(tfull + b));
+                }
+            }
+            if (!ok) atomicOr(&g_conv_tc_flags, 1u);
+            // the MMAs issued are done before the shared and tensor memory go
+            if (g > 0) mbar_wait(saddr(empty + (g - 1) % NS), (uint32_t)(((g - 1) / NS) & 1));
+        }
+        __syncwarp();
+    } else {
+        // ---- epilogue: warp w reads lanes 32 w .. 32 w + 31 = rows y = 4 w + lane / 8, x = lane % 8
+        const int m = 32 * warp + lane;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+            const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby), b = it & 1;
+            ok = mbar_wait(saddr(tfull + b), (uint32_t)((it / 2) & 1));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int gx = bx * TX + (m & 7), gy = by * TY + (m >> 3);
+            const bool in = gx < W && gy < H;
+#pragma unroll
+            for (int z = 0; z < kPipeZ; ++z) {
+                const int gz = bz * kPipeZ + z;
+                const int64_t vox = ((int64_t)gz * H + gy) * W + gx;
+#pragma unroll
+                for (int c16 = 0; c16 < CO / 16; ++c16) {
+                    float v[16];
+                    tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + b * ACC + (uint32_t)(z * CO + c16 * 16), v);
+                    if (in && gz < D) store16<CO>(v, bias, relu, y, y32, vox, c16);
+                    __syncwarp();
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(saddr(tempty + b));
+        }
+    }
+    if (!ok && lane == 0) atomicOr(&g_conv_tc_flags, 1u);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
@@ -575,18 +755,17 @@ EncodeTiled encode_tiled() {
     return f;
 }
 
-// The tensor map of x [Di][Hi][Wi][ci] BF16 for stride S: box 8 channels x
-// XH voxels along x (stride 2: 2 XH with element stride 2, one parity) x YB
-// x ZB, zero fill outside the tensor.
-template <int S>
-cudaError_t input_map(CUtensorMap* map, const bf16* x, int Di, int Hi, int Wi, int ci) {
-    using G = Geo<S>;
+// The tensor map of x [Di][Hi][Wi][ci] BF16 at stride 2: box 8 channels x
+// 2 XH voxels along x with element stride 2 (one parity) x YB x ZB, zero fill
+// outside the tensor.
+cudaError_t input_map_s2(CUtensorMap* map, const bf16* x, int Di, int Hi, int Wi, int ci) {
+    using G = Geo2;
     EncodeTiled f = encode_tiled();
     if (!f) return cudaErrorNotSupported;
     const cuuint64_t dims[4] = {(cuuint64_t)ci, (cuuint64_t)Wi, (cuuint64_t)Hi, (cuuint64_t)Di};
     const cuuint64_t strides[3] = {(cuuint64_t)ci * 2, (cuuint64_t)Wi * ci * 2, (cuuint64_t)Hi * Wi * ci * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)(S * G::XH), (cuuint32_t)G::YB, (cuuint32_t)G::ZB};
-    const cuuint32_t estride[4] = {1, (cuuint32_t)S, 1, 1};
+    const cuuint32_t box[4] = {8, (cuuint32_t)(2 * G::XH), (cuuint32_t)G::YB, (cuuint32_t)G::ZB};
+    const cuuint32_t estride[4] = {1, 2, 1, 1};
     const CUresult r = f(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), dims, strides, box, estride,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -629,45 +808,55 @@ cudaError_t launch_wgrad(const bf16* x, const bf16* dy, float* dw, int Di, int H
     return cudaGetLastError();
 }
 
-template <int S, int CO>
-cudaError_t launch_co(const bf16* x, const bf16* w, const float* bias, bf16* y, float* y32, int Di, int Hi, int Wi,
+template <int CO>
+cudaError_t launch_s2(const bf16* x, const bf16* w, const float* bias, bf16* y, float* y32, int Di, int Hi, int Wi,
                       int ci, int relu, cudaStream_t st) {
-    constexpr int bytes = smem_bytes<S, CO>();
-    static_assert(bytes <= 227 * 1024, "shared memory");
+    constexpr int bytes = smem_bytes<CO>();
+    // Resident CTAs per SM times their tensor-memory columns must fit the 512
+    // columns of an SM (an allocation that cannot be met waits for another
+    // CTA's release): shared memory bounds the residency below that here.
+    static_assert(bytes <= 227 * 1024 && (227 * 1024 / bytes) * tmem_cols<CO>() <= 512, "shared and tensor memory");
     CUtensorMap map;
-    cudaError_t e = input_map<S>(&map, x, Di, Hi, Wi, ci);
+    cudaError_t e = input_map_s2(&map, x, Di, Hi, Wi, ci);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_conv3_tc<S, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    e = cudaFuncSetAttribute(k_conv3_s2_tc<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    const int Do = Di / S, Ho = Hi / S, Wo = Wi / S;
-    const int64_t blocks = (int64_t)(Wo / TX) * (Ho / TY) * (Do / Geo<S>::TZ);
-    k_conv3_tc<S, CO><<<(unsigned)blocks, kThreads, bytes, st>>>(map, w, bias, y, y32, Do, Ho, Wo, ci, relu);
+    const int Do = Di / 2, Ho = Hi / 2, Wo = Wi / 2;
+    const int64_t blocks = (int64_t)(Wo / TX) * (Ho / TY) * Do;
+    k_conv3_s2_tc<CO><<<(unsigned)blocks, kThreads, bytes, st>>>(map, w, bias, y, y32, Do, Ho, Wo, ci, relu);
     return cudaGetLastError();
 }
 
-// Resident CTAs per SM times their tensor-memory columns must fit the 512
-// columns of an SM (an allocation that cannot be met waits for another
-// CTA's release): shared memory bounds the residency below that here --
-// stride 1: (co = 16) 4 x 64, (32) 3 x 128, (64) 2 x 256 columns; stride 2:
-// at most 3 x 32, 2 x 32, 2 x 64.
-template <int S, int CO>
-constexpr bool tmem_fits() {
-    return (227 * 1024 / smem_bytes<S, CO>()) * tmem_cols<S, CO>() <= 512;
+// Stride 1: one CTA an SM, its shared memory filled with input stages.
+template <int CO, bool WRES>
+cudaError_t launch_pipe_w(const bf16* x, const bf16* w, const float* bias, bf16* y, float* y32, int D, int H, int W,
+                          int ci, int relu, cudaStream_t st) {
+    const int64_t tiles = lbm::ceil_div(D, kPipeZ) * lbm::ceil_div(H, TY) * lbm::ceil_div(W, TX);
+    if (tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    constexpr int kMost = 227 * 1024, kStages = 6;  // (2 to 6 stages; the kernel has room for 8 barriers)
+    const int fixed = kPipeBars + (WRES ? 27 * CO * 2 * ci : 0);
+    int ns = (kMost - fixed) / pipe_stage<CO, WRES>();
+    ns = ns < kStages ? ns : kStages;
+    if (ns < 2) return cudaErrorInvalidConfiguration;
+    const int bytes = fixed + ns * pipe_stage<CO, WRES>();
+    cudaError_t e = cudaFuncSetAttribute(k_conv3_pipe<CO, WRES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+    if (e != cudaSuccess) return e;
+    // every CTA about the same number of blocks; more than half of an SM's
+    // shared memory each, so that one CTA's tensor memory is alone on its SM
+    const int64_t per = lbm::ceil_div(tiles, 152);
+    const int alone = bytes > 116 * 1024 ? bytes : 116 * 1024;
+    k_conv3_pipe<CO, WRES><<<(unsigned)lbm::ceil_div(tiles, per), kPipeThreads, alone, st>>>(x, w, bias, y, y32, D, H, W,
+                                                                                            ci, relu, (int)tiles, ns);
+    return cudaGetLastError();
 }
-static_assert(tmem_fits<1, 16>() && tmem_fits<1, 32>() && tmem_fits<1, 64>(), "tensor memory (stride 1)");
-static_assert(tmem_fits<2, 16>() && tmem_fits<2, 32>() && tmem_fits<2, 64>(), "tensor memory (stride 2)");
 
-template <int S>
-cudaError_t launch_s(const void* x, int Di, int Hi, int Wi, int ci, const void* w, const float* bias, int co,
-                     int relu, void* y, float* y32, cudaStream_t st) {
-    const bf16* xb = static_cast<const bf16*>(x);
-    const bf16* wb = static_cast<const bf16*>(w);
-    bf16* yb = static_cast<bf16*>(y);
-    switch (co) {
-        case 16: return launch_co<S, 16>(xb, wb, bias, yb, y32, Di, Hi, Wi, ci, relu, st);
-        case 32: return launch_co<S, 32>(xb, wb, bias, yb, y32, Di, Hi, Wi, ci, relu, st);
-        default: return launch_co<S, 64>(xb, wb, bias, yb, y32, Di, Hi, Wi, ci, relu, st);
-    }
+template <int CO>
+cudaError_t launch_pipe(const bf16* x, const bf16* w, const float* bias, bf16* y, float* y32, int D, int H, int W,
+                        int ci, int relu, cudaStream_t st) {
+    // the weights of all chunks beside at least two stages: all but 64 -> 64 channels (216 KB)
+    if (27 * CO * 2 * ci <= 112 * 1024) return launch_pipe_w<CO, true>(x, w, bias, y, y32, D, H, W, ci, relu, st);
+    if constexpr (CO == 64) return launch_pipe_w<CO, false>(x, w, bias, y, y32, D, H, W, ci, relu, st);
+    return cudaErrorInvalidConfiguration;
 }
 
 }  // namespace
@@ -677,17 +866,28 @@ namespace lbm {
 bool conv3_tc_applies(int D, int H, int W, int ci, int co, int stride) {
     const bool ch = (ci == 16 || ci == 32 || ci == 64) && (co == 16 || co == 32 || co == 64);
     if (!ch || D <= 0 || H <= 0 || W <= 0) return false;
-    if (stride == 1) return D % Geo<1>::TZ == 0 && H % TY == 0 && W % TX == 0;
-    if (stride == 2)
-        return D % 2 == 0 && H % 2 == 0 && W % 2 == 0 && (D / 2) % Geo<2>::TZ == 0 && (H / 2) % TY == 0 &&
-               (W / 2) % TX == 0;
+    if (stride == 1) return ceil_div(D, kPipeZ) * ceil_div(H, TY) * ceil_div(W, TX) <= 0x7fffffffLL;
+    if (stride == 2) return D % 2 == 0 && H % (2 * TY) == 0 && W % (2 * TX) == 0;
     return false;
 }
 
 cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, const float* bias, int co, int relu,
                      void* y, float* y32, int stride, cudaStream_t st) {
-    return stride == 2 ? launch_s<2>(x, D, H, W, ci, w, bias, co, relu, y, y32, st)
-                       : launch_s<1>(x, D, H, W, ci, w, bias, co, relu, y, y32, st);
+    const bf16* xb = static_cast<const bf16*>(x);
+    const bf16* wb = static_cast<const bf16*>(w);
+    bf16* yb = static_cast<bf16*>(y);
+    if (stride == 2) {
+        switch (co) {
+            case 16: return launch_s2<16>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
+            case 32: return launch_s2<32>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
+            default: return launch_s2<64>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
+        }
+    }
+    switch (co) {
+        case 16: return launch_pipe<16>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
+        case 32: return launch_pipe<32>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
+        default: return launch_pipe<64>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
+    }
 }
 
 bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride) {
