@@ -127,36 +127,52 @@ __device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_
         : "memory");
 }
 
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
+// 16 columns of this warp's 32 lanes, without waiting; tc_ld_wait waits for
+// every load issued and orders the registers' use behind it.
+__device__ __forceinline__ void tc_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
-// 16 channels (c16) of output voxel vox from their FP32 sums: bias, ReLU, BF16 (and FP32) store.
-template <int CO>
-__device__ __forceinline__ void store16(float (&v)[16], const float* __restrict__ bias, int relu, bf16* __restrict__ y,
-                                        float* __restrict__ y32, int64_t vox, int c16) {
+__device__ __forceinline__ void tc_ld_wait(uint32_t (&r)[4][16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(r[k][e]));
+}
+
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    tc_ld16_issue(taddr, r);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
-        v[k] += bias ? bias[c16 * 16 + k] : 0.f;
+        asm volatile("" : "+r"(r[k]));
+        v[k] = __uint_as_float(r[k]);
+    }
+}
+
+// 16 channels at element `at` of the output from their FP32 sums: bias (of those channels), ReLU, BF16 (and FP32) store.
+__device__ __forceinline__ void store16(float (&v)[16], const float* __restrict__ bias, int relu, bf16* __restrict__ y,
+                                        float* __restrict__ y32, int64_t at) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        v[k] += bias ? bias[k] : 0.f;
         if (relu) v[k] = fmaxf(v[k], 0.f);
     }
     uint4 p[2];
     __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(p);
 #pragma unroll
     for (int k = 0; k < 8; ++k) h[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-    uint4* dst = reinterpret_cast<uint4*>(y + vox * CO + c16 * 16);
+    uint4* dst = reinterpret_cast<uint4*>(y + at);
     dst[0] = p[0];
     dst[1] = p[1];
     if (y32) {
-        float4* d32 = reinterpret_cast<float4*>(y32 + vox * CO + c16 * 16);
+        float4* d32 = reinterpret_cast<float4*>(y32 + at);
 #pragma unroll
         for (int k = 0; k < 4; ++k) d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     }
@@ -169,6 +185,13 @@ __device__ __forceinline__ void store16(float (&v)[16], const float* __restrict_
 // of those planes are the adjacent tensor-memory column ranges (z co .. z co
 // + co - 1 for plane z).
 __host__ __device__ constexpr int weight_block(int t) { return ((t / 3) % 3 * 3 + t % 3) * 3 + (2 - t / 9); }
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -291,7 +314,7 @@ __global__ void __launch_bounds__(kThreads) k_conv3_s2_tc(const __grid_constant_
         for (int c16 = 0; c16 < CO / 16; ++c16) {
             float v[16];
             tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(c16 * 16), v);
-            store16<CO>(v, bias, relu, y, y32, vox, c16);
+            store16(v, bias ? bias + c16 * 16 : nullptr, relu, y, y32, vox * CO + c16 * 16);
         }
     } else if (c > 0) {
         // the wait of chunk c - 1 gave up: record it, wait (bounded) once
@@ -311,31 +334,31 @@ __global__ void __launch_bounds__(kThreads) k_conv3_s2_tc(const __grid_constant_
 // at the top, in one persistent CTA an SM whose warps each do one thing:
 //   warps 0-3  epilogue: tensor memory -> bias, ReLU -> global memory
 //   warp 4     one thread issues the MMAs
-//   warps 5-8  producers: the block's input voxels (16 channels) into the
+//   warps 5-12 producers: the block's input voxels (16 channels) into the
 //              next of NS stages by cp.async, zero outside the grid
 // so the copies of later blocks and the stores of the previous one run
 // beside the current one's MMAs (two sets of accumulators), and the weights
-// are staged once per CTA where they fit (WRES; 64 -> 64 channels: with each
-// stage).  mbarriers hand over the stages (full / empty) and accumulators
+// of CO output channels (16, or 32 of 32 or 64: grid.y) are staged once per
+// CTA.  mbarriers hand over the stages (full / empty) and accumulators
 // (tfull / tempty); every wait is bounded, and a role that gives up raises
 // the flag and leaves, whereupon the others' waits run out.
 //
-// What bounds it: an MMA reads its 4 KB of A from shared memory (32 cycles;
-// 54 a chunk) and, from 32 channels on, its N columns.  The kernel before
+// What bounds it: an M = 128, K = 16 MMA holds the tensor pipe for 64 cycles
+// up to N = 64 (ncu: 69.8k pipe cycles for 1091 MMAs a SM), 54 a chunk; at
+// 16 -> 16 channels (N = 16 to 48) that is 95 of 120 us.  The kernel before
 // staged with tensor copies, whose 8-channel layout is boxes of 16-byte
 // rows: 2160 a chunk at about 3 cycles each, 7.2k cycles a chunk whatever
-// its MMAs (16 -> 16: 2.4k).  The same bytes by cp.async are 68 warp
-// instructions.
+// its MMAs.  The same bytes by cp.async are 68 warp instructions.  256 x 128
+// x 128: 16 -> 16 196 -> 117 us, 32 -> 16 278 -> 186 us; 128 x 64 x 64:
+// 64 -> 32 82 -> 64 us (906 TFLOP/s), 64 -> 64 123 us (167 with all 64
+// output channels in one CTA, whose weights do not fit beside the stages).
 constexpr int kPipeZ = 4;                                  // output planes of a block
 constexpr int kPipeVox = (kPipeZ + 2) * 18 * 10;           // staged voxels of a block
 constexpr int kPipeHalf = kPipeVox * 16 + 64;              // bytes of an 8-channel half (+64: the halves in different banks)
 constexpr int kPipeTile = 2 * kPipeHalf;
-constexpr int kProducers = 128;
+constexpr int kProducers = 256;
 constexpr int kPipeThreads = 32 * (4 + 1) + kProducers;
 constexpr int kPipeBars = 256;                             // bytes for barriers and the tensor-memory address
-
-template <int CO, bool WRES>
-__host__ __device__ constexpr int pipe_stage() { return kPipeTile + (WRES ? 0 : 27 * CO * 32); }
 
 // The weights [co][27][ci] of 16-channel chunk c into dst: tap blocks of CO
 // rows in weight_block's order, canonical K-major core matrices.
@@ -348,22 +371,32 @@ __device__ __forceinline__ void stage_weights(uint32_t dst, const bf16* __restri
     }
 }
 
-template <int CO, bool WRES>
+// The five other warps' weight copies are done and visible to the MMAs.
+__device__ __forceinline__ void weights_staged() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(kPipeThreads - kProducers) : "memory");
+}
+
+template <int CO>
 __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                               const float* __restrict__ bias, bf16* __restrict__ y,
                                                               float* __restrict__ y32, int D, int H, int W, int ci,
-                                                              int relu, int ntiles, int NS) {
-    constexpr int STAGE = pipe_stage<CO, WRES>();
+                                                              int co, int relu, int ntiles, int NS) {
+    constexpr int STAGE = kPipeTile;
     constexpr uint32_t ACC = kPipeZ * CO, NCOL = 2 * ACC;  // tensor-memory columns of one / both accumulator sets
     extern __shared__ __align__(128) unsigned char smem[];
     const int chunks = ci / 16;
-    // [barriers][weights of all chunks (WRES)][stages]
+    const int o0 = blockIdx.y * CO;  // first output channel
+    w += (int64_t)o0 * 27 * ci;
+    if (bias) bias += o0;
+    // [barriers][weights of all chunks][stages]
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + 8;
     uint64_t* tfull = empty + 8;
     uint64_t* tempty = tfull + 2;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
-    const uint32_t wres = saddr(smem) + kPipeBars, stages = wres + (WRES ? 27 * CO * 32 * chunks : 0);
+    const uint32_t wres = saddr(smem) + kPipeBars, stages = wres + 27 * CO * 32 * chunks;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nbx = (W + TX - 1) / TX, nby = (H + TY - 1) / TY;
 
@@ -384,20 +417,23 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (WRES) {
-        for (int c = 0; c < chunks; ++c) stage_weights<CO>(wres + c * 27 * CO * 32, w, ci, c, tid, kPipeThreads);
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
     bool ok = true;
+    if (warp < 5) {
+        // the weights, while the producers' first copies are under way
+        for (int c = 0; c < chunks; ++c) stage_weights<CO>(wres + c * 27 * CO * 32, w, ci, c, tid, kPipeThreads - kProducers);
+        weights_staged();
+    }
 
     if (warp >= 5) {
-        // ---- producers: item = (voxel, 8-channel half); a thread's voxels lie 64 apart
+        // ---- producers: item = (voxel, 8-channel half); a thread's voxels lie 128 apart
         const int p = tid - 160;
+        static_assert(kProducers == 256, "a thread's next voxel: 128 on");
+        const int64_t next = (int64_t)(12 * W + 8) * ci, next_x = (int64_t)(W - 10) * ci,
+                      next_y = (int64_t)(H - 18) * W * ci;
         int g = 0;          // chunk count over all blocks
         int pend = -1;      // the stage written but not yet announced
         auto announce = [&](int newer, int s) {
@@ -420,18 +456,19 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
                     if (!ok) break;
                 }
                 const uint32_t dst = stages + s * STAGE + (p & 1) * kPipeHalf;
-                int v = p >> 1, vx = v % 10, vy = v / 10, vz = 0;  // v < 64: the first plane
-                int gx = bx * TX - 1 + vx, gy = by * TY - 1 + vy, gz = bz * kPipeZ - 1;
-                const bf16* src = x + c * 16 + (p & 1) * 8;
+                int v = p >> 1, vx = v % 10, gy = by * TY - 1 + v / 10, gz = bz * kPipeZ - 1;  // the first plane
+                int gx = bx * TX - 1 + vx;
+                const int yend = by * TY + 17;
+                int64_t at = (((int64_t)gz * H + gy) * W + gx) * ci + c * 16 + (p & 1) * 8;
                 while (v < kPipeVox) {
                     const bool in = (unsigned)gx < (unsigned)W && (unsigned)gy < (unsigned)H && (unsigned)gz < (unsigned)D;
-                    cp_async16(dst + v * 16, in ? src + (((int64_t)gz * H + gy) * W + gx) * ci : x, in);
-                    v += 64;  // 6 rows and 4 voxels on
-                    vx += 4; gx += 4; vy += 6; gy += 6;
-                    if (vx >= 10) { vx -= 10; gx -= 10; ++vy; ++gy; }
-                    if (vy >= 18) { vy -= 18; gy -= 18; ++vz; ++gz; }
+                    cp_async16(dst + v * 16, x + (in ? at : 0), in);
+                    // 128 voxels on: 12 rows and 8, wrapped into 10 x 18
+                    v += kProducers / 2;
+                    vx += 8; gx += 8; gy += 12; at += next;
+                    if (vx >= 10) { vx -= 10; gx -= 10; ++gy; at += next_x; }
+                    if (gy >= yend) { gy -= 18; ++gz; at += next_y; }
                 }
-                if (!WRES) stage_weights<CO>(stages + s * STAGE + kPipeTile, w, ci, c, p, kProducers);
                 asm volatile("cp.async.commit_group;" ::: "memory");
                 if (pend >= 0) announce(1, pend);
                 pend = s;
@@ -439,27 +476,32 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
         }
         if (pend >= 0) announce(0, pend);
     } else if (warp == 4) {
-        if (lane == 0) {
-            // per (ty, tx): one MMA per staged plane zz, into output planes
-            // lo .. hi - 1 (N = (hi - lo) co) with the taps tz = zz - lo ..
-            // zz - hi + 1 (weight_block); 54 MMAs, each reading its A operand
-            // once.  The first (ty, tx) of the first chunk starts with planes
-            // 2 and 5, whose output ranges (0..2 and 3) cover every
-            // accumulator once: they initialise it.
-            static_assert(kPipeZ == 4, "merged z taps: 4 output planes, 6 staged");
-            constexpr uint32_t ID[4] = {0, idesc_bf16(128, CO), idesc_bf16(128, 2 * CO), idesc_bf16(128, 3 * CO)};
-            int g = 0, it = 0;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
-                const int b = it & 1;
-                if (it >= 2) ok = mbar_wait(saddr(tempty + b), (uint32_t)((it / 2 - 1) & 1));
-                const uint32_t acc = tmem + b * ACC;
-                for (int c = 0; c < chunks && ok; ++c, ++g) {
-                    const int s = g % NS;
-                    ok = mbar_wait(saddr(full + s), (uint32_t)((g / NS) & 1));
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t ta = stages + s * STAGE, wa = WRES ? wres + c * 27 * CO * 32 : ta + kPipeTile;
-                    const uint64_t ad0 = smem_desc(ta, kPipeHalf, 160), bd0 = smem_desc(wa, 128, 256);
+        // ---- MMAs.  The whole warp runs the loop and one elected lane
+        // issues, so that descriptors are warp-uniform values (uniform
+        // registers, as the instruction takes them).
+        // Per (ty, tx): one MMA per staged plane zz, into output planes lo ..
+        // hi - 1 (N = (hi - lo) co) with the taps tz = zz - lo .. zz - hi + 1
+        // (weight_block); 54 MMAs, each reading its A operand once.  The
+        // first (ty, tx) of the first chunk starts with planes 2 and 5, whose
+        // output ranges (0..2 and 3) cover every accumulator once: they
+        // initialise it.
+        static_assert(kPipeZ == 4, "merged z taps: 4 output planes, 6 staged");
+        constexpr uint32_t ID[4] = {0, idesc_bf16(128, CO), idesc_bf16(128, 2 * CO), idesc_bf16(128, 3 * CO)};
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), st0 = __shfl_sync(0xffffffffu, stages, 0),
+                       w0 = __shfl_sync(0xffffffffu, wres, 0);
+        int g = 0, it = 0, s = 0, ph = 0;  // chunk and block counts; stage of chunk g and its phase
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+            const int b = it & 1;
+            if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(saddr(tempty + b), (uint32_t)((it / 2 - 1) & 1)));
+            const uint32_t acc = tm + b * ACC;
+            for (int c = 0; c < chunks && ok; ++c, ++g) {
+                ok = __all_sync(0xffffffffu, mbar_wait(saddr(full + s), (uint32_t)ph));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ta = st0 + s * STAGE, wa = w0 + c * 27 * CO * 32;
+                const uint64_t ad0 = smem_desc(ta, kPipeHalf, 160), bd0 = smem_desc(wa, 128, 256);
+                if (leader) {
 #pragma unroll
                     for (int u = 0; u < 9; ++u) {
                         const int ty = u / 3, tx = u % 3;
@@ -470,19 +512,21 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
                             const int lo = zz > 2 ? zz - 2 : 0, hi = zz + 1 < kPipeZ ? zz + 1 : kPipeZ;
                             const int b0 = 2 - (zz - lo);
                             // addresses below 256 KB: the offsets never carry out of the descriptor's address field
-                            mma_bf16(acc + (uint32_t)(lo * CO), ad0 + (uint64_t)((zz * 18 + ty) * 10 + tx),
-                                     bd0 + (uint64_t)((u * 3 + b0) * (CO * 2)), ID[hi - lo],
-                                     (c > 0 || u > 0 || j >= 2) ? 1u : 0u);
+                            const uint64_t ad = ad0 + (uint64_t)((zz * 18 + ty) * 10 + tx);
+                            const uint64_t bd = bd0 + (uint64_t)((u * 3 + b0) * (CO * 2));
+                            if (u > 0 || j >= 2) mma_bf16(acc + (uint32_t)(lo * CO), ad, bd, ID[hi - lo], 1u);
+                            else mma_bf16(acc + (uint32_t)(lo * CO), ad, bd, ID[hi - lo], c > 0 ? 1u : 0u);
                         }
                     }
                     tc_commit(saddr(empty + s));
                     if (c == chunks - 1) tc_commit(saddr(tfull + b));
                 }
+                __syncwarp();
+                if (++s == NS) { s = 0; ph ^= 1; }
             }
-            if (!ok) atomicOr(&g_conv_tc_flags, 1u);
-            // the MMAs issued are done before the shared and tensor memory go
-            if (g > 0) mbar_wait(saddr(empty + (g - 1) % NS), (uint32_t)(((g - 1) / NS) & 1));
         }
+        // the MMAs issued are done before the shared and tensor memory go
+        if (g > 0) mbar_wait(saddr(empty + (g - 1) % NS), (uint32_t)(((g - 1) / NS) & 1));
         __syncwarp();
     } else {
         // ---- epilogue: warp w reads lanes 32 w .. 32 w + 31 = rows y = 4 w + lane / 8, x = lane % 8
@@ -496,21 +540,34 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int gx = bx * TX + (m & 7), gy = by * TY + (m >> 3);
             const bool in = gx < W && gy < H;
+            // 64 accumulator columns a pass, their loads in flight together;
+            // the set is handed back once the last pass has been read
 #pragma unroll
-            for (int z = 0; z < kPipeZ; ++z) {
-                const int gz = bz * kPipeZ + z;
-                const int64_t vox = ((int64_t)gz * H + gy) * W + gx;
+            for (int pass = 0; pass < (int)ACC / 64; ++pass) {
+                uint32_t r[4][16];
 #pragma unroll
-                for (int c16 = 0; c16 < CO / 16; ++c16) {
-                    float v[16];
-                    tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + b * ACC + (uint32_t)(z * CO + c16 * 16), v);
-                    if (in && gz < D) store16<CO>(v, bias, relu, y, y32, vox, c16);
+                for (int k = 0; k < 4; ++k)
+                    tc_ld16_issue(tmem + ((uint32_t)(32 * warp) << 16) + b * ACC + (uint32_t)(pass * 64 + k * 16), r[k]);
+                tc_ld_wait(r);
+                if (pass == (int)ACC / 64 - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
+                    if (lane == 0) mbar_arrive(saddr(tempty + b));
                 }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int col = pass * 64 + k * 16, z = col / CO, c16 = col % CO / 16;
+                    const int gz = bz * kPipeZ + z;
+                    if (in && gz < D) {
+                        float v[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[k][e]);
+                        store16(v, bias ? bias + c16 * 16 : nullptr, relu, y, y32,
+                                (((int64_t)gz * H + gy) * W + gx) * co + o0 + c16 * 16);
+                    }
+                }
+                __syncwarp();
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(saddr(tempty + b));
         }
     }
     if (!ok && lane == 0) atomicOr(&g_conv_tc_flags, 1u);
@@ -827,36 +884,36 @@ cudaError_t launch_s2(const bf16* x, const bf16* w, const float* bias, bf16* y, 
     return cudaGetLastError();
 }
 
-// Stride 1: one CTA an SM, its shared memory filled with input stages.
-template <int CO, bool WRES>
-cudaError_t launch_pipe_w(const bf16* x, const bf16* w, const float* bias, bf16* y, float* y32, int D, int H, int W,
-                          int ci, int relu, cudaStream_t st) {
-    const int64_t tiles = lbm::ceil_div(D, kPipeZ) * lbm::ceil_div(H, TY) * lbm::ceil_div(W, TX);
-    if (tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    constexpr int kMost = 227 * 1024, kStages = 6;  // (2 to 6 stages; the kernel has room for 8 barriers)
-    const int fixed = kPipeBars + (WRES ? 27 * CO * 2 * ci : 0);
-    int ns = (kMost - fixed) / pipe_stage<CO, WRES>();
-    ns = ns < kStages ? ns : kStages;
-    if (ns < 2) return cudaErrorInvalidConfiguration;
-    const int bytes = fixed + ns * pipe_stage<CO, WRES>();
-    cudaError_t e = cudaFuncSetAttribute(k_conv3_pipe<CO, WRES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
-    if (e != cudaSuccess) return e;
-    // every CTA about the same number of blocks; more than half of an SM's
-    // shared memory each, so that one CTA's tensor memory is alone on its SM
-    const int64_t per = lbm::ceil_div(tiles, 152);
-    const int alone = bytes > 116 * 1024 ? bytes : 116 * 1024;
-    k_conv3_pipe<CO, WRES><<<(unsigned)lbm::ceil_div(tiles, per), kPipeThreads, alone, st>>>(x, w, bias, y, y32, D, H, W,
-                                                                                            ci, relu, (int)tiles, ns);
-    return cudaGetLastError();
+// Shared memory of a persistent CTA: `fixed` bytes and as many stages as fit
+// (2 to 6; the kernels have room for 8 barriers); more than half of an SM's,
+// so that a CTA's tensor memory is alone on its SM.
+struct PipeShape {
+    int stages, bytes;
+};
+PipeShape pipe_shape(int fixed, int stage) {
+    constexpr int kMost = 227 * 1024, kLeast = 116 * 1024;
+    int ns = (kMost - fixed) / stage;
+    ns = ns < 6 ? ns : 6;
+    const int bytes = fixed + ns * stage;
+    return {ns, bytes > kLeast ? bytes : kLeast};
 }
 
+// Stride 1: one CTA an SM over all blocks and channel parts, every CTA about
+// the same number of blocks.
 template <int CO>
 cudaError_t launch_pipe(const bf16* x, const bf16* w, const float* bias, bf16* y, float* y32, int D, int H, int W,
-                        int ci, int relu, cudaStream_t st) {
-    // the weights of all chunks beside at least two stages: all but 64 -> 64 channels (216 KB)
-    if (27 * CO * 2 * ci <= 112 * 1024) return launch_pipe_w<CO, true>(x, w, bias, y, y32, D, H, W, ci, relu, st);
-    if constexpr (CO == 64) return launch_pipe_w<CO, false>(x, w, bias, y, y32, D, H, W, ci, relu, st);
-    return cudaErrorInvalidConfiguration;
+                        int ci, int co, int relu, cudaStream_t st) {
+    const int64_t tiles = lbm::ceil_div(D, kPipeZ) * lbm::ceil_div(H, TY) * lbm::ceil_div(W, TX);
+    if (tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    static_assert(kPipeBars + 27 * 32 * 2 * 64 + 2 * kPipeTile <= 227 * 1024, "32 of 64 -> 64 channels");
+    const PipeShape p = pipe_shape(kPipeBars + 27 * CO * 2 * ci, kPipeTile);
+    cudaError_t e = cudaFuncSetAttribute(k_conv3_pipe<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    const int parts = co / CO;
+    const int64_t per = lbm::ceil_div(tiles, 152 / parts);
+    k_conv3_pipe<CO><<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)parts), kPipeThreads, p.bytes, st>>>(
+        x, w, bias, y, y32, D, H, W, ci, co, relu, (int)tiles, p.stages);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -883,11 +940,8 @@ cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, 
             default: return launch_s2<64>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
         }
     }
-    switch (co) {
-        case 16: return launch_pipe<16>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
-        case 32: return launch_pipe<32>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
-        default: return launch_pipe<64>(xb, wb, bias, yb, y32, D, H, W, ci, relu, st);
-    }
+    return co == 16 ? launch_pipe<16>(xb, wb, bias, yb, y32, D, H, W, ci, co, relu, st)
+                    : launch_pipe<32>(xb, wb, bias, yb, y32, D, H, W, ci, co, relu, st);
 }
 
 bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride) {

@@ -242,8 +242,8 @@ cudaError_t nw_readout_f32(const float2* accf, const float* ring, int64_t nnw, i
 
 // 3x3x3 convolutions of the warm-start network on tcgen05 tensor cores
 // (conv_tc.cu): the shapes they take (channels 16 / 32 / 64; input grid D x
-// H x W with, at stride 1, D % 4, H % 16, W % 8 == 0, at stride 2 even
-// dimensions and H / 2 % 16, W / 2 % 8 == 0), the forward convolution, the
+// H x W any at stride 1, at stride 2 with even dimensions and H / 2 % 16,
+// W / 2 % 8 == 0), the forward convolution, the
 // flipped-transposed weights that turn a stride-1 input gradient into a
 // forward convolution, and the flag of a bounded wait that gave up (read
 // and cleared).
