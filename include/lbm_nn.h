@@ -28,9 +28,9 @@ lbm_status lbm_nn_conv3d_fwd(const void* x, const int dims_in[3], int ci, const 
 
 /* Convolution engine.  LBM_NN_ENGINE_AUTO (default): 3x3x3 convolutions
  * run on the tcgen05 tensor cores with tensor-memory accumulators
- * (conv_tc.cu) -- the forward pass and input gradient at stride 1 on any
- * grid, the forward pass at stride 2 on even grids whose output has H % 16
- * and W % 8 == 0; the others run on mma.sync, the weight gradients (kernel size 3
+ * (conv_tc.cu) -- the forward pass at stride 1 and the input gradients on
+ * any grid, the forward pass at stride 2 on even grids whose output has
+ * H % 16 and W % 8 == 0; the others run on mma.sync, the weight gradients (kernel size 3
  * and 1, any grid) on the staged-tile kernel of conv_tc.cu.
  * LBM_NN_ENGINE_MMA_SYNC: the plain mma.sync kernels everywhere (the
  * comparison path).

@@ -578,6 +578,221 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
 }
 
 // ---------------------------------------------------------------------------
+// Input gradient at stride 2, any grid: dx[i] = sum over taps t of
+// dY[(i + 1 - t) / 2] W[t] where i + 1 - t is even (per axis).  With i =
+// 2 j + p, an even i (p = 0) has one tap, t = 1 at dY[j]; an odd one two,
+// t = 2 at dY[j] and t = 0 at dY[j + 1].  So the 8 parity classes of an 8 x
+// 16 block of j share one staged block of dY (9 x 17 x 2 voxels, all co
+// channels), and each of its 8 offsets in {0, 1}^3 is one view (as the taps
+// above) that feeds the classes with p = 1 wherever the offset is 1: 8, 4, 2
+// or 1 of them, 27 (offset, class) blocks of CI columns.  The classes'
+// accumulators lie side by side in tensor memory (class 4 pz + 2 py + px), so
+// neighbouring classes take one MMA: 14 MMAs per 16 channels of dY, N = CI to
+// 8 CI, the first (offset 0) initialising every class.  Roles and barriers as
+// in k_conv3_pipe; a stage holds all co channels of a block.
+// (The fallback read dY once per tap, 7/8 of them for nothing: 2293 us for
+// 32 -> 16 channels onto 256 x 128 x 128, 57 us here; 64 -> 32 onto 128 x 64 x
+// 64 489 -> 44 us; bound by the MMAs, 64 cycles each and 128 at N = 256.)
+constexpr int kD2Vox = 2 * 17 * 9;
+constexpr int kD2Half = kD2Vox * 16 + 64;
+
+// First block (of the 27) of an offset, offsets ordered zyx = 000, 100, 010,
+// 001, 110, 101, 011, 111.
+struct D2Off {
+    int z, y, x, first;
+};
+__host__ __device__ constexpr D2Off d2_off(int k) {
+    constexpr D2Off t[8] = {{0, 0, 0, 0},  {1, 0, 0, 8},  {0, 1, 0, 12}, {0, 0, 1, 16},
+                            {1, 1, 0, 20}, {1, 0, 1, 22}, {0, 1, 1, 24}, {1, 1, 1, 26}};
+    return t[k];
+}
+// Tap of class bit p at offset o along one axis.
+__host__ __device__ constexpr int d2_tap(int p, int o) { return p == 0 ? 1 : (o == 0 ? 2 : 0); }
+
+template <int CI>
+__global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_dx2(const bf16* __restrict__ dy, const bf16* __restrict__ wt,
+                                                             bf16* __restrict__ dx, int D, int H, int W, int ci,
+                                                             int Do, int Ho, int Wo, int co, int ntiles, int NS) {
+    constexpr uint32_t ACC = 8 * CI, NCOL = 2 * ACC;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int groups = co / 8, chunks = co / 16, stage_bytes = groups * kD2Half;
+    const int c0 = blockIdx.y * CI;  // first input channel
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);
+    uint64_t* empty = full + 8;
+    uint64_t* tfull = empty + 8;
+    uint64_t* tempty = tfull + 2;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
+    const uint32_t wres = saddr(smem) + kPipeBars, stages = wres + 27 * CI * 2 * co;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nbx = (Wo + TX - 1) / TX, nby = (Ho + TY - 1) / TY;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tslot)),
+                     "r"(NCOL)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(saddr(full + s), kProducers / 32);
+            mbar_init(saddr(empty + s), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(saddr(tfull + b), 1);
+            mbar_init(saddr(tempty + b), 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tslot;
+    bool ok = true;
+    if (warp < 5) {
+        // wt [ci][27][co]: rows c of the block of (offset, class), 16-byte pieces of 8 co
+        for (int i = tid; i < 27 * CI * groups; i += kPipeThreads - kProducers) {
+            const int k8 = i % groups, n = (i / groups) % CI, blk = i / (groups * CI);
+            int k = 0;
+            while (k < 7 && blk >= d2_off(k + 1).first) ++k;
+            const D2Off o = d2_off(k);
+            const int need = 4 * o.z + 2 * o.y + o.x;
+            int cls = 0;  // the (blk - first)-th class with p = 1 where the offset is 1
+            for (int m = blk - o.first; (cls & need) != need || m-- > 0; ++cls) {}
+            const int t = (d2_tap(cls >> 2, o.z) * 3 + d2_tap((cls >> 1) & 1, o.y)) * 3 + d2_tap(cls & 1, o.x);
+            cp_async16(wres + ((k8 >> 1) * 27 + blk) * (CI * 32) + (n >> 3) * 256 + (k8 & 1) * 128 + (n & 7) * 16,
+                       wt + ((int64_t)(c0 + n) * 27 + t) * co + k8 * 8, true);
+        }
+        weights_staged();
+    }
+
+    if (warp >= 5) {
+        // ---- producers: item = (voxel, 8-channel group), groups fastest
+        const int p = tid - 160, gsh = 31 - __clz(groups);
+        int it = 0, pend = -1;
+        auto announce = [&](int newer, int s) {
+            if (newer) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(saddr(full + s));
+        };
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+            const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
+            const int s = it % NS;
+            if (it >= NS && !__all_sync(0xffffffffu, mbar_try(saddr(empty + s), (uint32_t)((it / NS - 1) & 1)))) {
+                if (pend >= 0) announce(0, pend);
+                pend = -1;
+                ok = mbar_wait(saddr(empty + s), (uint32_t)((it / NS - 1) & 1));
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+            }
+            const uint32_t dst = stages + s * stage_bytes;
+            for (int i = p; i < kD2Vox << gsh; i += kProducers) {
+                const int v = i >> gsh, k8 = i & (groups - 1);
+                const int vx = v % 9, vy = (v / 9) % 17, vz = v / 153;
+                const int gx = bx * TX + vx, gy = by * TY + vy, gz = bz + vz;
+                const bool in = gx < Wo && gy < Ho && gz < Do;
+                cp_async16(dst + k8 * kD2Half + v * 16,
+                           dy + (in ? (((int64_t)gz * Ho + gy) * Wo + gx) * co + k8 * 8 : 0), in);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (pend >= 0) announce(1, pend);
+            pend = s;
+        }
+        if (pend >= 0) announce(0, pend);
+    } else if (warp == 4) {
+        // ---- MMAs (whole warp, one elected lane issues)
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), st0 = __shfl_sync(0xffffffffu, stages, 0),
+                       w0 = __shfl_sync(0xffffffffu, wres, 0);
+        int it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+            const int b = it & 1, s = it % NS;
+            if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(saddr(tempty + b), (uint32_t)((it / 2 - 1) & 1)));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(saddr(full + s), (uint32_t)((it / NS) & 1)));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tm + b * ACC;
+            if (leader) {
+                for (int c = 0; c < chunks; ++c) {
+                    const uint64_t ad0 = smem_desc(st0 + s * stage_bytes + 2 * c * kD2Half, kD2Half, 144);
+                    const uint64_t bd0 = smem_desc(w0 + c * 27 * CI * 32, 128, 256);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        constexpr D2Off kOffs[8] = {d2_off(0), d2_off(1), d2_off(2), d2_off(3),
+                                                    d2_off(4), d2_off(5), d2_off(6), d2_off(7)};
+                        const D2Off o = kOffs[k];
+                        const uint64_t ad = ad0 + (uint64_t)((o.z * 17 + o.y) * 9 + o.x);
+                        const int need = 4 * o.z + 2 * o.y + o.x;
+                        // runs of neighbouring classes
+                        int blk = o.first;
+#pragma unroll
+                        for (int cls = 0; cls < 8; ++cls) {
+                            if ((cls & need) != need || (cls > 0 && ((cls - 1) & need) == need)) continue;
+                            int run = 1;
+#pragma unroll
+                            for (int e = 1; e < 8; ++e)
+                                if (run == e && cls + e < 8 && ((cls + e) & need) == need) run = e + 1;
+                            mma_bf16(acc + (uint32_t)(cls * CI), ad, bd0 + (uint64_t)(blk * (CI * 2)),
+                                     idesc_bf16(128, run * CI), c > 0 || k > 0 ? 1u : 0u);
+                            blk += run;
+                        }
+                    }
+                }
+                tc_commit(saddr(empty + s));
+                tc_commit(saddr(tfull + b));
+            }
+            __syncwarp();
+        }
+        // the MMAs issued are done before the shared and tensor memory go
+        if (it > 0) mbar_wait(saddr(empty + (it - 1) % NS), (uint32_t)(((it - 1) / NS) & 1));
+        __syncwarp();
+    } else {
+        // ---- epilogue: lane = coarse voxel (rows y = 4 w + lane / 8, x = lane % 8), columns = (class, channel)
+        const int m = 32 * warp + lane;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+            const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby), b = it & 1;
+            ok = mbar_wait(saddr(tfull + b), (uint32_t)((it / 2) & 1));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int gx = 2 * (bx * TX + (m & 7)), gy = 2 * (by * TY + (m >> 3)), gz = 2 * bz;
+#pragma unroll
+            for (int pass = 0; pass < (int)ACC / 64; ++pass) {
+                uint32_t r[4][16];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    tc_ld16_issue(tmem + ((uint32_t)(32 * warp) << 16) + b * ACC + (uint32_t)(pass * 64 + k * 16), r[k]);
+                tc_ld_wait(r);
+                if (pass == (int)ACC / 64 - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(saddr(tempty + b));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int col = pass * 64 + k * 16, cls = col / CI, c16 = col % CI / 16;
+                    const int x = gx + (cls & 1), y = gy + ((cls >> 1) & 1), z = gz + (cls >> 2);
+                    if (x < W && y < H && z < D) {
+                        float v[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[k][e]);
+                        store16(v, nullptr, 0, dx, nullptr, (((int64_t)z * H + y) * W + x) * ci + c0 + c16 * 16);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    if (!ok && lane == 0) atomicOr(&g_conv_tc_flags, 1u);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // Weight gradient dW[o][t][c] += sum over output voxels m of
 // dY[m][o] X[src(m, t)][c] (kernel size 3, stride 1 or 2, or kernel size 1).
 // A contraction over the voxels with few rows and columns (co x ci of 16 to
@@ -916,6 +1131,21 @@ cudaError_t launch_pipe(const bf16* x, const bf16* w, const float* bias, bf16* y
     return cudaGetLastError();
 }
 
+template <int CI>
+cudaError_t launch_dx2(const bf16* dy, const bf16* wt, bf16* dx, int D, int H, int W, int ci, int co, cudaStream_t st) {
+    const int Do = (D - 1) / 2 + 1, Ho = (H - 1) / 2 + 1, Wo = (W - 1) / 2 + 1;
+    const int64_t tiles = (int64_t)Do * lbm::ceil_div(Ho, TY) * lbm::ceil_div(Wo, TX);
+    static_assert(kPipeBars + 27 * 32 * 2 * 64 + 2 * 8 * kD2Half <= 227 * 1024, "64 channels of dY, 32 of dx");
+    const PipeShape p = pipe_shape(kPipeBars + 27 * CI * 2 * co, co / 8 * kD2Half);
+    cudaError_t e = cudaFuncSetAttribute(k_conv3_dx2<CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    const int parts = ci / CI;
+    const int64_t per = lbm::ceil_div(tiles, 152 / parts);
+    k_conv3_dx2<CI><<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)parts), kPipeThreads, p.bytes, st>>>(
+        dy, wt, dx, D, H, W, ci, Do, Ho, Wo, co, (int)tiles, p.stages);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 namespace lbm {
@@ -942,6 +1172,19 @@ cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, 
     }
     return co == 16 ? launch_pipe<16>(xb, wb, bias, yb, y32, D, H, W, ci, co, relu, st)
                     : launch_pipe<32>(xb, wb, bias, yb, y32, D, H, W, ci, co, relu, st);
+}
+
+bool conv3_dx2_applies(int D, int H, int W, int ci, int co) {
+    const bool ch = (ci == 16 || ci == 32 || ci == 64) && (co == 16 || co == 32 || co == 64);
+    return ch && D > 0 && H > 0 && W > 0 &&
+           ((int64_t)(D + 1) / 2) * ceil_div((H + 1) / 2, TY) * ceil_div((W + 1) / 2, TX) <= 0x7fffffffLL;
+}
+
+cudaError_t conv3_dx2(const void* dy, const void* wt, void* dx, int D, int H, int W, int ci, int co, cudaStream_t st) {
+    const bf16* db = static_cast<const bf16*>(dy);
+    const bf16* wb = static_cast<const bf16*>(wt);
+    return ci == 16 ? launch_dx2<16>(db, wb, static_cast<bf16*>(dx), D, H, W, ci, co, st)
+                    : launch_dx2<32>(db, wb, static_cast<bf16*>(dx), D, H, W, ci, co, st);
 }
 
 bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride) {

@@ -251,6 +251,10 @@ bool conv3_tc_applies(int D, int H, int W, int ci, int co, int stride);
 cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, const float* bias, int co, int relu,
                      void* y, float* y32, int stride, cudaStream_t st);
 cudaError_t conv3_flip_transpose(const void* w, void* wt, int co, int ci, cudaStream_t st);
+// Input gradient of a 3x3x3 stride-2 convolution (input grid D x H x W, any)
+// on tcgen05; wt: the weights as [ci][27][co].
+bool conv3_dx2_applies(int D, int H, int W, int ci, int co);
+cudaError_t conv3_dx2(const void* dy, const void* wt, void* dx, int D, int H, int W, int ci, int co, cudaStream_t st);
 // Weight gradient dw += dL/dw of a 3x3x3 (stride 1 or 2) or 1x1x1
 // convolution from staged tiles (conv_tc.cu), any grid.
 bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride);

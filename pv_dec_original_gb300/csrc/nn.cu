@@ -6,8 +6,8 @@
 // Activations are BF16, channels-last (voxel-major, channel counts padded to
 // multiples of 16); weights are BF16 [co][tap][ci] with an FP32 master copy
 // for Adam; every product accumulates in FP32 on the tensor cores.  The
-// 3x3x3 forward convolutions and stride-1 input gradients run on tcgen05
-// where the grid tiles, the weight gradients on staged tiles (conv_tc.cu);
+// 3x3x3 forward convolutions (at stride 2 where the grid tiles) and input
+// gradients run on tcgen05, the weight gradients on staged tiles (conv_tc.cu);
 // the kernels here (mma.sync m16n8k16 BF16) take the rest and the comparison engine
 // (lbm_nn_set_conv_engine).  A convolution is an implicit GEMM:
 //   forward      rows = output voxels, cols = output channels, K = taps x ci
@@ -694,9 +694,9 @@ bool padded16(int c) { return c == 16 || c == 32 || c == 64; }  // the channel c
 // apply, or mma.sync everywhere.
 std::atomic<int> g_engine{LBM_NN_ENGINE_AUTO};
 
-// 3x3x3 on shapes the tensor-core kernels tile (conv_tc.cu): the forward
-// convolution at stride 1 or 2, the input gradient at stride 1 (the weight
-// gradient: conv_wgrad_tiles_applies).
+// 3x3x3 on shapes the tensor-core kernels take (conv_tc.cu): the forward
+// convolution at stride 1 or 2, the input gradient at stride 1 (at stride 2:
+// conv3_dx2_applies; the weight gradient: conv_wgrad_tiles_applies).
 bool use_tc(const Conv& g) {
     return g_engine.load() == LBM_NN_ENGINE_AUTO && g.ks == 3 &&
            lbm::conv3_tc_applies(g.D, g.H, g.W, g.ci, g.co, g.stride);
@@ -829,7 +829,11 @@ lbm_status lbm_nn_conv3d_bwd(const void* x, const int dims_in[3], int ci, const 
         const int64_t nw = (int64_t)co * taps * ci;
         k_transpose_w<<<grid1(nw), 256, 0, st>>>(static_cast<const bf16*>(w), static_cast<bf16*>(w_t), co, taps, ci);
         e = cudaGetLastError();
-        if (e == cudaSuccess)
+        if (e != cudaSuccess) {
+        } else if (g_engine.load() == LBM_NN_ENGINE_AUTO && ksize == 3 && stride == 2 &&
+                   lbm::conv3_dx2_applies(g.D, g.H, g.W, ci, co))
+            e = lbm::conv3_dx2(dy, w_t, dx, g.D, g.H, g.W, ci, co, st);
+        else
             e = launch_gemm<1>(ci, static_cast<const bf16*>(dy), static_cast<const bf16*>(w_t), nullptr,
                                static_cast<bf16*>(dx), nullptr, g, rows_in, co, 0, st);
     }
