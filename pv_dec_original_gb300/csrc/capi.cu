@@ -1032,14 +1032,7 @@ lbm_status lbm_set_normals_from_surface(lbm_handle* h, const double* tri12, int6
     if (ntri > 0) e = cudaMemcpyAsync(d_tri, tri12, sizeof(double) * 12 * ntri, cudaMemcpyHostToDevice, h->st);
     if (e == cudaSuccess)
         e = surface_normals(d_tri, ntri, h->g.nw_pt, h->g.nnw, h->nx, h->ny, h->d.origin, h->d.spacing, h->nw_n, h->st);
-    if (e == cudaSuccess && h->g.nnw > 0) {
-        // FP32 copy for the FP32-arithmetic formats
-        std::vector<double> nd(3 * h->g.nnw);
-        e = cudaMemcpyAsync(nd.data(), h->nw_n, sizeof(double) * nd.size(), cudaMemcpyDeviceToHost, h->st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-        const std::vector<float> nf = float_normals(nd, h->g.nnw, h->nw_stride);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h->nw_nf, nf.data(), sizeof(float) * nf.size(), cudaMemcpyHostToDevice, h->st);
-    }
+    if (e == cudaSuccess) e = normals_to_float(h->nw_n, h->g.nnw, h->nw_stride, h->nw_nf, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
     cudaFree(d_tri);
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("normals: ") + cudaGetErrorString(e));
@@ -1075,27 +1068,19 @@ lbm_status lbm_set_normals_from_surface_box(lbm_handle* h, const double* tri12, 
     const int64_t m = (int64_t)sel_pt.size();
     if (m == 0) return LBM_OK;
     double* d_tri = nullptr;
-    int64_t* d_pt = nullptr;
+    int64_t* d_pt = nullptr;  // points, then their places in the next-to-wall list
     double* d_out = nullptr;
     cudaError_t e = cudaMalloc(&d_tri, sizeof(double) * 12 * (ntri > 0 ? ntri : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&d_pt, sizeof(int64_t) * m);
+    if (e == cudaSuccess) e = cudaMalloc(&d_pt, sizeof(int64_t) * 2 * m);
     if (e == cudaSuccess) e = cudaMalloc(&d_out, sizeof(double) * 3 * m);
     if (e == cudaSuccess && ntri > 0)
         e = cudaMemcpyAsync(d_tri, tri12, sizeof(double) * 12 * ntri, cudaMemcpyHostToDevice, h->st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_pt, sel_pt.data(), sizeof(int64_t) * m, cudaMemcpyHostToDevice, h->st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(d_pt + m, sel_idx.data(), sizeof(int64_t) * m, cudaMemcpyHostToDevice, h->st);
     if (e == cudaSuccess) e = surface_normals(d_tri, ntri, d_pt, m, h->nx, h->ny, h->d.origin, h->d.spacing, d_out, h->st);
-    std::vector<double> part(3 * m), nd(3 * nn);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(part.data(), d_out, sizeof(double) * 3 * m, cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(nd.data(), h->nw_n, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-    std::vector<float> nf;
-    if (e == cudaSuccess) {
-        for (int64_t k = 0; k < m; ++k)
-            for (int a = 0; a < 3; ++a) nd[a * nn + sel_idx[k]] = part[a * m + k];
-        nf = float_normals(nd, nn, h->nw_stride);
-        e = cudaMemcpyAsync(h->nw_n, nd.data(), sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, h->st);
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h->nw_nf, nf.data(), sizeof(float) * nf.size(), cudaMemcpyHostToDevice, h->st);
+    if (e == cudaSuccess) e = scatter_normals(d_out, d_pt + m, m, nn, h->nw_n, h->st);
+    if (e == cudaSuccess) e = normals_to_float(h->nw_n, nn, h->nw_stride, h->nw_nf, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
     cudaFree(d_tri);
     cudaFree(d_pt);

@@ -227,6 +227,11 @@ cudaError_t exclusive_scan_i64(const int64_t* d_in, int64_t* d_out, int64_t n, i
 cudaError_t surface_normals(const double* d_tri, int64_t ntri, const int64_t* d_pts, int64_t npts, int nx, int ny,
                             const double origin[3], double spacing, double* d_out, cudaStream_t s);
 
+// m normals ([3][m]) into places idx of the list n ([3][nn]); n's FP32 copy in
+// planes of `stride` (zero past nn).
+cudaError_t scatter_normals(const double* part, const int64_t* idx, int64_t m, int64_t nn, double* n, cudaStream_t s);
+cudaError_t normals_to_float(const double* n, int64_t nn, int64_t stride, float* out, cudaStream_t s);
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Entries per pull-segment row of the delta table: Q offsets padded to a
