@@ -28,6 +28,7 @@ UNITS = [
     ("scan.cu", True),
     ("voxelize.cu", False),
     ("setup.cu", False),
+    ("segments.cu", True),
     ("step_f64.cu", False),
     ("step_f32.cu", True),
     ("step_f16.cu", True),

@@ -599,142 +599,16 @@ void reference_bbox(const double* t, int64_t ntri, double spacing, double* bb, i
     dims[2] = (int)std::ceil((mxz - mnz) / spacing);
 }
 
-// Pull segments.  With populations stored by active index a, the source of
-// population q at node a is the active index of point x_a - c_q.  Along an
-// x-run that index is a + delta_q with delta_q constant; a segment is a
-// maximal stretch of consecutive active nodes whose valid (non-missing)
-// offsets agree for every q.  Output: per active node its segment, per
-// segment Q offsets (0 where no node of the segment has that source), each
-// row padded with zeros to kDeltaRow<Q> entries so that the step kernel
-// reads it with 16-byte loads.
-template <int Q>
-void build_segments_q(const uint8_t* mask, int nx, int ny, int nz, int64_t& nact, std::vector<int32_t>& seg_of,
-                      std::vector<int32_t>& delta) {
-    const int64_t nxy = (int64_t)nx * ny, npts = nxy * nz;
-    std::vector<int32_t> aidx((size_t)npts);
-    int64_t a = 0;
-    for (int64_t n = 0; n < npts; ++n) aidx[n] = mask[n] ? (int32_t)a++ : -1;
-    nact = a;
-    seg_of.assign((size_t)nact, 0);
-    delta.clear();
-    int32_t cur[Q];
-    bool has[Q];
-    int64_t seg = -1;
-    auto flush = [&]() {
-        for (int q = 0; q < Q; ++q) delta.push_back(has[q] ? cur[q] : 0);
-        for (int q = Q; q < kDeltaRow<Q>; ++q) delta.push_back(0);
-    };
-    for (int k = 0; k < nz; ++k)
-        for (int j = 0; j < ny; ++j)
-            for (int i = 0; i < nx; ++i) {
-                const int64_t n = (int64_t)k * nxy + (int64_t)j * nx + i;
-                if (!mask[n]) continue;
-                const int32_t an = aidx[n];
-                int32_t d[Q];
-                bool v[Q];
-                bool fresh = seg < 0;
-                for (int q = 0; q < Q; ++q) {
-                    const int x = i - Lat<Q>::cx(q), y = j - Lat<Q>::cy(q), z = k - Lat<Q>::cz(q);
-                    v[q] = x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz &&
-                           mask[(int64_t)z * nxy + (int64_t)y * nx + x];
-                    d[q] = v[q] ? aidx[(int64_t)z * nxy + (int64_t)y * nx + x] - an : 0;
-                    if (!fresh && v[q] && has[q] && d[q] != cur[q]) fresh = true;
-                }
-                if (fresh) {
-                    if (seg >= 0) flush();
-                    ++seg;
-                    for (int q = 0; q < Q; ++q) has[q] = false;
-                }
-                for (int q = 0; q < Q; ++q)
-                    if (v[q] && !has[q]) { cur[q] = d[q]; has[q] = true; }
-                seg_of[an] = (int32_t)seg;
-            }
-    if (seg >= 0) flush();
-}
-
-void build_segments(int Q, const uint8_t* mask, int nx, int ny, int nz, int64_t& nact, std::vector<int32_t>& seg_of,
-                    std::vector<int32_t>& delta) {
-    if (Q == 19) build_segments_q<19>(mask, nx, ny, nz, nact, seg_of, delta);
-    else build_segments_q<27>(mask, nx, ny, nz, nact, seg_of, delta);
-}
-
-// FP32 copy of the normals [3][nn] with plane stride `stride`.
-std::vector<float> float_normals(const std::vector<double>& nd, int64_t nn, int64_t stride) {
-    std::vector<float> nf(3 * stride, 0.f);
-    for (int a = 0; a < 3; ++a)
-        for (int64_t k = 0; k < nn; ++k) nf[a * stride + k] = (float)nd[a * nn + k];
-    return nf;
-}
-
-// Plan of the tiled step kernel: per tile of kTileNodes active nodes and
-// population plane q, the window of plane q holding every valid pull source
-// of the tile's nodes (widened to 16-byte boundaries); the tile's pull
-// segments and next-to-wall entries; the shared-memory layout of a pipeline
-// stage.  Returns false (no plan) when a stage does not fit.
-template <int Q>
-bool build_tile_plan_q(const uint8_t* mask, int nx, int ny, int nz, int64_t nact, int64_t stride, int es,
-                       const std::vector<int32_t>& seg_of, const std::vector<int32_t>& delta,
-                       const std::vector<int32_t>& sp_of_act, int64_t nnw, std::vector<int32_t>& plan, TileGeom& G) {
-    constexpr int T = kTileNodes, DR = kDeltaRow<Q>, PI = 2 * Q + kTilePlanExtra;
-    const int A = 16 / es;  // elements per 16 bytes
-    const int64_t ntiles = ceil_div(nact, T);
-    const int64_t nxy = (int64_t)nx * ny;
-    std::vector<int64_t> lo((size_t)ntiles * Q, INT64_MAX), hi((size_t)ntiles * Q, -1);
-    int64_t an = 0;
-    for (int k = 0; k < nz; ++k)
-        for (int j = 0; j < ny; ++j)
-            for (int i = 0; i < nx; ++i) {
-                if (!mask[(int64_t)k * nxy + (int64_t)j * nx + i]) continue;
-                const int32_t* d = delta.data() + (int64_t)seg_of[an] * DR;
-                const int64_t t = an / T;
-                for (int q = 0; q < Q; ++q) {
-                    const int x = i - Lat<Q>::cx(q), y = j - Lat<Q>::cy(q), z = k - Lat<Q>::cz(q);
-                    if (x < 0 || x >= nx || y < 0 || y >= ny || z < 0 || z >= nz ||
-                        !mask[(int64_t)z * nxy + (int64_t)y * nx + x])
-                        continue;
-                    const int64_t src = an + d[q];
-                    int64_t& l = lo[t * Q + q];
-                    int64_t& h = hi[t * Q + q];
-                    if (src < l) l = src;
-                    if (src > h) h = src;
-                }
-                ++an;
-            }
-    plan.assign((size_t)ntiles * PI, 0);
-    int64_t wcap = A, segmax = 1, nwcap = 4;
-    for (int64_t t = 0; t < ntiles; ++t) {
-        int32_t* pl = plan.data() + t * PI;
-        for (int q = 0; q < Q; ++q) {
-            const int64_t h = hi[t * Q + q];
-            if (h < 0) continue;
-            const int64_t l0 = lo[t * Q + q] / A * A, h1 = ceil_div(h + 1, A) * A;
-            if (h1 > stride) return false;
-            pl[q] = (int32_t)l0;
-            pl[Q + q] = (int32_t)(h1 - l0);
-            wcap = std::max(wcap, h1 - l0);
-        }
-        const int64_t a0 = t * T, a1 = std::min(nact, a0 + T) - 1;
-        pl[2 * Q] = seg_of[a0];
-        pl[2 * Q + 1] = seg_of[a1] - seg_of[a0] + 1;
-        segmax = std::max<int64_t>(segmax, pl[2 * Q + 1]);
-        int64_t smin = INT64_MAX, smax = -1;
-        for (int64_t a = a0; a <= a1; ++a)
-            if (sp_of_act[a] >= 0 && sp_of_act[a] < nnw) {
-                smin = std::min<int64_t>(smin, sp_of_act[a]);
-                smax = std::max<int64_t>(smax, sp_of_act[a]);
-            }
-        if (smax >= 0) {
-            pl[2 * Q + 2] = (int32_t)(smin / 4 * 4);
-            pl[2 * Q + 3] = (int32_t)(ceil_div(smax + 1, 4) * 4 - smin / 4 * 4);
-            nwcap = std::max<int64_t>(nwcap, pl[2 * Q + 3]);
-        }
-    }
-    const int segcap = (int)std::min<int64_t>(segmax, 64);
-    for (int64_t t = 0; t < ntiles; ++t) {
-        int32_t* pl = plan.data() + t * PI;
-        pl[2 * Q + 1] = std::min(pl[2 * Q + 1], segcap);  // the rest read their rows from global memory
-    }
-    wcap = ceil_div(wcap, 8) * 8;
+// Shared-memory layout of the tiled step kernel from its plan's largest
+// window, segment and next-to-wall counts (build_tile_plan); false when a
+// stage does not fit.
+bool tile_geometry(int Q, int es, int64_t ntiles, const int most[4], TileGeom& G) {
+    constexpr int T = kTileNodes;
+    if (most[3]) return false;
+    const int DR = Q == 19 ? kDeltaRow<19> : kDeltaRow<27>;
+    const int64_t wcap = ceil_div(std::max(most[0], 16 / es), 8) * 8, nwcap = std::max(most[2], 4);
+    const int segcap = std::min(std::max(most[1], 1), 64);
+    if (Q * wcap * es > 232448 || 12 * nwcap > 232448) return false;
     auto al = [](int64_t v) { return (int)ceil_div(v, 128) * 128; };
     TileGeom g{};
     g.ntiles = ntiles;
@@ -752,11 +626,11 @@ bool build_tile_plan_q(const uint8_t* mask, int nx, int ny, int nz, int64_t nact
     // deepest pipeline and most CTAs per SM that fit 227 KB per CTA / 228 KB per SM
     const int choices[4][2] = {{3, 2}, {2, 2}, {3, 1}, {2, 1}};
     for (const auto& c : choices) {
-        const int smem = c[0] * g.stage_bytes + c[0] * 8;
+        const int64_t smem = (int64_t)c[0] * g.stage_bytes + c[0] * 8;
         if (smem <= 232448 && c[1] * (smem + 1024) <= 233472) {
             g.nstage = c[0];
             g.ctas_per_sm = c[1];
-            g.smem_bytes = smem;
+            g.smem_bytes = (int)smem;
             G = g;
             return true;
         }
@@ -900,30 +774,24 @@ lbm_status lbm_set_geometry(lbm_handle* h, const uint8_t* mask, const int dims[3
     free_geometry(h);
     h->nx = dims[0]; h->ny = dims[1]; h->nz = dims[2];
     h->npts = npts;
-    int64_t nact = 0;
-    std::vector<int32_t> seg_of, delta;
-    build_segments(h->d.Q, mask, h->nx, h->ny, h->nz, nact, seg_of, delta);
-    REQUIRE(h, nact < (int64_t)1 << 31, LBM_ERR_ARG, "too many active nodes");
-    h->nseg = (int64_t)delta.size() / (h->d.Q == 19 ? kDeltaRow<19> : kDeltaRow<27>);
-    h->stride = ceil_div(nact > 0 ? nact : 1, 128) * 128;
-    CK(h, dalloc(h, &h->seg_delta, sizeof(int32_t) * (delta.size() + 1)));
-    if (!delta.empty())
-        CK(h, cudaMemcpyAsync(h->seg_delta, delta.data(), sizeof(int32_t) * delta.size(), cudaMemcpyHostToDevice, h->st));
     uint8_t* d_mask = nullptr;
-    int32_t* d_seg = nullptr;
+    int32_t* seg_of = nullptr;  // segment of every active node (set-up only)
     CK(h, cudaMalloc(&d_mask, npts));
-    cudaError_t e = cudaMalloc(&d_seg, sizeof(int32_t) * (nact + 1));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_mask, mask, npts, cudaMemcpyHostToDevice, h->st);
-    if (e == cudaSuccess && nact)
-        e = cudaMemcpyAsync(d_seg, seg_of.data(), sizeof(int32_t) * nact, cudaMemcpyHostToDevice, h->st);
+    cudaError_t e = cudaMemcpyAsync(d_mask, mask, npts, cudaMemcpyHostToDevice, h->st);
     std::string err;
     if (e == cudaSuccess)
-        e = build_geometry(h->d.Q, d_mask, h->nx, h->ny, h->nz, bc, nbc, h->d.origin, h->d.spacing, d_seg, h->g,
-                           h->st, err);
+        e = build_geometry(h->d.Q, d_mask, h->nx, h->ny, h->nz, bc, nbc, h->d.origin, h->d.spacing, h->g,
+                           &h->seg_delta, &h->nseg, &seg_of, h->st, err);
     cudaFree(d_mask);
-    if (d_seg) cudaFree(d_seg);
+    struct Release {  // seg_of goes with every return
+        int32_t*& p;
+        cudaStream_t st;
+        ~Release() { if (p) cudaFreeAsync(p, st); }
+    } release{seg_of, h->st};
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, "set_geometry: " + (err.empty() ? cudaGetErrorString(e) : err));
     REQUIRE(h, h->g.nact < (int64_t)1 << 31, LBM_ERR_ARG, "too many active nodes");
+    h->geo_bytes += sizeof(int32_t) * (h->nseg * (h->d.Q == 19 ? kDeltaRow<19> : kDeltaRow<27>) + 1);
+    h->stride = ceil_div(h->g.nact > 0 ? h->g.nact : 1, 128) * 128;
     h->nbc = nbc;
     h->bc.assign(nbc, BCDev{});
     for (int b = 0; b < nbc; ++b) {
@@ -1000,21 +868,20 @@ lbm_status lbm_set_geometry(lbm_handle* h, const uint8_t* mask, const int dims[3
     h->counts = c;
     // plan of the tiled step kernel (physics mode, FP32-arithmetic formats)
     if (h->d.mode == LBM_PHYSICS && h->d.precision != LBM_F64 && h->g.nact > 0) {
-        std::vector<int32_t> spa(h->g.nact);
-        CK(h, cudaMemcpyAsync(spa.data(), h->g.sp_of_act, sizeof(int32_t) * h->g.nact, cudaMemcpyDeviceToHost, h->st));
-        CK(h, cudaStreamSynchronize(h->st));
-        std::vector<int32_t> plan;
+        const int64_t ntiles = ceil_div(h->g.nact, kTileNodes);
+        int32_t* plan = nullptr;
+        const size_t bytes = sizeof(int32_t) * ntiles * (2 * Q + kTilePlanExtra);
+        CK(h, cudaMalloc(&plan, bytes));
+        int most[4];
         TileGeom G{};
-        const int es = (int)elem_size(h->d.precision);
-        const bool ok = Q == 19 ? build_tile_plan_q<19>(mask, h->nx, h->ny, h->nz, h->g.nact, h->stride, es, seg_of,
-                                                         delta, spa, h->g.nnw, plan, G)
-                                : build_tile_plan_q<27>(mask, h->nx, h->ny, h->nz, h->g.nact, h->stride, es, seg_of,
-                                                         delta, spa, h->g.nnw, plan, G);
+        cudaError_t te = build_tile_plan(Q, h->g, h->nx, h->ny, h->nz, seg_of, h->stride, (int)es, plan, most, h->st);
+        const bool ok = te == cudaSuccess && tile_geometry(Q, (int)es, ntiles, most, G);
+        if (ok) te = cap_tile_segments(Q, plan, ntiles, G.segcap, h->st);
+        if (te != cudaSuccess || !ok) cudaFree(plan);
+        if (te != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("tile plan: ") + cudaGetErrorString(te));
         if (ok) {
-            CK(h, dalloc(h, &h->tile_plan, sizeof(int32_t) * plan.size()));
-            CK(h, cudaMemcpyAsync(h->tile_plan, plan.data(), sizeof(int32_t) * plan.size(), cudaMemcpyHostToDevice,
-                                  h->st));
-            CK(h, cudaStreamSynchronize(h->st));
+            h->tile_plan = plan;
+            h->geo_bytes += bytes;
             h->tile = G;
         }
     }

@@ -42,12 +42,26 @@ __global__ void k_boundary(const uint8_t* __restrict__ mask, int nx, int ny, int
 
 // Extreme fluid layer per axis: ext[0..2] = min index, ext[3..5] = max index.
 __global__ void k_extent(const uint8_t* __restrict__ mask, int nx, int ny, int nz, int* __restrict__ ext) {
-    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // warps reduce before their atomics (6 words for the whole lattice)
     const int64_t npts = (int64_t)nx * ny * nz;
-    if (n >= npts || !mask[n]) return;
-    const int i = (int)(n % nx), j = (int)((n / nx) % ny), k = (int)(n / ((int64_t)nx * ny));
-    atomicMin(ext + 0, i); atomicMin(ext + 1, j); atomicMin(ext + 2, k);
-    atomicMax(ext + 3, i); atomicMax(ext + 4, j); atomicMax(ext + 5, k);
+    int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-1, -1, -1};
+    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < npts; n += (int64_t)gridDim.x * blockDim.x) {
+        if (!mask[n]) continue;
+        const int c[3] = {(int)(n % nx), (int)((n / nx) % ny), (int)(n / ((int64_t)nx * ny))};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = min(lo[d], c[d]);
+            hi[d] = max(hi[d], c[d]);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int l = __reduce_min_sync(0xffffffffu, lo[d]), h = __reduce_max_sync(0xffffffffu, hi[d]);
+        if ((threadIdx.x & 31) == 0 && h >= 0) {
+            atomicMin(ext + d, l);
+            atomicMax(ext + 3 + d, h);
+        }
+    }
 }
 
 struct Rules {
@@ -187,25 +201,26 @@ __global__ void k_active_flags(const uint8_t* __restrict__ cls, int64_t npts, in
     flag[n] = cls[n] != CLS_SOLID ? 1 : 0;
 }
 
-// Per active node: index maps and the step kernel's packed word
+// Per active node: index maps.
+__global__ void k_active_index(const int64_t* __restrict__ flag, const int64_t* __restrict__ pos, int64_t npts,
+                               int32_t* __restrict__ act_idx, int64_t* __restrict__ act_pt) {
+    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= npts) return;
+    const bool f = flag[n] != 0;
+    act_idx[n] = f ? (int32_t)pos[n] : -1;
+    if (f) act_pt[pos[n]] = n;
+}
+
+// Per active node: the step kernel's packed word
 // (segment | special << 31 | missing mask << 32 | class << 59 | next-to-wall << 63).
 template <int Q>
-__global__ void k_active_index(const int64_t* __restrict__ flag, const int64_t* __restrict__ pos,
-                               const int64_t* __restrict__ spflag, const int64_t* __restrict__ sppos,
-                               const uint8_t* __restrict__ cls, int nx, int ny, int nz,
-                               const int32_t* __restrict__ seg_of_act, int32_t* __restrict__ act_idx,
-                               int64_t* __restrict__ act_pt,
-                               uint64_t* __restrict__ act_word, int32_t* __restrict__ sp_of_act) {
-    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t npts = (int64_t)nx * ny * nz;
-    if (n >= npts) return;
-    if (!flag[n]) {
-        act_idx[n] = -1;
-        return;
-    }
-    const int64_t a = pos[n];
-    act_idx[n] = (int32_t)a;
-    act_pt[a] = n;
+__global__ void k_active_word(const int64_t* __restrict__ act_pt, int64_t nact, const int64_t* __restrict__ spflag,
+                              const int64_t* __restrict__ sppos, const uint8_t* __restrict__ cls, int nx, int ny,
+                              int nz, const int32_t* __restrict__ seg_of_act, uint64_t* __restrict__ act_word,
+                              int32_t* __restrict__ sp_of_act) {
+    const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= nact) return;
+    const int64_t n = act_pt[a];
     const int i = (int)(n % nx), j = (int)((n / nx) % ny), k = (int)(n / ((int64_t)nx * ny));
     uint64_t miss = 0;
 #pragma unroll
@@ -355,8 +370,8 @@ inline unsigned blocks(int64_t n, int t = 256) { return (unsigned)ceil_div(n > 0
     } while (0)
 
 cudaError_t build_geometry(int Q, const uint8_t* d_mask, int nx, int ny, int nz, const lbm_bc_spec* bc, int nbc,
-                           const double origin[3], double spacing, const int32_t* d_seg_of_act, GeometryLists& out,
-                           cudaStream_t st, std::string& err) {
+                           const double origin[3], double spacing, GeometryLists& out, int32_t** seg_rows,
+                           int64_t* nseg, int32_t** seg_of, cudaStream_t st, std::string& err) {
     const int64_t npts = (int64_t)nx * ny * nz;
     out.npts = npts;
     // padded to whole 32-point segments: the bulk kernel reads the class
@@ -379,7 +394,7 @@ cudaError_t build_geometry(int Q, const uint8_t* d_mask, int nx, int ny, int nz,
         int init[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, -1, -1, -1};
         SETUP_CHECK(cudaMallocAsync(&d_ext, sizeof(init), st));
         SETUP_CHECK(cudaMemcpyAsync(d_ext, init, sizeof(init), cudaMemcpyHostToDevice, st));
-        k_extent<<<blocks(npts), 256, 0, st>>>(d_mask, nx, ny, nz, d_ext);
+        k_extent<<<std::min(blocks(npts), 608u), 256, 0, st>>>(d_mask, nx, ny, nz, d_ext);
         SETUP_CHECK(cudaMemcpyAsync(ext, d_ext, sizeof(ext), cudaMemcpyDeviceToHost, st));
         SETUP_CHECK(cudaStreamSynchronize(st));
         cudaFreeAsync(d_ext, st);
@@ -458,12 +473,16 @@ cudaError_t build_geometry(int Q, const uint8_t* d_mask, int nx, int ny, int nz,
     SETUP_CHECK(cudaMallocAsync(&out.act_word, sizeof(uint64_t) * (out.nact + 1), st));
     // padded: the tiled step kernel copies whole 16-byte groups
     SETUP_CHECK(cudaMallocAsync(&out.sp_of_act, sizeof(int32_t) * (out.nact + 4), st));
+    k_active_index<<<blocks(npts), 256, 0, st>>>(aflag, apos, npts, out.act_idx, out.act_pt);
+    SETUP_CHECK(cudaGetLastError());
+    SETUP_CHECK(cudaMallocAsync(seg_of, sizeof(int32_t) * (out.nact + 1), st));
+    SETUP_CHECK(build_segments(Q, out, nx, ny, nz, seg_rows, nseg, *seg_of, st));
     if (Q == 19)
-        k_active_index<19><<<blocks(npts), 256, 0, st>>>(aflag, apos, flag, pos, out.cls, nx, ny, nz, d_seg_of_act,
-                                                         out.act_idx, out.act_pt, out.act_word, out.sp_of_act);
+        k_active_word<19><<<blocks(out.nact), 256, 0, st>>>(out.act_pt, out.nact, flag, pos, out.cls, nx, ny, nz, *seg_of,
+                                                           out.act_word, out.sp_of_act);
     else
-        k_active_index<27><<<blocks(npts), 256, 0, st>>>(aflag, apos, flag, pos, out.cls, nx, ny, nz, d_seg_of_act,
-                                                         out.act_idx, out.act_pt, out.act_word, out.sp_of_act);
+        k_active_word<27><<<blocks(out.nact), 256, 0, st>>>(out.act_pt, out.nact, flag, pos, out.cls, nx, ny, nz, *seg_of,
+                                                           out.act_word, out.sp_of_act);
     SETUP_CHECK(cudaGetLastError());
     cudaFreeAsync(aflag, st);
     cudaFreeAsync(apos, st);

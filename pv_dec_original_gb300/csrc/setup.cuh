@@ -36,10 +36,22 @@ struct GeometryLists {
     int plane[LBM_MAX_BC] = {0};
 };
 
-// d_seg_of_act: per active node, its pull segment (see capi.cu build_segments).
+// seg_rows / nseg / seg_of: the pull segments (segments.cu): cudaMalloc'ed
+// rows of kDeltaRow<Q> offsets, and the segment of every active node
+// (cudaMallocAsync'ed; the caller frees it).
 cudaError_t build_geometry(int Q, const uint8_t* d_mask, int nx, int ny, int nz, const lbm_bc_spec* bc, int nbc,
-                           const double origin[3], double spacing, const int32_t* d_seg_of_act, GeometryLists& out,
-                           cudaStream_t st, std::string& err);
+                           const double origin[3], double spacing, GeometryLists& out, int32_t** seg_rows,
+                           int64_t* nseg, int32_t** seg_of, cudaStream_t st, std::string& err);
+
+// Pull segments of the active nodes (act_idx, act_pt): rows cudaMalloc'ed.
+cudaError_t build_segments(int Q, const GeometryLists& g, int nx, int ny, int nz, int32_t** rows, int64_t* nseg,
+                           int32_t* seg_of, cudaStream_t st);
+// Plan of the tiled step kernel, 2 Q + kTilePlanExtra int32 per tile; most:
+// the largest source window (elements), segment count and next-to-wall entry
+// count of a tile, and whether a window leaves its plane.
+cudaError_t build_tile_plan(int Q, const GeometryLists& g, int nx, int ny, int nz, const int32_t* seg_of,
+                            int64_t stride, int elem_size, int32_t* plan, int most[4], cudaStream_t st);
+cudaError_t cap_tile_segments(int Q, int32_t* plan, int64_t ntiles, int cap, cudaStream_t st);
 
 // Nearest next-to-wall node (index into the next-to-wall list, -1 if none
 // within rmax lattice spacings) and its distance of each of nv points xyz
