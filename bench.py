@@ -735,7 +735,7 @@ def read_traffic(name, variant):
     p = os.path.join(ROOT, "profiles", name)
     if not os.path.exists(p):
         return None
-    key = "traffic_bytes_per_launch[%s]" % ("compact" if variant in (6, 7) else "flat")
+    key = "traffic_bytes_per_launch[%s]" % ("compact" if variant in (3, 4, 6, 7) else "flat")
     for line in open(p):
         if line.startswith(key):
             try:
@@ -986,7 +986,7 @@ def run_ours(args):
                             "the read-back copies of one batch overlap the next batch's steps)"},
             "gpu_launches": launches,
             "autotune": {"variant": tuned[0], "ms_per_step_by_variant": tuned[1],
-                         "variants": "(block, min blocks/SM): (128,12) (128,10) (128,8) (256,3) (256,1); 5: tiled bulk-copy kernel"},
+                         "variants": "(block, min blocks/SM): flat (128,12) (128,10) (128,8); compact (256,4) (128,8); 5: tiled bulk-copy kernel; compact (128,10) (128,12)"},
             "clocks": clk.summary(),
             "extra": extra,
         }

@@ -331,15 +331,16 @@ lbm_status lbm_preset_barrier(lbm_handle* h, unsigned extra_arrivals);
 #define LBM_FLAG_BOUNDS 4
 lbm_status lbm_preset_flags(lbm_handle* h, unsigned flags);
 
-/* Launch-shape variants of the step kernel: one node per thread with
- * (block size, minimum resident blocks per SM) = (128,12) (128,10) (128,8)
- * (256,3) (256,1), the last (64,8) in FP64; variant 5, the tiled kernel (bulk copies stage each
- * 256-node tile's sources in shared memory; physics mode, FP32 / FP16 /
- * BF16; elsewhere it runs variant 0, or 4 for FP64); variants 6 (128,10)
- * and 7 (128,12), the compact kernel (32 bytes of node metadata per warp of
- * 32 nodes instead of 12 bytes a node; physics mode, FP32 / FP16 / BF16,
- * half-way bounce-back; elsewhere variant 0).  A new handle starts on
- * variant 0, FP64 on variant 4.  lbm_autotune times each variant for
+/* Launch-shape variants of the step kernel, as (block size, minimum resident
+ * blocks per SM).  0 (128,12), 1 (128,10), 2 (128,8): the flat kernel, one node
+ * per thread.  3 (256,4), 4 (128,8), 6 (128,10), 7 (128,12): the compact kernel
+ * (32 bytes of node metadata per warp of 32 nodes instead of 12 bytes a node;
+ * physics mode, FP32 / FP16 / BF16, half-way bounce-back); elsewhere flat: 3
+ * (256,3), 4 (256,1) or in FP64 (64,8), 6 and 7 variant 0.  5: the tiled kernel
+ * (bulk copies stage each 256-node tile's sources in shared memory; physics mode,
+ * FP32 / FP16 / BF16; elsewhere variant 0, or 4 for FP64).  A handle on which
+ * none was set takes one by its lattice, precision and number of nodes.
+ * lbm_autotune times each variant for
  * trial_steps steps on a snapshot of the current state, restores the
  * state, keeps the fastest and reports it (and, if ms_per_step is not NULL,
  * the time of every variant: LBM_NUM_VARIANTS floats).  No reference

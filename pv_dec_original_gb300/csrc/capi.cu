@@ -92,7 +92,7 @@ struct lbm_handle {
     cudaGraphExec_t gexec = nullptr;
     int gexec_parity = -1;
     int gexec_cur = -1;
-    int variant = 0;            // launch shape of the step kernel (lbm_autotune)
+    int variant = -1;           // launch shape of the step kernel (lbm_autotune); -1: default_variant's
     size_t geo_bytes = 0;
     lbm_counts counts{};
 };
@@ -278,6 +278,7 @@ StepParams make_params(lbm_handle* h, int kind) {
         p.fin = h->since_start == 0 ? h->buf[0] : h->buf[1 - h->cur];
         p.direct = h->since_start == 0 ? 1 : 0;
     }
+    p.odd = h->cur;
     p.stride = h->stride;
     p.seg_delta = h->seg_delta;
     p.seg_abs = h->seg_abs;
@@ -711,9 +712,6 @@ lbm_status lbm_create(const lbm_desc* desc, lbm_handle** out) {
     lbm_handle* h = new lbm_handle();
     h->d = *desc;
     if (h->d.tawss_div == 0.0) h->d.tawss_div = 0.9;
-    // FP64 keeps every population in two registers: start it on the
-    // unconstrained shape, the FP32-arithmetic formats on the 40-register one
-    h->variant = h->d.precision == LBM_F64 ? 4 : 0;
     e = cudaSetDevice(desc->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&h->slots, 2 * sizeof(int64_t));

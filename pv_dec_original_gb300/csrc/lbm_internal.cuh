@@ -120,6 +120,8 @@ struct StepParams {
     float* nw_ring;           // float4 [kRingSlots][nnw]: step s in slot s % kRingSlots
     int64_t fold_blocks;      // leading blocks of a step launch that fold the ring, or (FP64) compute the
                               // next-to-wall stress (set by the launcher)
+    int odd;                  // which of the two buffers fin is
+    int stream, reverse;      // compact step kernel, set by its launcher: evict-first loads, blocks in the other order
     int pdl_early;            // step launch: let the next launch begin at block start (else at block end)
     float2* nw_accf;          // [4][nnw]
     void* nw_prev;            // parity: rho, ux, uy, uz of the previous collision, [4][nnw]

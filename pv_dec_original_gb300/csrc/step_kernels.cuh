@@ -1263,6 +1263,30 @@ __global__ void __launch_bounds__(BT, MINB) step_kernel(const StepParams P) {
 // rows and masks beside the lane masks (prefetched to L1, or both rows in
 // registers) did not shorten the step (FP32 30.7 / 37.1 us against 30.3 us,
 // FP16 28.7 / 33.8 against 26.5 us), so the chain is not what bounds it.
+//
+// What bounds it is the populations' traffic, and how much of it L2 keeps from
+// one step to the next: a step reads the buffer that the step before wrote.
+// P.stream loads the populations evict-first: a line read is dead (the next
+// step overwrites it), and leaving it early keeps what this step writes for the
+// next one's reads.  P.reverse runs the blocks in the other order on every
+// second step: what the step before wrote last is read first.  The rule for
+// both is at launch_compact.
+template <typename S>
+__device__ __forceinline__ S load_hinted(const S* p, uint64_t policy) {
+    if constexpr (sizeof(S) == 4) {
+        float v;
+        asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+        return v;
+    } else {
+        static_assert(sizeof(S) == 2, "FP32, FP16 or BF16");
+        unsigned short v;
+        asm volatile("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(policy));
+        S h;
+        memcpy(&h, &v, 2);
+        return h;
+    }
+}
+
 template <int Q, typename S, int BT, int MINB>
 __global__ void __launch_bounds__(BT, MINB) step_compact_kernel(const StepParams P) {
     using R = typename Store<S>::real;
@@ -1282,6 +1306,7 @@ __global__ void __launch_bounds__(BT, MINB) step_compact_kernel(const StepParams
     {
         // blocks from both ends of the active-node order first (step_kernel)
         const uint32_t nm = (uint32_t)((P.nact + BT - 1) / BT);
+        if (P.reverse) blk = nm - 1 - blk;
         blk = (blk & 1) ? nm - 1 - (blk >> 1) : (blk >> 1);
     }
     const uint32_t a = blk * BT + threadIdx.x;
@@ -1325,13 +1350,17 @@ __global__ void __launch_bounds__(BT, MINB) step_compact_kernel(const StepParams
     if (a < (uint32_t)P.nact) {
         const S* __restrict__ fin = static_cast<const S*>(P.fin);
         const uint32_t st = (uint32_t)P.stride;
+        uint64_t keep, policy;
+        asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(keep));
+        asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+        if (!P.stream) policy = keep;
         R g[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             uint32_t idx = a + (uint32_t)row[q];
             if (q != Lat<Q>::REST && (miss & (1u << Lat<Q>::opp(q)))) idx = a + (uint32_t)Lat<Q>::opp(q) * st;
             if (in_bounds(idx, (int64_t)Q * st, P.flags))
-                g[q] = Store<S>::template load<Q>(fin + idx, q);  // w_opp(q) == w_q: the same decode
+                g[q] = Store<S>::template decode<Q>(load_hinted(fin + idx, policy), q);  // w_opp(q) == w_q: the same decode
             else
                 g[q] = R(0);
         }
@@ -1351,7 +1380,7 @@ __global__ void __launch_bounds__(BT, MINB) step_compact_kernel(const StepParams
 struct Variant {
     int bt, minb;
 };
-constexpr int kFlatVariants = 5;  // 0..4; 5 = tiled
+constexpr int kFlatVariants = 5;  // 0..4 (3, 4: where the compact kernel's do not run); 5 = tiled
 constexpr Variant kVariants[kFlatVariants] = {{128, 12}, {128, 10}, {128, 8}, {256, 3}, {256, 1}};
 // Variant 4 in FP64 (its default; 128 registers): the FP64 pipe is shared by the SM's warps,
 // so an SM's time is its number of warps; blocks of two warps spread a small
@@ -1821,32 +1850,74 @@ cudaError_t launch_tile(const StepParams& p, cudaStream_t st) {
 }
 
 // The compact kernel where its warp blocks exist (physics, FP32-arithmetic
-// formats, 32-bit offsets, half-way bounce-back); the flat kernel's default
-// shape elsewhere.
-template <int Q, typename S, int MODE, int BT, int MB>
+// formats, 32-bit offsets, half-way bounce-back); the flat kernel's shape FB
+// elsewhere.
+//
+// Evict-first loads up to kStreamBytes of one population buffer, the other
+// block order on every second step from kReverseBytes.  L2 holds 129 MB; us a
+// step (tubes; D3Q19 FP32 (128,10), FP16 (128,12), D3Q27 (128,8)), plain /
+// evict-first / the other order / both:
+//   FP32  38 MB 11.78 / 11.24 / - / 11.61       68 MB 23.85 / 18.74 / 22.15 / 19.64
+//         91 MB 31.30 / 29.67 / 29.42 / 27.76  122 MB 40.08 / 43.74 / 38.43 / 37.87
+//        152 MB 49.39 / 54.94 / 47.79 / 48.41  190 MB 61.23 / 67.87 / 59.61 / 62.01
+//   FP16  38 MB 18.74 / 18.43 / 19.46 / 18.89   61 MB 30.96 / 28.17 / 29.88 / 28.89
+//         87 MB 42.75 / 41.05 / 42.20 / 40.99  122 MB 57.90 / 59.65 / 57.28 / 56.47
+//   D3Q27 FP32 76 MB 25.75 / 21.24 / 24.12 / 21.73   130 MB 42.55 / 46.82 / 40.72 / 40.76
+// Below 38 MB both buffers stay in L2 either way (equal within 0.5%).
+constexpr int64_t kStreamBytes = 138000000, kReverseBytes = 86000000;
+template <int Q, typename S, int MODE, int BT, int MB, int FB>
 cudaError_t launch_compact(const StepParams& p, cudaStream_t st) {
     if constexpr (Store<S>::offset && MODE == MODE_PHYSICS) {
         if (p.warp_block && p.seg_abs && !p.sp_q && (int64_t)Q * p.stride < ((int64_t)1 << 31)) {
             StepParams q = p;
+            const int64_t bytes = (int64_t)Q * p.stride * (int64_t)sizeof(S);
+            q.stream = bytes <= kStreamBytes ? 1 : 0;
+            q.reverse = bytes >= kReverseBytes ? p.odd : 0;
             q.fold_blocks = ceil_div(p.nnw, (int64_t)BT * kFoldNodes);
             const int64_t nb = ceil_div(p.nact, BT);
             if (nb <= 0) return cudaSuccess;
             return launch_dependent(step_compact_kernel<Q, S, BT, MB>, q.fold_blocks + nb, BT, MB, q, st);
         }
+        return launch_step_variant<Q, S, MODE, 0>(p, st);
     }
-    return launch_step_variant<Q, S, MODE, 0>(p, st);
+    return launch_step_variant<Q, S, MODE, FB>(p, st);
+}
+
+// The variant of a handle for which none was set (variant < 0), us a step on
+// tubes.  FP64: (64,8) (variant_shape).  Parity: the flat (128,12).  Physics in
+// the FP32-arithmetic formats, the compact kernel:
+//   up to 12k nodes a launch's latency counts, and blocks of 256 spread it over
+//   fewer: FP32 9k nodes (256,4) 3.21, (128,8) 3.55, (128,10) 3.90; 16k 3.66,
+//   3.56, 3.87;
+//   then registers before warps: 75k (128,8) 4.00, (128,10) 4.25, (128,12) 4.31;
+//   330k 7.59, 7.65, 8.31; D3Q27 at every size (550k 15.6, 17.3, 25.4);
+//   D3Q19 from 32 MB a buffer on: the populations come from memory, more
+//   loads in flight pay: FP32 550k (128,8) 11.71, (128,10) 11.56; 900k 19.31,
+//   18.74; 16-bit 1.6M (128,8) 29.23, (128,10) 28.28, (128,12) 28.17; 3.2M 62.5,
+//   57.9, 56.5.
+// The flat (128,12) that every such handle started on: 4.41 us at 20k nodes,
+// 8.29 at 250k (compact (128,8) 6.6), D3Q27 13.6 (8.3), FP32 1.4M 40.8 (35.5).
+constexpr int64_t kLatencyNodes = 12000, kMemoryBytes = 32000000;
+template <int Q, typename S, int MODE>
+int default_variant(const StepParams& p) {
+    if (!Store<S>::offset) return 4;
+    if (MODE != MODE_PHYSICS) return 0;
+    if (p.nact <= kLatencyNodes) return 3;
+    if (Q == 27 || (int64_t)Q * p.stride * (int64_t)sizeof(S) < kMemoryBytes) return 4;
+    return sizeof(S) == 4 ? 6 : 7;
 }
 
 template <int Q, typename S, int MODE>
 cudaError_t launch_family(int kind, int variant, const StepParams& p, cudaStream_t st) {
     if (kind == KIND_STEP) {
+        if (variant < 0) variant = default_variant<Q, S, MODE>(p);
         switch (variant) {
             case 1: return launch_step_variant<Q, S, MODE, 1>(p, st);
             case 2: return launch_step_variant<Q, S, MODE, 2>(p, st);
-            case 3: return launch_step_variant<Q, S, MODE, 3>(p, st);
-            case 4: return launch_step_variant<Q, S, MODE, 4>(p, st);
-            case 6: return launch_compact<Q, S, MODE, 128, 10>(p, st);
-            case 7: return launch_compact<Q, S, MODE, 128, 12>(p, st);
+            case 3: return launch_compact<Q, S, MODE, 256, 4, 3>(p, st);
+            case 4: return launch_compact<Q, S, MODE, 128, 8, 4>(p, st);
+            case 6: return launch_compact<Q, S, MODE, 128, 10, 0>(p, st);
+            case 7: return launch_compact<Q, S, MODE, 128, 12, 0>(p, st);
             case 5:
                 // the tiled kernel where a plan exists (physics, FP32-arithmetic
                 // formats, 32-bit offsets, half-way bounce-back); the default
