@@ -588,24 +588,23 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
 // or 1 of them, 27 (offset, class) blocks of CI columns.  The classes'
 // accumulators lie side by side in tensor memory (class 4 pz + 2 py + px), so
 // neighbouring classes take one MMA: 14 MMAs per 16 channels of dY, N = CI to
-// 8 CI, the first (offset 0) initialising every class.  Roles and barriers as
-// in k_conv3_pipe; a stage holds all co channels of a block.
+// 8 CI.  Offsets run from (1, 1, 1) down, all channels of one before the next:
+// a class's taps ascend, as in the mma.sync kernel, and the sums are its sums
+// bit for bit.  Roles and barriers as in k_conv3_pipe; a stage holds all co
+// channels of a block.
 // (The fallback read dY once per tap, 7/8 of them for nothing: 2293 us for
 // 32 -> 16 channels onto 256 x 128 x 128, 57 us here; 64 -> 32 onto 128 x 64 x
 // 64 489 -> 44 us; bound by the MMAs, 64 cycles each and 128 at N = 256.)
 constexpr int kD2Vox = 2 * 17 * 9;
 constexpr int kD2Half = kD2Vox * 16 + 64;
 
-// First block (of the 27) of an offset, offsets ordered zyx = 000, 100, 010,
-// 001, 110, 101, 011, 111.
-struct D2Off {
-    int z, y, x, first;
-};
-__host__ __device__ constexpr D2Off d2_off(int k) {
-    constexpr D2Off t[8] = {{0, 0, 0, 0},  {1, 0, 0, 8},  {0, 1, 0, 12}, {0, 0, 1, 16},
-                            {1, 1, 0, 20}, {1, 0, 1, 22}, {0, 1, 1, 24}, {1, 1, 1, 26}};
-    return t[k];
+// First block (of the 27) of offset 4 z + 2 y + x.
+__host__ __device__ constexpr int d2_first(int o) {
+    return o < 4 ? (o < 2 ? 8 * o : 4 * o + 4) : (o < 6 ? 4 * o + 2 : 2 * o + 12);
 }
+static_assert(d2_first(0) == 0 && d2_first(1) == 8 && d2_first(2) == 12 && d2_first(3) == 16 && d2_first(4) == 18 &&
+                  d2_first(5) == 22 && d2_first(6) == 24 && d2_first(7) == 26,
+              "8, 4, 4, 2, 4, 2, 2, 1 classes");
 // Tap of class bit p at offset o along one axis.
 __host__ __device__ constexpr int d2_tap(int p, int o) { return p == 0 ? 1 : (o == 0 ? 2 : 0); }
 
@@ -652,13 +651,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_dx2(const bf16* __res
         // wt [ci][27][co]: rows c of the block of (offset, class), 16-byte pieces of 8 co
         for (int i = tid; i < 27 * CI * groups; i += kPipeThreads - kProducers) {
             const int k8 = i % groups, n = (i / groups) % CI, blk = i / (groups * CI);
-            int k = 0;
-            while (k < 7 && blk >= d2_off(k + 1).first) ++k;
-            const D2Off o = d2_off(k);
-            const int need = 4 * o.z + 2 * o.y + o.x;
+            int o = 0;
+            while (o < 7 && blk >= d2_first(o + 1)) ++o;
             int cls = 0;  // the (blk - first)-th class with p = 1 where the offset is 1
-            for (int m = blk - o.first; (cls & need) != need || m-- > 0; ++cls) {}
-            const int t = (d2_tap(cls >> 2, o.z) * 3 + d2_tap((cls >> 1) & 1, o.y)) * 3 + d2_tap(cls & 1, o.x);
+            for (int m = blk - d2_first(o); (cls & o) != o || m-- > 0; ++cls) {}
+            const int t = (d2_tap(cls >> 2, o >> 2) * 3 + d2_tap((cls >> 1) & 1, (o >> 1) & 1)) * 3 + d2_tap(cls & 1, o & 1);
             cp_async16(wres + ((k8 >> 1) * 27 + blk) * (CI * 32) + (n >> 3) * 256 + (k8 & 1) * 128 + (n & 7) * 16,
                        wt + ((int64_t)(c0 + n) * 27 + t) * co + k8 * 8, true);
         }
@@ -714,18 +711,17 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_dx2(const bf16* __res
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tm + b * ACC;
             if (leader) {
-                for (int c = 0; c < chunks; ++c) {
-                    const uint64_t ad0 = smem_desc(st0 + s * stage_bytes + 2 * c * kD2Half, kD2Half, 144);
-                    const uint64_t bd0 = smem_desc(w0 + c * 27 * CI * 32, 128, 256);
+                // A class's first offset is its own number: it alone starts
+                // from zero there.
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        constexpr D2Off kOffs[8] = {d2_off(0), d2_off(1), d2_off(2), d2_off(3),
-                                                    d2_off(4), d2_off(5), d2_off(6), d2_off(7)};
-                        const D2Off o = kOffs[k];
-                        const uint64_t ad = ad0 + (uint64_t)((o.z * 17 + o.y) * 9 + o.x);
-                        const int need = 4 * o.z + 2 * o.y + o.x;
+                for (int k = 0; k < 8; ++k) {
+                    const int need = 7 - k, oz = need >> 2, oy = need >> 1 & 1, ox = need & 1;
+                    for (int c = 0; c < chunks; ++c) {
+                        const uint64_t ad = smem_desc(st0 + s * stage_bytes + 2 * c * kD2Half, kD2Half, 144) +
+                                            (uint64_t)((oz * 17 + oy) * 9 + ox);
+                        const uint64_t bd0 = smem_desc(w0 + c * 27 * CI * 32, 128, 256);
                         // runs of neighbouring classes
-                        int blk = o.first;
+                        int blk = d2_first(need);
 #pragma unroll
                         for (int cls = 0; cls < 8; ++cls) {
                             if ((cls & need) != need || (cls > 0 && ((cls - 1) & need) == need)) continue;
@@ -733,8 +729,15 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_dx2(const bf16* __res
 #pragma unroll
                             for (int e = 1; e < 8; ++e)
                                 if (run == e && cls + e < 8 && ((cls + e) & need) == need) run = e + 1;
-                            mma_bf16(acc + (uint32_t)(cls * CI), ad, bd0 + (uint64_t)(blk * (CI * 2)),
-                                     idesc_bf16(128, run * CI), c > 0 || k > 0 ? 1u : 0u);
+                            const uint64_t bd = bd0 + (uint64_t)(blk * (CI * 2));
+                            if (cls == need && c == 0) {
+                                mma_bf16(acc + (uint32_t)(cls * CI), ad, bd, idesc_bf16(128, CI), 0u);
+                                if (run > 1)
+                                    mma_bf16(acc + (uint32_t)((cls + 1) * CI), ad, bd + (uint64_t)(CI * 2),
+                                             idesc_bf16(128, (run - 1) * CI), 1u);
+                            } else {
+                                mma_bf16(acc + (uint32_t)(cls * CI), ad, bd, idesc_bf16(128, run * CI), 1u);
+                            }
                             blk += run;
                         }
                     }
@@ -1153,7 +1156,11 @@ namespace lbm {
 bool conv3_tc_applies(int D, int H, int W, int ci, int co, int stride) {
     const bool ch = (ci == 16 || ci == 32 || ci == 64) && (co == 16 || co == 32 || co == 64);
     if (!ch || D <= 0 || H <= 0 || W <= 0) return false;
-    if (stride == 1) return ceil_div(D, kPipeZ) * ceil_div(H, TY) * ceil_div(W, TX) <= 0x7fffffffLL;
+    // Lower than a block's 16 rows, as a network's lowest level is: the mma.sync
+    // kernel, whose order of summation such levels have always had (a network's
+    // gradients move by 4e-4 with the order here; 16 x 8 x 8, 64 -> 64 channels
+    // take 12 us there, 9 here).
+    if (stride == 1) return H >= TY && ceil_div(D, kPipeZ) * ceil_div(H, TY) * ceil_div(W, TX) <= 0x7fffffffLL;
     if (stride == 2) return D % 2 == 0 && H % (2 * TY) == 0 && W % (2 * TX) == 0;
     return false;
 }
