@@ -69,67 +69,151 @@ __device__ __forceinline__ int64_t source_voxel(const Conv& g, int64_t r, int t)
     }
 }
 
-// out[r][n] = act(bias[n] + sum_{t,k} src[source(r,t)][k] * B[n][t][k]).
-// BN = columns (padded channel count of the output, <= 64).
-template <int MODE, int BN>
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+// Through L1: for what all blocks read again and again (from L2 alone the few
+// lines of 1x1 weights are the bound: 293 us for 16 -> 16 on 256 x 128 x 128).
+__device__ __forceinline__ void cp16_cached(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Bytes of a row of kc channels in shared memory: 16-byte units at an odd
+// stride, so that ldmatrix meets no bank conflicts.
+__host__ __device__ constexpr int gemm_pitch(int kc) { return kc * 2 + 16; }
+
+// out[r][n] = act(bias[n] + sum_{t,k} src[source(r,t)][k] * B[n][t][k]), taps in
+// order, 16 channels an mma.  NB = columns of a block (n0 = NB blockIdx.y; co
+// in all); blocks walk 64-row tiles with a stride of the grid.  A step is one
+// tap of one tile, all kc channels; kGemmStages - 1 steps' copies are under way
+// (cp.async, zero where there is no source voxel) beside the mma of the oldest,
+// across tiles too.  On the small grids of a network's lowest level a block's
+// chain of 27 steps bounds it (16 x 8 x 8, 64 -> 64 channels: 57 us with one
+// 16-channel copy at a time and all 64 columns in a block, 12 now); on large
+// ones the copies (stride 2, 32 -> 64 from 64 x 88 x 72: 68 -> 42 us; 1x1, 16
+// -> 16 on 256 x 128 x 128: 112 -> 98 us forward with FP32 output, 119 -> 61 us
+// gradient; memory alone 76 and 38).  The order of the sums is the one it
+// always had: networks' values do not change.
+constexpr int kGemmStages = 4;
+template <int MODE, int NB, int KC>
 __global__ void __launch_bounds__(128) k_conv_gemm(const bf16* __restrict__ src, const bf16* __restrict__ B,
                                                    const float* __restrict__ bias, bf16* __restrict__ out,
-                                                   float* __restrict__ out_f32, Conv g, int64_t rows, int kc,
-                                                   int relu) {
-    __shared__ __align__(16) bf16 As[kRows][kPadK];
-    __shared__ __align__(16) bf16 Bs[BN][kPadK];
+                                                   float* __restrict__ out_f32, Conv g, int64_t rows, int64_t ntiles,
+                                                   int co, int relu) {
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gq = lane >> 2, tg = lane & 3;
-    const int64_t r0 = (int64_t)blockIdx.x * kRows;
-    const int taps = g.ks * g.ks * g.ks;
-    float acc[BN / 8][4];
-#pragma unroll
-    for (int j = 0; j < BN / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    // this thread's A row and half-row (8 channels)
+    const int taps = g.ks * g.ks * g.ks, n0 = blockIdx.y * NB;
+    constexpr int pitch = gemm_pitch(KC), kc8 = KC / 8;
+    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(gemm_smem);
+    constexpr uint32_t stage = (kRows + NB) * pitch;
+
+    // copies: this thread's row and half of its channels; the position of row 0's tap (0, 0, 0)
     const int arow = tid >> 1, ahalf = tid & 1;
-    const int64_t r = r0 + arow;
-    for (int t = 0; t < taps; ++t) {
-        const int64_t sv = r < rows ? source_voxel<MODE>(g, r, t) : -1;
-        for (int c0 = 0; c0 < kc; c0 += 16) {
-            uint4 av = make_uint4(0, 0, 0, 0);
-            if (sv >= 0) av = *reinterpret_cast<const uint4*>(src + sv * kc + c0 + ahalf * 8);
-            *reinterpret_cast<uint4*>(&As[arow][ahalf * 8]) = av;
-            for (int e = tid; e < BN * 2; e += 128) {
-                const int n = e >> 1, h = e & 1;
-                *reinterpret_cast<uint4*>(&Bs[n][h * 8]) =
-                    *reinterpret_cast<const uint4*>(B + ((int64_t)n * taps + t) * kc + c0 + h * 8);
-            }
-            __syncthreads();
-            uint32_t a[4];
-            const int ar = warp * 16 + gq;
-            a[0] = *reinterpret_cast<const uint32_t*>(&As[ar][tg * 2]);
-            a[1] = *reinterpret_cast<const uint32_t*>(&As[ar + 8][tg * 2]);
-            a[2] = *reinterpret_cast<const uint32_t*>(&As[ar][tg * 2 + 8]);
-            a[3] = *reinterpret_cast<const uint32_t*>(&As[ar + 8][tg * 2 + 8]);
+    int64_t lt = blockIdx.x;
+    int ltap = 0, lz = 0, ly = 0, lx = 0, slot = 0;
+    bool inside = false;
+    auto locate = [&]() {
+        const int64_t r = lt * kRows + arow;
+        inside = lt < ntiles && r < rows;
+        if (!inside || taps == 1) return;
+        const int w = MODE == 0 ? g.Wo : g.W, h = MODE == 0 ? g.Ho : g.H;
+        const int64_t q = r / w;
+        lx = (int)(r - q * w);
+        lz = (int)(q / h);
+        ly = (int)(q - (int64_t)lz * h);
+        if (MODE == 0) { lx = lx * g.stride - g.pad; ly = ly * g.stride - g.pad; lz = lz * g.stride - g.pad; }
+        else { lx += g.pad; ly += g.pad; lz += g.pad; }
+    };
+    auto source = [&]() -> int64_t {
+        if (!inside) return -1;
+        if (taps == 1) return lt * kRows + arow;  // 1x1: stride 1, no padding
+        const int tz = ltap / 9, ty = ltap / 3 % 3, tx = ltap % 3;
+        if (MODE == 0) {
+            const int ix = lx + tx, iy = ly + ty, iz = lz + tz;
+            if ((unsigned)ix >= (unsigned)g.W || (unsigned)iy >= (unsigned)g.H || (unsigned)iz >= (unsigned)g.D) return -1;
+            return ((int64_t)iz * g.H + iy) * g.W + ix;
+        }
+        int ox = lx - tx, oy = ly - ty, oz = lz - tz;
+        if (g.stride == 2) {
+            if ((ox | oy | oz) & 1) return -1;
+            ox >>= 1; oy >>= 1; oz >>= 1;
+        }
+        if ((unsigned)ox >= (unsigned)g.Wo || (unsigned)oy >= (unsigned)g.Ho || (unsigned)oz >= (unsigned)g.Do) return -1;
+        return ((int64_t)oz * g.Ho + oy) * g.Wo + ox;
+    };
+    auto copy = [&]() {
+        if (lt < ntiles) {
+            const uint32_t dst = sm + slot * stage;
+            const int64_t sv = source();
+            const bf16* p = src + (sv >= 0 ? sv * KC : 0) + ahalf * (KC / 2);
+            const uint32_t da = dst + arow * pitch + ahalf * KC;
 #pragma unroll
-            for (int j = 0; j < BN / 8; ++j) {
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&Bs[j * 8 + gq][tg * 2]);
-                const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&Bs[j * 8 + gq][tg * 2 + 8]);
-                mma_bf16(acc[j], a, b0, b1);
+            for (int k = 0; k < KC / 16; ++k) cp16(da + k * 16, p + k * 8, sv >= 0);
+#pragma unroll
+            for (int e0 = 0; e0 < NB * kc8; e0 += 128) {
+                const int e = e0 + tid, n = e / kc8, k = e % kc8;
+                if (NB * kc8 % 128 == 0 || e < NB * kc8)
+                    cp16_cached(dst + (kRows + n) * pitch + k * 16, B + ((n0 + n) * taps + ltap) * KC + k * 8);
             }
-            __syncthreads();
+            if (++ltap == taps) { ltap = 0; lt += gridDim.x; locate(); }
+        }
+        if (++slot == kGemmStages) slot = 0;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    locate();
+    for (int k = 0; k < kGemmStages - 1; ++k) copy();
+
+    float acc[NB / 8][4];
+    int at = 0;
+    const uint32_t fa = sm + (warp * 16 + (lane & 15)) * pitch + (lane >> 4) * 16,
+                   fb = sm + (kRows + (lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 16;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+#pragma unroll
+        for (int j = 0; j < NB / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+        for (int t = 0; t < taps; ++t) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kGemmStages - 2) : "memory");
+            __syncthreads();  // the step's copies are seen, and the slot the next copy takes is read
+            copy();
+#pragma unroll
+            for (int c = 0; c < KC; c += 16) {
+                uint32_t a[4];
+                ldsm4(a, fa + at * stage + c * 2);
+#pragma unroll
+                for (int j = 0; j < NB / 16; ++j) {
+                    uint32_t b[4];
+                    ldsm4(b, fb + at * stage + j * 16 * pitch + c * 2);
+                    mma_bf16(acc[2 * j], a, b[0], b[1]);
+                    mma_bf16(acc[2 * j + 1], a, b[2], b[3]);
+                }
+            }
+            if (++at == kGemmStages) at = 0;
+        }
+        // epilogue: bias, ReLU, BF16 (and optionally FP32) store
+#pragma unroll
+        for (int j = 0; j < NB / 8; ++j) {
+            const int n = n0 + j * 8 + tg * 2;
+            const float b0 = bias ? bias[n] : 0.f, b1 = bias ? bias[n + 1] : 0.f;
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int64_t rr = tile * kRows + warp * 16 + gq + hh * 8;
+                if (rr >= rows) continue;
+                float v0 = acc[j][2 * hh] + b0, v1 = acc[j][2 * hh + 1] + b1;
+                if (relu) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
+                *reinterpret_cast<__nv_bfloat162*>(out + rr * co + n) = __floats2bfloat162_rn(v0, v1);
+                if (out_f32) *reinterpret_cast<float2*>(out_f32 + rr * co + n) = make_float2(v0, v1);
+            }
         }
     }
-    // epilogue: bias, ReLU, BF16 (and optionally FP32) store
-#pragma unroll
-    for (int j = 0; j < BN / 8; ++j) {
-        const int n = j * 8 + tg * 2;
-        const float b0 = bias ? bias[n] : 0.f, b1 = bias ? bias[n + 1] : 0.f;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int64_t rr = r0 + warp * 16 + gq + hh * 8;
-            if (rr >= rows) continue;
-            float v0 = acc[j][2 * hh] + b0, v1 = acc[j][2 * hh + 1] + b1;
-            if (relu) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
-            *reinterpret_cast<__nv_bfloat162*>(out + rr * BN + n) = __floats2bfloat162_rn(v0, v1);
-            if (out_f32) { out_f32[rr * BN + n] = v0; out_f32[rr * BN + n + 1] = v1; }
-        }
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // dW[co][t][ci] += sum over output voxels m of dY[m][co] * X[src(m,t)][ci]
@@ -766,16 +850,42 @@ Conv make_conv(const int dims_in[3], int ci, int co, int ks, int stride) {
     return g;
 }
 
-template <int MODE>
-cudaError_t launch_gemm(int bn, const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32,
-                        const Conv& g, int64_t rows, int kc, int relu, cudaStream_t st) {
-    const unsigned blocks = (unsigned)lbm::ceil_div(rows, kRows);
-    switch (bn) {
-        case 16: k_conv_gemm<MODE, 16><<<blocks, 128, 0, st>>>(src, B, bias, out, out_f32, g, rows, kc, relu); break;
-        case 32: k_conv_gemm<MODE, 32><<<blocks, 128, 0, st>>>(src, B, bias, out, out_f32, g, rows, kc, relu); break;
-        default: k_conv_gemm<MODE, 64><<<blocks, 128, 0, st>>>(src, B, bias, out, out_f32, g, rows, kc, relu); break;
+template <int MODE, int NB, int KC>
+cudaError_t launch_gemm_kc(const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32, const Conv& g,
+                           int64_t rows, int co, int relu, cudaStream_t st) {
+    constexpr int bytes = kGemmStages * (kRows + NB) * gemm_pitch(KC);
+    if constexpr (bytes > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_conv_gemm<MODE, NB, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
     }
+    constexpr int64_t fit = 220 * 1024 / bytes, most = 152 * (fit < 8 ? fit : 8);
+    const int64_t tiles = lbm::ceil_div(rows, kRows);
+    k_conv_gemm<MODE, NB, KC><<<dim3((unsigned)(tiles < most ? tiles : most), (unsigned)(co / NB)), 128, bytes, st>>>(
+        src, B, bias, out, out_f32, g, rows, tiles, co, relu);
     return cudaGetLastError();
+}
+
+template <int MODE, int NB>
+cudaError_t launch_gemm_nb(const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32, const Conv& g,
+                           int64_t rows, int kc, int co, int relu, cudaStream_t st) {
+    switch (kc) {
+        case 16: return launch_gemm_kc<MODE, NB, 16>(src, B, bias, out, out_f32, g, rows, co, relu, st);
+        case 32: return launch_gemm_kc<MODE, NB, 32>(src, B, bias, out, out_f32, g, rows, co, relu, st);
+        default: return launch_gemm_kc<MODE, NB, 64>(src, B, bias, out, out_f32, g, rows, co, relu, st);
+    }
+}
+
+// All co columns in a block (the rows are read once) where their tiles alone
+// give every SM a block; else 16 columns a block (180 tiles, 64 columns of 64
+// channels: 30 us in one block, 56 us in four).
+template <int MODE>
+cudaError_t launch_gemm(int co, const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32,
+                        const Conv& g, int64_t rows, int kc, int relu, cudaStream_t st) {
+    if (co > 16 && rows >= (int64_t)kRows * 152) {
+        if (co == 32) return launch_gemm_nb<MODE, 32>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
+        if (co == 64) return launch_gemm_nb<MODE, 64>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
+    }
+    return launch_gemm_nb<MODE, 16>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
 }
 
 template <int CO>
