@@ -201,7 +201,9 @@ def voxelize(tri12, spacing, bbox=None, origin=None, dims=None):
     _check(L.lbm_voxelize(_ptr(tri), len(tri), C.byref(d), None))
     nx, ny, nz = d.dims
     mask = np.zeros(nx * ny * nz, np.uint8)
+    rule, d.reference_bbox = d.reference_bbox, 0  # the box is in d now: not from the triangles again
     _check(L.lbm_voxelize(_ptr(tri), len(tri), C.byref(d), _ptr(mask)))
+    d.reference_bbox = rule
     return mask.reshape(nz, ny, nx), d
 
 
