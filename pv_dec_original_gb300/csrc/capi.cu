@@ -1223,8 +1223,7 @@ int macro_to_staging(lbm_handle* h) {
     StepParams p = make_params(h, 2);
     p.out_rho = h->macro;
     p.out_u = h->macro + (na + 1);
-    CK(h, launch(h, 2, p));
-    CK(h, reduce_partials(h->partials, h->nblocks, h->sums, h->st));
+    CK(h, launch(h, 3, p));
     return LBM_OK;
 }
 

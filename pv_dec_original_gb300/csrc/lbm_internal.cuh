@@ -162,7 +162,7 @@ constexpr int kPartialStride = 4;
 constexpr int kStepThreads = 256;
 
 // Launchers (one per translation unit family).  kind: 0 step, 1 prologue
-// (collide the initial state), 2 materialize (post-boundary f + sums).
+// (collide the initial state), 2 materialize (post-boundary f + sums), 3 rho and u.
 constexpr int kRingSlots = 32;  // FP32 stress ring: two halves of kFoldEvery steps
 constexpr int kFoldEvery = 16;  // steps between folds of the FP32 stress ring
 constexpr int kNumVariants = LBM_NUM_VARIANTS;  // launch-shape variants of the step kernel (step_kernels.cuh)

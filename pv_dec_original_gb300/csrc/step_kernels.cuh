@@ -44,7 +44,9 @@ namespace lbm {
 
 constexpr int MODE_PARITY = LBM_PARITY;
 constexpr int MODE_PHYSICS = LBM_PHYSICS;
-constexpr int KIND_STEP = 0, KIND_PROLOGUE = 1, KIND_READOUT = 2;
+constexpr int KIND_STEP = 0, KIND_PROLOGUE = 1, KIND_READOUT = 2, KIND_MACRO = 3;
+// KIND_READOUT: FP64 distributions, sums and fluxes; KIND_MACRO: rho and u of every node.
+__host__ __device__ constexpr bool reads_out(int kind) { return kind == KIND_READOUT || kind == KIND_MACRO; }
 
 // Momentum sums with the reference's explicit index lists (Simulation.cpp:66-175);
 // the same lists apply to offsets because sum_q w_q c_q = 0.
@@ -749,9 +751,80 @@ __device__ __forceinline__ void block_partials(double (&v)[kPartialStride], doub
     }
 }
 
-template <int Q, typename R, bool OFF>
-__device__ __forceinline__ double full_value(R v, int q) {
-    return OFF ? Lat<Q>::w(q) + (double)v : (double)v;
+// The full f in FP64 of the value g that the arithmetic holds.
+template <int Q, typename S>
+__device__ __forceinline__ double full_population(typename Store<S>::real v, int q) {
+    if constexpr (Store<S>::scaled) return Lat<Q>::w(q) + (double)Store<S>::template unit<Q>(q) * (double)v;
+    else return Store<S>::offset ? Lat<Q>::w(q) + (double)v : (double)v;
+}
+
+// A sum of FP32 values with the rounding errors of its additions kept
+// (two-sum, Knuth, The Art of Computer Programming 2, 4.2.2): s + c is the sum
+// to about 2^-48 of the largest partial sum.
+struct ErrorFreeSum {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = s + x, b = t - s;
+        c += (s - (t - b)) + (x - b);
+        s = t;
+    }
+    __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+};
+
+// rho and u (FP64) of an FP32-arithmetic node: rho = 1 + sum g, u = sum c g /
+// rho.  An SM does two FP64 operations a cycle, and the full f in FP64 and its
+// moments were 130 of them a node.  The offsets are added in FP32 with their
+// rounding errors kept (some 300 operations of the full FP32 rate); only the
+// four sums, their scaling and the divisions are in FP64.  D3Q19: 2.8M nodes in
+// FP16 665 -> 176 us, 0.9M in FP32 218 -> 50 us; D3Q27, 0.25M 93 -> 24 us.  Against the exact sums
+// (D3Q19, |u| about 0.3): rho's error 1.9e-16 before (the weights' sum is not
+// exactly 1), none beyond its own rounding now; u's 6.1e-17 before, 1.3e-17 now.
+// In the scaled formats the terms are brought to the smallest weight's unit by
+// exact powers of two, but for D3Q19's rest population, whose unit is no such
+// multiple.  Sums near the end of FP32's range take the full f.
+template <int Q, typename S>
+__device__ __forceinline__ void macro_of_offsets(const float (&g)[Q], double& rho, double& ux, double& uy, double& uz) {
+    constexpr bool SC = Store<S>::scaled;
+    constexpr int small = Q == 19 ? 6 : 19;  // a direction of the smallest weight
+    constexpr bool rest_apart = SC && Q == 19;
+    auto term = [&](int q) -> float {
+        if constexpr (SC) return g[q] * (Store<S>::template unit<Q>(q) / Store<S>::template unit<Q>(small));
+        else return g[q];
+    };
+    ErrorFreeSum r, p[3];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+        if (!(rest_apart && q == Lat<Q>::REST)) r.add(term(q));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int o = Lat<Q>::opp(q);
+        if (q >= o) continue;
+        const float v = term(q), w = term(o), d = v - w, b = v - d, e = (v - (d + b)) + (b - w);
+        const int c[3] = {Lat<Q>::cx(q), Lat<Q>::cy(q), Lat<Q>::cz(q)};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (c[k] == 0) continue;
+            p[k].add(c[k] > 0 ? d : -d);
+            p[k].c += c[k] > 0 ? e : -e;
+        }
+    }
+    if (fmaxf(fmaxf(fabsf(r.s), fabsf(p[0].s)), fmaxf(fabsf(p[1].s), fabsf(p[2].s))) < 1e30f && r.s == r.s &&
+        p[0].s == p[0].s && p[1].s == p[1].s && p[2].s == p[2].s) {
+        double n = r.value(), jx = p[0].value(), jy = p[1].value(), jz = p[2].value();
+        if constexpr (SC) {
+            constexpr double unit = (double)Store<S>::template unit<Q>(small);
+            n *= unit; jx *= unit; jy *= unit; jz *= unit;
+            if constexpr (rest_apart)
+                n = __fma_rn((double)Store<S>::template unit<Q>(Lat<Q>::REST), (double)g[Lat<Q>::REST], n);
+        }
+        rho = 1.0 + n;
+        divide3(jx, jy, jz, rho, ux, uy, uz);
+        return;
+    }
+    double f[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) f[q] = full_population<Q, S>(g[q], q);
+    moments<Q, double, false>(f, rho, ux, uy, uz);
 }
 
 // f* == 0.0 in the arithmetic's own representation.
@@ -793,8 +866,8 @@ __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a
     constexpr bool OFF = Store<S>::offset;
     constexpr bool SC = Store<S>::scaled;  // g in storage units (FP16, BF16)
     S* __restrict__ fout = static_cast<S*>(P.fout);
-    const bool direct = (KIND == KIND_PROLOGUE) || (KIND == KIND_READOUT && P.direct);
-    constexpr bool parity_readout = (KIND == KIND_READOUT && MODE == MODE_PARITY);
+    const bool direct = (KIND == KIND_PROLOGUE) || (reads_out(KIND) && P.direct);
+    constexpr bool parity_readout = (reads_out(KIND) && MODE == MODE_PARITY);
     const I ai = (I)a, st = (I)P.stride;
     // f == 0 in the values g holds
     auto exact_zero = [](R v, int q) {
@@ -861,33 +934,21 @@ __device__ __forceinline__ void node_finish(const StepParams& P, const int64_t a
         if (zero) atomicOr(P.flags, FLAG_EXACT_ZERO);
     }
 
-    if constexpr (KIND == KIND_READOUT) {
+    if constexpr (KIND == KIND_MACRO) {
+        double rr, vx, vy, vz;
+        if constexpr (OFF) macro_of_offsets<Q, S>(g, rr, vx, vy, vz);
+        else moments<Q, double, false>(g, rr, vx, vy, vz);
+        P.out_rho[a] = rr;
+        P.out_u[3 * a] = vx; P.out_u[3 * a + 1] = vy; P.out_u[3 * a + 2] = vz;
+    } else if constexpr (KIND == KIND_READOUT) {
         R r, ux, uy, uz;
         mom(g, r, ux, uy, uz);
         const double rho = OFF ? 1.0 + (double)r : (double)r;
         part[0] = OFF ? (double)r : rho - 1.0;
         part[1] = rho * ux; part[2] = rho * uy; part[3] = rho * uz;
-        if (P.out_f || P.out_rho) {
-            double fd[Q];  // the full f in FP64
+        if (P.out_f) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                if constexpr (SC)
-                    fd[q] = Lat<Q>::w(q) + (double)Store<S>::template unit<Q>(q) * (double)g[q];
-                else
-                    fd[q] = full_value<Q, R, OFF>(g[q], q);
-            }
-            if (P.out_f) {
-#pragma unroll
-                for (int q = 0; q < Q; ++q) P.out_f[a * Q + q] = fd[q];
-            }
-            if (P.out_rho) {
-                // the FP64 moments of the full f (Collision's formulas), as
-                // the FP64 distributions of lbm_get_distributions would give them
-                double rr, vx, vy, vz;
-                moments<Q, double, false>(fd, rr, vx, vy, vz);
-                P.out_rho[a] = rr;
-                P.out_u[3 * a] = vx; P.out_u[3 * a + 1] = vy; P.out_u[3 * a + 2] = vz;
-            }
+            for (int q = 0; q < Q; ++q) P.out_f[a * Q + q] = full_population<Q, S>(g[q], q);
         }
     } else {
         // ---- moments of the post-boundary populations: they serve the
@@ -1032,7 +1093,7 @@ __device__ __forceinline__ void pull_node(const StepParams& P, const int64_t a, 
     constexpr bool OFF = Store<S>::offset;
     constexpr int DR = kDeltaRow<Q>;
     const S* __restrict__ fin = static_cast<const S*>(P.fin);
-    const bool direct = (KIND == KIND_PROLOGUE) || (KIND == KIND_READOUT && P.direct);
+    const bool direct = (KIND == KIND_PROLOGUE) || (reads_out(KIND) && P.direct);
     const uint32_t miss = word_miss(word);  // zero on interior nodes
     const int c = word_class(word);
     // Boundary-list work: in parity mode every boundary-list node (history
@@ -1907,6 +1968,18 @@ int default_variant(const StepParams& p) {
     return sizeof(S) == 4 ? 6 : 7;
 }
 
+template <int Q, typename S, int MODE, int KIND>
+void launch_readout(const StepParams& p, int64_t nblocks, cudaStream_t st) {
+    if constexpr (MODE == MODE_PHYSICS) {
+        if (p.sp_q != nullptr) {
+            // the read-out's pull applies the same interpolated bounce-back
+            step_kernel<Q, S, MODE, KIND, kStepThreads, 1, true, true><<<(unsigned)nblocks, kStepThreads, 0, st>>>(p);
+            return;
+        }
+    }
+    step_kernel<Q, S, MODE, KIND><<<(unsigned)nblocks, kStepThreads, 0, st>>>(p);
+}
+
 template <int Q, typename S, int MODE>
 cudaError_t launch_family(int kind, int variant, const StepParams& p, cudaStream_t st) {
     if (kind == KIND_STEP) {
@@ -1930,20 +2003,16 @@ cudaError_t launch_family(int kind, int variant, const StepParams& p, cudaStream
             default: return launch_step_variant<Q, S, MODE, 0>(p, st);
         }
     }
-    // prologue and read-out: default shape (the read-out's partial sums are per 256-thread block)
+    // prologue and read-outs: default shape (the read-out's partial sums are per 256-thread block)
     const int64_t nblocks = ceil_div(p.nact, kStepThreads);
     if (nblocks <= 0) return cudaSuccess;
     if (nblocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if (kind == KIND_PROLOGUE) {
+    if (kind == KIND_PROLOGUE)
         step_kernel<Q, S, MODE, KIND_PROLOGUE><<<(unsigned)nblocks, kStepThreads, 0, st>>>(p);
-    } else if (MODE == MODE_PHYSICS && p.sp_q != nullptr) {
-        // the read-out's pull applies the same interpolated bounce-back
-        if constexpr (MODE == MODE_PHYSICS)
-            step_kernel<Q, S, MODE, KIND_READOUT, kStepThreads, 1, true, true>
-                <<<(unsigned)nblocks, kStepThreads, 0, st>>>(p);
-    } else {
-        step_kernel<Q, S, MODE, KIND_READOUT><<<(unsigned)nblocks, kStepThreads, 0, st>>>(p);
-    }
+    else if (kind == KIND_MACRO)
+        launch_readout<Q, S, MODE, KIND_MACRO>(p, nblocks, st);
+    else
+        launch_readout<Q, S, MODE, KIND_READOUT>(p, nblocks, st);
     return cudaGetLastError();
 }
 
