@@ -48,6 +48,12 @@ lbm_status lbm_nn_conv_status(void);
 lbm_status lbm_nn_conv3d_bwd(const void* x, const int dims_in[3], int ci, const void* w, void* w_t, int co,
                              int ksize, int stride, const void* dy, void* dx, float* dw, float* db, void* stream);
 
+/* The gradient at a ReLU layer's output, [rows][c] BF16 (c 16, 32 or 64; 16-byte
+ * aligned), in one pass: dy += add (if not NULL; rounded as lbm_nn_add does),
+ * copy = dy (if not NULL), dy *= (y > 0), db[c] += sum over the rows of dy. */
+lbm_status lbm_nn_layer_grad(const void* y, const void* add, void* dy, void* copy, float* db, int64_t rows, int c,
+                             void* stream);
+
 /* dy *= (y > 0) over n elements (ReLU backward from the stored output). */
 lbm_status lbm_nn_relu_bwd(const void* y, void* dy, int64_t n, void* stream);
 

@@ -71,7 +71,7 @@ EXPORTS = [
     "lbm_preset_flags", "lbm_autotune", "lbm_set_variant",
     "lbm_moment_sums_noalloc",
     "lbm_nn_conv3d_fwd", "lbm_nn_conv3d_bwd", "lbm_nn_set_conv_engine", "lbm_nn_conv_status",
-    "lbm_nn_relu_bwd", "lbm_nn_upsample2", "lbm_nn_add", "lbm_nn_mse",
+    "lbm_nn_layer_grad", "lbm_nn_relu_bwd", "lbm_nn_upsample2", "lbm_nn_add", "lbm_nn_mse",
     "lbm_nn_adam", "lbm_sdf_from_mask", "lbm_ws_prior", "lbm_ws_smooth", "lbm_ws_features", "lbm_ws_output", "lbm_ws_gather",
     "lbm_init_from_macro_device", "lbm_nearest_next_to_wall", "lbm_set_wall_distances", "lbm_get_wall_distances",
     "lbm_get_macro_async", "lbm_get_wss_async", "lbm_wait_outputs",
@@ -145,6 +145,7 @@ def load(build_if_missing: bool = True):
     L.lbm_nn_conv3d_bwd.argtypes = [P, I3, C.c_int, P, P, C.c_int, C.c_int, C.c_int, P, P, P, P, P]
     L.lbm_nn_set_conv_engine.argtypes = [C.c_int]
     L.lbm_nn_conv_status.argtypes = []
+    L.lbm_nn_layer_grad.argtypes = [P, P, P, P, P, C.c_int64, C.c_int, P]
     L.lbm_nn_relu_bwd.argtypes = [P, P, C.c_int64, P]
     L.lbm_nn_upsample2.argtypes = [P, I3, C.c_int, P, C.c_int, P]
     L.lbm_nn_add.argtypes = [P, P, P, C.c_int64, P]

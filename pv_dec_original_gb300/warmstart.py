@@ -210,15 +210,24 @@ class WarmStartNet:
         the parameter gradients into gw / gb."""
         L = self.L
         self.grad["out"].copy_(dy_out)
+        pending = set()  # layers whose gradient still lacks their skip's
         for name in reversed(list(self.meta.keys())):
             m = self.meta[name]
             g = self.grad[name]
-            if m["skip"]:
-                # the sum's gradient also reaches the skip source
-                self.skip_grad[m["skip"]].copy_(g)
+            add = self.skip_grad[name] if name in pending else None
+            # the sum's gradient also reaches the skip source
+            copy = self.skip_grad[m["skip"]] if m["skip"] else None
+            gb = self.gb[m["b_off"]:m["b_off"] + m["co"]]
             if m["relu"]:
                 y = self.pre[name] if m["skip"] else self.act[name]
-                self._check(L.lbm_nn_relu_bwd(_ptr(y), _ptr(g), g.numel(), self.st))
+                self._check(L.lbm_nn_layer_grad(_ptr(y), _ptr(add), _ptr(g), _ptr(copy), _ptr(gb),
+                                                self.nvox(m["lvl_out"]), m["co"], self.st))
+                gb = None
+            else:
+                if add is not None:
+                    self._check(L.lbm_nn_add(_ptr(g), _ptr(add), _ptr(g), g.numel(), self.st))
+                if copy is not None:
+                    copy.copy_(g)
             src = m["src"]
             if src.startswith("up:"):
                 xin, dx = self.up[name], self.grad_up[name]
@@ -229,14 +238,13 @@ class WarmStartNet:
             w = self.wb[m["w_off"]:m["w_off"] + m["w_n"]]
             self._check(L.lbm_nn_conv3d_bwd(_ptr(xin), _dims(self.grid(m["lvl_in"])), m["ci"], _ptr(w),
                                             _ptr(self.wt), m["co"], m["ks"], m["stride"], _ptr(g), _ptr(dx),
-                                            _ptr(self.gw[m["w_off"]:m["w_off"] + m["w_n"]]),
-                                            _ptr(self.gb[m["b_off"]:m["b_off"] + m["co"]]), self.st))
+                                            _ptr(self.gw[m["w_off"]:m["w_off"] + m["w_n"]]), _ptr(gb), self.st))
             if src.startswith("up:"):
                 s = src[3:]
                 self._check(L.lbm_nn_upsample2(_ptr(dx), _dims(self.grid(self.level[s])), m["ci"],
                                                _ptr(self.grad[s]), 1, self.st))
             elif src in self.skip_grad:
-                self._check(L.lbm_nn_add(_ptr(dx), _ptr(self.skip_grad[src]), _ptr(dx), dx.numel(), self.st))
+                pending.add(src)
 
     def zero_grad(self):
         self.gw.zero_()
