@@ -343,9 +343,11 @@ __global__ void __launch_bounds__(kThreads) k_conv3_s2_tc(const __grid_constant_
 // (tfull / tempty); every wait is bounded, and a role that gives up raises
 // the flag and leaves, whereupon the others' waits run out.
 //
-// What bounds it: an M = 128, K = 16 MMA holds the tensor pipe for 64 cycles
-// up to N = 64 (ncu: 69.8k pipe cycles for 1091 MMAs a SM), 54 a chunk; at
-// 16 -> 16 channels (N = 16 to 48) that is 95 of 120 us.  The kernel before
+// What bounds it: the MMAs, at 77 to 83 SM cycles each whatever their N up to
+// 192 (ncu: 4364 a SM in 335k cycles at N = 64 to 192, 1091 in 90k at N = 16 to
+// 48; each reads a 4 KB A operand from shared memory), 54 a chunk.  Neighbours
+// that add to the same accumulators are not the reason: two blocks' MMAs
+// issued in turn ran the same 117 us at 16 -> 16 channels.  The kernel before
 // staged with tensor copies, whose 8-channel layout is boxes of 16-byte
 // rows: 2160 a chunk at about 3 cycles each, 7.2k cycles a chunk whatever
 // its MMAs.  The same bytes by cp.async are 68 warp instructions.  256 x 128
@@ -594,7 +596,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
 // channels of a block.
 // (The fallback read dY once per tap, 7/8 of them for nothing: 2293 us for
 // 32 -> 16 channels onto 256 x 128 x 128, 57 us here; 64 -> 32 onto 128 x 64 x
-// 64 489 -> 44 us; bound by the MMAs, 64 cycles each and 128 at N = 256.)
+// 64 489 -> 38 us; bound by the MMAs, as k_conv3_pipe.)
 constexpr int kD2Vox = 2 * 17 * 9;
 constexpr int kD2Half = kD2Vox * 16 + 64;
 
