@@ -818,10 +818,14 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_dx2(const bf16* __res
 // phase lie in different banks at stride 1 for any tap.  Warps are NG tap
 // groups (TPW taps each) x KG groups of voxel rows; D = dY^T X with
 // m16n8k16 (M = 16 output channels, N = 8 input channels, K = 16 voxels of
-// an x-run).  Bound by shared memory: an ldmatrix.x4 (4 cycles) per two MMAs
-// of 2 cycles at 16 channels, per four at 32.  256 x 128 x 128: 16 -> 16
-// 162 us (1122 before), 32 -> 16 316 us (2493), stride-2 16 -> 32 63 us
-// (153), 1x1x1 61 us (411); 128 x 64 x 64, 32 -> 32: 92 us (327).
+// an x-run).  Bound by the MMAs and shared memory together: an ldmatrix.x4
+// (4 cycles) per four MMAs of 2 cycles at 32 channels.  At 16, a view of an
+// input row serves one output row's MMAs per tap, two per ldmatrix.x4; so a warp
+// with all 9 taps of a tz goes down the rows and uses a view for the three output
+// rows that it meets (ROLL): 4 ldmatrix.x4 for 18 MMAs, 16 -> 16 channels 162 ->
+// 142 us.  256 x 128 x 128: 16 -> 16 142 us (1122 with the tcgen05 im2col), 32 ->
+// 16 275 us (2493), stride-2 16 -> 32 63 us (153), 1x1x1 61 us (411); 128 x 64 x
+// 64, 32 -> 32: 92 us (327).
 // grid.y walks the (co / COB) x (ci / 16) channel blocks.  Every
 // FLUSH tiles the KG groups add their sums in turn to the CTA's in shared
 // memory: an MMA drops bits of its accumulator, so that chains of 216 MMAs
@@ -838,6 +842,7 @@ struct WGeo {
     static constexpr int XD = S * (TZ - 1) + KS, XH = S * (TY - 1) + KS, XW = S * (TX - 1) + KS;
     static constexpr int TPW = KS == 1 ? 1 : (COB == 16 ? 9 : 3);
     static constexpr int NG = TAPS / TPW;
+    static constexpr bool ROLL = KS == 3 && S == 1 && TPW == 9;  // rows in turn, views kept for three ty
     static constexpr int KG = KS == 1 ? 12 : (COB == 16 ? 4 : 2);
     static constexpr int THREADS = 32 * NG * KG;
     static constexpr int KSTEPS = TZ * TY * TX / 16;
@@ -962,6 +967,32 @@ __global__ void __launch_bounds__(G::THREADS, 1) k_conv_wgrad_tiles(const __grid
         ok = __syncthreads_and(ok);
         if (!ok) break;
         const uint32_t xs = base + s * G::STAGE, ys = xs + G::XPAD;
+        if constexpr (G::ROLL) {
+            // x-runs of 16 voxels down the rows: an input row's three views
+            // (tx) meet the output rows of all three ty while they are at hand
+            constexpr int RUNS = G::TX / 16;
+            for (int run = kg; run < G::TZ * RUNS; run += G::KG) {
+                const int z = run / RUNS, x = run % RUNS * 16;
+                const uint32_t dv = (uint32_t)(z * G::TY * G::TX + x) + lv, xv = (uint32_t)(z * G::XH * G::XW + x) + lv + tapv;
+                uint32_t a[3][4];
+#pragma unroll
+                for (int r = 0; r < G::XH; ++r) {
+                    if (r < G::TY) ldmatrix4_trans(a[r % 3], ys + chunk16(dv + (uint32_t)(r * G::TX), lc));
+#pragma unroll
+                    for (int tx = 0; tx < 3; ++tx) {
+                        uint32_t b[4];
+                        ldmatrix4_trans(b, xs + chunk16(xv + (uint32_t)(r * G::XW + tx), lc));
+#pragma unroll
+                        for (int ty = 0; ty < 3; ++ty) {
+                            const int y = r - ty;
+                            if (y < 0 || y >= G::TY) continue;
+                            mma_m16n8k16(acc[ty * 3 + tx][0][0], a[y % 3], b[0], b[2]);
+                            mma_m16n8k16(acc[ty * 3 + tx][0][1], a[y % 3], b[1], b[3]);
+                        }
+                    }
+                }
+            }
+        } else
         for (int ks = kg; ks < G::KSTEPS; ks += G::KG) {
             constexpr int RUNS = G::TX / 16;
             const int row = ks / RUNS, x = (ks % RUNS) * 16, z = row / G::TY, y = row % G::TY;
