@@ -503,12 +503,11 @@ def ensemble_extra(capi, cr, device, Q, nmem=64, steps=64, groups=4):
 
 
 def voxelizer_extra(capi, tri, spacing=1.0, repeats=3):
-    """The +z ray-parity voxelizer on the bifurcation's STL: ray-triangle
-    tests per second (each test: 13 FP64 adds / multiplies and one FP64
-    division for the plane crossing; the in-triangle test runs only for
-    crossings), host wall clock around lbm_voxelize (triangle upload, column
-    binning, ray kernel, mask copy back), best of `repeats` after one
-    warm-up call."""
+    """The +z ray-parity voxelizer on the bifurcation's STL: (point, candidate
+    triangle) tests settled per second -- most of them a column at a time, the
+    undecided ones each in the reference's FP64 arithmetic -- host wall clock
+    around capi.voxelize (bounding box, triangle upload, column decisions, mask
+    copy back), best of `repeats` after one warm-up call."""
     capi.voxelize(tri, spacing)
     best, desc = None, None
     for _ in range(repeats):
@@ -517,12 +516,10 @@ def voxelizer_extra(capi, tri, spacing=1.0, repeats=3):
         dt = time.perf_counter() - t0
         best = dt if best is None else min(best, dt)
     tests = int(desc.ray_tests)
-    fp64_nominal = 1.25e12  # GB300 FP64 FLOP/s, nominal (no measured FP64 peak is recorded)
     return {"lattice": list(desc.dims), "triangles": int(len(tri)), "points": int(np.prod(list(desc.dims))),
             "fluid_points": int(desc.fluid_count), "ray_tests": tests, "seconds": best,
-            "tests_per_s": tests / best, "fp64_flop_per_test": 14,
-            "fp64_frac_of_nominal": tests * 14 / best / fp64_nominal,
-            "timing": "host wall clock around lbm_voxelize, best of %d after a warm-up call" % repeats}
+            "tests_per_s": tests / best,
+            "timing": "host wall clock around capi.voxelize, best of %d after a warm-up call" % repeats}
 
 
 def small_ensembles_extra(cr, device, sizes=(1, 4, 16, 64), steps=3000):
