@@ -331,6 +331,16 @@ __device__ __forceinline__ TriExtent tri_extent(const VoxParams& P, const double
         nj += y >= yl - m && y <= yh + m;
     }
     e.pairs = ni * nj;
+    // A facet normal so flat in z that the reference rejects the plane crossing
+    // of every ray (its denominator, the ray's length times the normal's z, is
+    // below 1e-16; a ray's ends move by 0.02 each at most): counted, no columns.
+    // Vertical walls whose vertices are rounded out of the vertical: column_pair
+    // decides none of their pairs.
+    if ((fabs(P.dz) + 0.1 + 1e-12 * P.zabs) * fabs(T[11]) < 1e-16 && isfinite(T[9]) && isfinite(T[10])) {
+        e.i0 = e.j0 = 0;
+        e.i1 = e.j1 = -1;
+        return e;
+    }
     const double uX = T[3] - T[0], uY = T[4] - T[1], uZ = T[5] - T[2];
     const double vX = T[6] - T[0], vY = T[7] - T[1], vZ = T[8] - T[2];
     const double nX = uY * vZ - uZ * vY, nY = uZ * vX - uX * vZ, nZ = uX * vY - uY * vX;
@@ -426,7 +436,8 @@ __global__ void __launch_bounds__(128) k_exact_pairs(const VoxParams P, const do
                                                      uint32_t* __restrict__ bits, const int2* __restrict__ list,
                                                      const VoxCounters* __restrict__ cnt) {
     const int lane = threadIdx.x & 31;
-    const unsigned long long n = min(cnt->npair, (unsigned long long)P.cap);
+    if (cnt->npair > (unsigned long long)P.cap) return;  // the list is not whole: all of it in the second run
+    const unsigned long long n = cnt->npair;
     const int nw = (P.nz + 31) / 32;
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
     for (unsigned long long e = (unsigned long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; e < n * nw;
@@ -451,6 +462,7 @@ __global__ void __launch_bounds__(128) k_exact_pairs(const VoxParams P, const do
 __global__ void __launch_bounds__(128) k_mask(const VoxParams P, const double* __restrict__ tri,
                                               const uint32_t* __restrict__ bits, const int32_t* __restrict__ glob,
                                               uint8_t* __restrict__ mask, VoxCounters* __restrict__ cnt) {
+    if (cnt->npair > (unsigned long long)P.cap) return;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned fluid = 0;
     uint32_t below = 0;  // XOR of the words below kw
