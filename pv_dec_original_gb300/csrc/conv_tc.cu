@@ -37,6 +37,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "lbm_internal.cuh"
 
@@ -813,19 +814,21 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_dx2(const bf16* __res
 //
 // A CTA walks output tiles of TZ x TY x TX voxels, NS of them in flight:
 // per tile a tensor copy of dY (COB channels) and of the input voxels its
-// taps read (16 channels), zero-filled outside the grids (the padding, and
-// ragged tiles, add nothing), swizzled so that the 8 rows of an ldmatrix
-// phase lie in different banks at stride 1 for any tap.  Warps are NG tap
-// groups (TPW taps each) x KG groups of voxel rows; D = dY^T X with
-// m16n8k16 (M = 16 output channels, N = 8 input channels, K = 16 voxels of
-// an x-run).  Bound by the MMAs and shared memory together: an ldmatrix.x4
-// (4 cycles) per four MMAs of 2 cycles at 32 channels.  At 16, a view of an
-// input row serves one output row's MMAs per tap, two per ldmatrix.x4; so a warp
-// with all 9 taps of a tz goes down the rows and uses a view for the three output
-// rows that it meets (ROLL): 4 ldmatrix.x4 for 18 MMAs, 16 -> 16 channels 162 ->
-// 142 us.  256 x 128 x 128: 16 -> 16 142 us (1122 with the tcgen05 im2col), 32 ->
-// 16 275 us (2493), stride-2 16 -> 32 63 us (153), 1x1x1 61 us (411); 128 x 64 x
-// 64, 32 -> 32: 92 us (327).
+// taps read (16 channels), zero-filled outside the grids (the padding),
+// swizzled so that the 8 rows of an ldmatrix phase lie in different banks at
+// stride 1 for any tap.  Warps are NG tap groups (TPW taps each) x KG groups
+// of voxel rows; D = dY^T X with m16n8k16 (M = 16 output channels, N = 8 input
+// channels, K = 16 voxels of an x-run).  Bound by the MMAs and shared memory
+// together: an ldmatrix.x4 (4 cycles) per four MMAs of 2 cycles at 32 channels.
+// At 16, a view of an input row serves one output row's MMAs per tap, two per
+// ldmatrix.x4; so a warp with all 9 taps of a tz goes down the rows and uses a
+// view for the three output rows that it meets (ROLL): 4 ldmatrix.x4 for 18
+// MMAs, 16 -> 16 channels 162 -> 142 us.  256 x 128 x 128: 16 -> 16 142 us (1122
+// with the tcgen05 im2col), 32 -> 16 275 us (2493), stride-2 16 -> 32 63 us
+// (153), 1x1x1 61 us (411); 128 x 64 x 64, 32 -> 32: 92 us (327).
+// A tile at the grid's end leaves out the output voxels outside it: their dY
+// is zero, but X beside them need not be finite, and 0 x Inf would reach taps
+// that no Inf belongs to.
 // grid.y walks the (co / COB) x (ci / 16) channel blocks.  Every
 // FLUSH tiles the KG groups add their sums in turn to the CTA's in shared
 // memory: an MMA drops bits of its accumulator, so that chains of 216 MMAs
@@ -854,7 +857,9 @@ struct WGeo {
     static constexpr int ROW = TAPS * 16 % 32 == 16 ? TAPS * 16 + 8 : TAPS * 16 + 24;
     static constexpr int SUMS = COB * ROW * 4;
     static constexpr int NS = 3 * STAGE + SUMS <= 220 * 1024 ? 3 : 2;
-    static constexpr int SMEM = NS * STAGE + SUMS + 1024;  // stages from a 1024-byte boundary
+    // voxels of zeros, read in place of what no sum may meet: all views of one voxel (ROLL: one row, by itself)
+    static constexpr int ZROWS = ROLL ? 1 : (TPW == 9 ? 2 * XW + 3 : 3);
+    static constexpr int SMEM = NS * STAGE + SUMS + ZROWS * 32 + 1024;  // stages from a 1024-byte boundary
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
 
@@ -877,14 +882,18 @@ __device__ __forceinline__ void mma_m16n8k16(float (&c)[4], const uint32_t (&a)[
 __device__ __forceinline__ uint32_t chunk16(uint32_t v, uint32_t k) { return (v << 5) | ((k << 4) ^ ((v & 4u) << 2)); }
 __device__ __forceinline__ uint32_t chunk32(uint32_t v, uint32_t k) { return (v << 6) | ((k << 4) ^ ((v & 6u) << 3)); }
 
-template <class G>
+// RAGGED: some tiles reach past the grid (the others take the plain sums; a kernel
+// of its own, whose test alone costs whole grids 1.5%).  Without a halo, X is zero
+// wherever dY is: never RAGGED.
+template <class G, bool RAGGED>
 __global__ void __launch_bounds__(G::THREADS, 1) k_conv_wgrad_tiles(const __grid_constant__ CUtensorMap xmap,
                                                                    const __grid_constant__ CUtensorMap ymap,
                                                                    float* __restrict__ dw, int Do, int Ho, int Wo,
-                                                                   int ci, int ntiles) {
+                                                                   int ci, int ntiles, uint32_t copied) {
     constexpr int S = G::S, KS = G::KS, COB = G::COB, NS = G::NS, MT = COB / 16;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[NS];
+    __shared__ int inside[NS];  // of the tile in a stage: its output voxels inside the grid per axis, x | y << 8 | z << 16
     unsigned char* smem = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
     const uint32_t base = saddr(smem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -895,7 +904,9 @@ __global__ void __launch_bounds__(G::THREADS, 1) k_conv_wgrad_tiles(const __grid
     auto issue = [&](int tile, int s) {
         const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
         const uint32_t bar = saddr(full + s), dst = base + s * G::STAGE;
-        mbar_expect_tx(bar, (uint32_t)(G::XBYTES + G::YBYTES));
+        if constexpr (RAGGED)
+            inside[s] = min(Wo - bx * G::TX, G::TX) | min(Ho - by * G::TY, G::TY) << 8 | min(Do - bz * G::TZ, G::TZ) << 16;
+        mbar_expect_tx(bar, copied);
         tma_load4(dst, &xmap, c0, S * bx * G::TX - KS / 2, S * by * G::TY - KS / 2, S * bz * G::TZ - KS / 2, bar);
         tma_load4(dst + G::XPAD, &ymap, o0, bx * G::TX, by * G::TY, bz * G::TZ, bar);
     };
@@ -904,6 +915,10 @@ __global__ void __launch_bounds__(G::THREADS, 1) k_conv_wgrad_tiles(const __grid
         for (int s = 0; s < NS; ++s) mbar_init(saddr(full + s), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    const uint32_t zero = base + NS * G::STAGE + G::SUMS;
+    if constexpr (RAGGED)
+        for (int e = tid; e < G::ZROWS * 2; e += G::THREADS)
+            reinterpret_cast<uint4*>(smem + NS * G::STAGE + G::SUMS)[e] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const int first = blockIdx.x, step = gridDim.x;
     int issued = 0;  // thread 0: tiles issued
@@ -967,52 +982,65 @@ __global__ void __launch_bounds__(G::THREADS, 1) k_conv_wgrad_tiles(const __grid
         ok = __syncthreads_and(ok);
         if (!ok) break;
         const uint32_t xs = base + s * G::STAGE, ys = xs + G::XPAD;
-        if constexpr (G::ROLL) {
-            // x-runs of 16 voxels down the rows: an input row's three views
-            // (tx) meet the output rows of all three ty while they are at hand
+        constexpr int kWhole = G::TX | G::TY << 8 | G::TZ << 16;
+        const int part = RAGGED ? inside[s] : kWhole, ex = part & 0xff, ey = (part >> 8) & 0xff, ez = part >> 16;
+        auto sums = [&](auto whole) {
+            constexpr bool WHOLE = decltype(whole)::value;
             constexpr int RUNS = G::TX / 16;
-            for (int run = kg; run < G::TZ * RUNS; run += G::KG) {
-                const int z = run / RUNS, x = run % RUNS * 16;
-                const uint32_t dv = (uint32_t)(z * G::TY * G::TX + x) + lv, xv = (uint32_t)(z * G::XH * G::XW + x) + lv + tapv;
-                uint32_t a[3][4];
+            if constexpr (G::ROLL) {
+                // x-runs of 16 voxels down the rows: an input row's three views
+                // (tx) meet the output rows of all three ty while they are at hand
+                for (int run = kg; run < G::TZ * RUNS; run += G::KG) {
+                    const int z = run / RUNS, x = run % RUNS * 16;
+                    if (!WHOLE && (z >= ez || x >= ex)) continue;
+                    const bool in = WHOLE || x + (int)lv < ex;
+                    const uint32_t dv = (uint32_t)(z * G::TY * G::TX + x) + lv,
+                                   xv = (uint32_t)(z * G::XH * G::XW + x) + lv + tapv;
+                    uint32_t a[3][4];
 #pragma unroll
-                for (int r = 0; r < G::XH; ++r) {
-                    if (r < G::TY) ldmatrix4_trans(a[r % 3], ys + chunk16(dv + (uint32_t)(r * G::TX), lc));
+                    for (int r = 0; r < G::XH; ++r) {
+                        if (r < G::TY) ldmatrix4_trans(a[r % 3], ys + chunk16(dv + (uint32_t)(r * G::TX), lc));
 #pragma unroll
-                    for (int tx = 0; tx < 3; ++tx) {
+                        for (int tx = 0; tx < 3; ++tx) {
+                            uint32_t b[4];
+                            const uint32_t at = xs + chunk16(xv + (uint32_t)(r * G::XW + tx), lc);
+                            ldmatrix4_trans(b, in ? at : zero);
+#pragma unroll
+                            for (int ty = 0; ty < 3; ++ty) {
+                                const int y = r - ty;
+                                if (y < 0 || y >= G::TY || (!WHOLE && y >= ey)) continue;
+                                mma_m16n8k16(acc[ty * 3 + tx][0][0], a[y % 3], b[0], b[2]);
+                                mma_m16n8k16(acc[ty * 3 + tx][0][1], a[y % 3], b[1], b[3]);
+                            }
+                        }
+                    }
+                }
+            } else {
+                for (int ks = kg; ks < G::KSTEPS; ks += G::KG) {
+                    const int row = ks / RUNS, x = (ks % RUNS) * 16, z = row / G::TY, y = row % G::TY;
+                    if (!WHOLE && (z >= ez || y >= ey || x >= ex)) continue;
+                    const bool in = WHOLE || x + (int)lv < ex;
+                    const uint32_t dv = (uint32_t)(row * G::TX + x) + lv;
+                    uint32_t a[MT][4];
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+                        ldmatrix4_trans(a[m], ys + (COB == 16 ? chunk16(dv, lc) : chunk32(dv, 2 * m + lc)));
+                    const uint32_t xv = in ? (uint32_t)((S * z * G::XH + S * y) * G::XW + S * x) + S * lv + tapv : (zero - xs) >> 5;
+#pragma unroll
+                    for (int t = 0; t < G::TPW; ++t) {
                         uint32_t b[4];
-                        ldmatrix4_trans(b, xs + chunk16(xv + (uint32_t)(r * G::XW + tx), lc));
+                        ldmatrix4_trans(b, xs + chunk16(xv + (uint32_t)((t / 3) * G::XW + t % 3), lc));
 #pragma unroll
-                        for (int ty = 0; ty < 3; ++ty) {
-                            const int y = r - ty;
-                            if (y < 0 || y >= G::TY) continue;
-                            mma_m16n8k16(acc[ty * 3 + tx][0][0], a[y % 3], b[0], b[2]);
-                            mma_m16n8k16(acc[ty * 3 + tx][0][1], a[y % 3], b[1], b[3]);
+                        for (int m = 0; m < MT; ++m) {
+                            mma_m16n8k16(acc[t][m][0], a[m], b[0], b[2]);
+                            mma_m16n8k16(acc[t][m][1], a[m], b[1], b[3]);
                         }
                     }
                 }
             }
-        } else
-        for (int ks = kg; ks < G::KSTEPS; ks += G::KG) {
-            constexpr int RUNS = G::TX / 16;
-            const int row = ks / RUNS, x = (ks % RUNS) * 16, z = row / G::TY, y = row % G::TY;
-            const uint32_t dv = (uint32_t)(row * G::TX + x) + lv;
-            uint32_t a[MT][4];
-#pragma unroll
-            for (int m = 0; m < MT; ++m)
-                ldmatrix4_trans(a[m], ys + (COB == 16 ? chunk16(dv, lc) : chunk32(dv, 2 * m + lc)));
-            const uint32_t xv = (uint32_t)((S * z * G::XH + S * y) * G::XW + S * x) + S * lv + tapv;
-#pragma unroll
-            for (int t = 0; t < G::TPW; ++t) {
-                uint32_t b[4];
-                ldmatrix4_trans(b, xs + chunk16(xv + (uint32_t)((t / 3) * G::XW + t % 3), lc));
-#pragma unroll
-                for (int m = 0; m < MT; ++m) {
-                    mma_m16n8k16(acc[t][m][0], a[m], b[0], b[2]);
-                    mma_m16n8k16(acc[t][m][1], a[m], b[1], b[3]);
-                }
-            }
-        }
+        };
+        if (!RAGGED || part == kWhole) sums(std::integral_constant<bool, true>());
+        else if constexpr (RAGGED) sums(std::integral_constant<bool, false>());
         __syncthreads();
         if ((it + 1) % G::FLUSH == 0) flush();
     }
@@ -1101,18 +1129,24 @@ cudaError_t launch_wgrad(const bf16* x, const bf16* dy, float* dw, int Di, int H
                          cudaStream_t st) {
     const int Do = (Di - 1) / G::S + 1, Ho = (Hi - 1) / G::S + 1, Wo = (Wi - 1) / G::S + 1;
     CUtensorMap xm, ym;
-    cudaError_t e = tile_map(&xm, x, Di, Hi, Wi, ci, G::XD, G::XH, G::XW, 16);
-    if (e == cudaSuccess) e = tile_map(&ym, dy, Do, Ho, Wo, co, G::TZ, G::TY, G::TX, G::COB);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_conv_wgrad_tiles<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+    // a grid of fewer planes than a tile's copies no more of them (they are not read)
+    const int tz = G::KS == 3 && Do < G::TZ ? Do : G::TZ, xd = G::S * (tz - 1) + G::KS;
+    cudaError_t e = tile_map(&xm, x, Di, Hi, Wi, ci, xd, G::XH, G::XW, 16);
+    if (e == cudaSuccess) e = tile_map(&ym, dy, Do, Ho, Wo, co, tz, G::TY, G::TX, G::COB);
+    bool ragged = false;
+    if constexpr (G::KS == 3) ragged = Do % G::TZ || Ho % G::TY || Wo % G::TX;
+    auto kern = k_conv_wgrad_tiles<G, false>;
+    if constexpr (G::KS == 3)
+        if (ragged) kern = k_conv_wgrad_tiles<G, true>;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
     if (e != cudaSuccess) return e;
     const int64_t tiles = lbm::ceil_div(Do, G::TZ) * lbm::ceil_div(Ho, G::TY) * lbm::ceil_div(Wo, G::TX);
     const int roles = co / G::COB * (ci / 16);
     // one CTA an SM over all channel blocks, each with about the same number of tiles
     const int64_t want = 152 / roles > 1 ? 152 / roles : 1;
     const int64_t per = lbm::ceil_div(tiles, want);
-    k_conv_wgrad_tiles<G><<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)roles), G::THREADS, G::SMEM, st>>>(
-        xm, ym, dw, Do, Ho, Wo, ci, (int)tiles);
+    kern<<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)roles), G::THREADS, G::SMEM, st>>>(
+        xm, ym, dw, Do, Ho, Wo, ci, (int)tiles, (uint32_t)(G::XBYTES / G::XD * xd + G::YBYTES / G::TZ * tz));
     return cudaGetLastError();
 }
 
