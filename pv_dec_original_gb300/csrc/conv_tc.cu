@@ -1263,8 +1263,15 @@ cudaError_t conv3_dx2(const void* dy, const void* wt, void* dx, int D, int H, in
 
 bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride) {
     const bool ch = (ci == 16 || ci == 32 || ci == 64) && (co == 16 || co == 32 || co == 64);
-    return ch && D > 0 && H > 0 && W > 0 && ((ks == 3 && (stride == 1 || stride == 2)) || (ks == 1 && stride == 1)) &&
-           (int64_t)D * H * W < ((int64_t)1 << 31);
+    if (!ch || D <= 0 || H <= 0 || W <= 0 || !((ks == 3 && (stride == 1 || stride == 2)) || (ks == 1 && stride == 1)))
+        return false;
+    // Of a few voxels a sum costs less than a tile's way through shared memory and
+    // the block's sums: the plain mma.sync kernel, a block a tap (us here / there, 3x3x3
+    // stride 1, 16 -> 16 and 64 -> 64 channels: 1 voxel 8.6 / 4.3 and 10.5 / 4.4, 64 10.8 / 6.5
+    // and 12.6 / 8.3, 93 10.6 / 8.4 and 14.6 / 10.3, 128 9.2 / 10.4 and 12.5 / 12.4, 512
+    // 11.5 / 32.0; stride 2, 64: 8.4 / 6.5, 125 8.6 / 10.4; 1x1x1, 16: 6.1 / 4.2, 51 5.7 / 6.4).
+    const int64_t out = (int64_t)((D - 1) / stride + 1) * ((H - 1) / stride + 1) * ((W - 1) / stride + 1);
+    return out > (ks == 3 ? 96 : 24) && (int64_t)D * H * W < ((int64_t)1 << 31);
 }
 
 cudaError_t conv_wgrad_tiles(const void* x, int D, int H, int W, int ci, const void* dy, int co, int ks, int stride,

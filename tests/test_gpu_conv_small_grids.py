@@ -1,0 +1,44 @@
+"""Weight gradients on either side of the line of the dispatch -- the plain kernel
+up to 96 output voxels at kernel size 3 and 24 at 1 -- and on grids thinner than a
+tile along z, against PyTorch in FP64."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _bf(a):
+    return torch.as_tensor(a).to(torch.bfloat16).to(torch.float64)
+
+
+@pytest.mark.parametrize("dims,ks,s", [((1, 1, 96), 3, 1), ((1, 1, 97), 3, 1), ((4, 8, 3), 3, 1), ((7, 2, 7), 3, 1),
+                                       ((1, 1, 191), 3, 2), ((1, 1, 193), 3, 2), ((8, 8, 11), 3, 2), ((1, 1, 24), 1, 1),
+                                       ((1, 5, 5), 1, 1), ((1, 20, 37), 3, 1), ((2, 9, 33), 3, 1), ((3, 17, 15), 3, 1),
+                                       ((1, 20, 37), 3, 2), ((2, 33, 36), 3, 2), ((3, 18, 70), 3, 2), ((1, 11, 13), 1, 1)])
+@pytest.mark.parametrize("ci,co", [(16, 16), (32, 64), (64, 16)])
+def test_gpu_weight_gradient_small_grids(gpu_lib, ci, co, dims, ks, s):
+    """FP32 sums of BF16-exact products: 1e-5 of the gradient's scale, the
+    tolerance of the other weight-gradient tests."""
+    L = gpu_lib.load()
+    rng = np.random.default_rng(ci + 2 * co + sum(dims) + ks + s)
+    x = _bf(rng.normal(size=(*dims, ci)))
+    w = torch.zeros((co, ci, ks, ks, ks), dtype=torch.float64, requires_grad=True)
+    y = torch.nn.functional.conv3d(x.permute(3, 0, 1, 2)[None], w, None, stride=s, padding=ks // 2)
+    dy = _bf(rng.normal(size=(*y.shape[2:], co)))
+    y.backward(dy.permute(3, 0, 1, 2)[None])
+    ref = w.grad.permute(0, 2, 3, 4, 1).reshape(-1)
+    xd, dyd = x.to(torch.bfloat16).cuda().reshape(-1), dy.to(torch.bfloat16).cuda().reshape(-1)
+    wd = torch.zeros(ref.numel(), dtype=torch.bfloat16, device="cuda")
+    dw = torch.full((ref.numel(),), 0.25, device="cuda")
+    gpu_lib._check(L.lbm_nn_conv3d_bwd(_p(xd), (C.c_int * 3)(*dims), ci, _p(wd), None, co, ks, s, _p(dyd), None, _p(dw),
+                                       None, None))
+    torch.cuda.synchronize()
+    gpu_lib._check(L.lbm_nn_conv_status())
+    assert float((dw.cpu().double() - 0.25 - ref).abs().max()) <= 1e-5 * float(ref.abs().max()) + 1e-6
