@@ -1250,6 +1250,11 @@ cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, 
 
 bool conv3_dx2_applies(int D, int H, int W, int ci, int co) {
     const bool ch = (ci == 16 || ci == 32 || ci == 64) && (co == 16 || co == 32 || co == 64);
+    // Columns of a few voxels a plane leave nearly all of a block's 8 x 16 rows
+    // empty: the mma.sync kernel, the same sums bit for bit (64 -> 64 channels, us
+    // here / there: 4096 x 1 x 1 92.6 / 18.7, 2048 x 2 x 2 61.8 / 24.5, 1024 x 4 x 4
+    // 45.3 / 26.9, but 1024 x 8 x 8 44.7 / 73.0).
+    if ((int64_t)((H + 1) / 2) * ((W + 1) / 2) <= 8) return false;
     return ch && D > 0 && H > 0 && W > 0 &&
            ((int64_t)(D + 1) / 2) * ceil_div((H + 1) / 2, TY) * ceil_div((W + 1) / 2, TX) <= 0x7fffffffLL;
 }
