@@ -93,7 +93,7 @@ __host__ __device__ constexpr int gemm_pitch(int kc) { return kc * 2 + 16; }
 // out[r][n] = act(bias[n] + sum_{t,k} src[source(r,t)][k] * B[n][t][k]), taps in
 // order, 16 channels an mma.  NB = columns of a block (n0 = NB blockIdx.y; co
 // in all); blocks walk 64-row tiles with a stride of the grid.  A step is one
-// tap of one tile, all kc channels; kGemmStages - 1 steps' copies are under way
+// tap of one tile, all kc channels; ST - 1 steps' copies are under way
 // (cp.async, zero where there is no source voxel) beside the mma of the oldest,
 // across tiles too.  On the small grids of a network's lowest level a block's
 // chain of 27 steps bounds it (16 x 8 x 8, 64 -> 64 channels: 57 us with one
@@ -102,9 +102,22 @@ __host__ __device__ constexpr int gemm_pitch(int kc) { return kc * 2 + 16; }
 // -> 16 on 256 x 128 x 128: 112 -> 98 us forward with FP32 output, 119 -> 61 us
 // gradient; memory alone 76 and 38).  The order of the sums is the one it
 // always had: networks' values do not change.
-constexpr int kGemmStages = 4;
-template <int MODE, int NB, int KC>
-__global__ void __launch_bounds__(128) k_conv_gemm(const bf16* __restrict__ src, const bf16* __restrict__ B,
+// ST: 4; 2 for the 64 columns of a 1x1 layer, where a block has hardly any sums
+// to hide its stores behind and more blocks an SM do it instead (64 -> 64 on 256 x
+// 128 x 128: 535 us with 4 and 3 blocks an SM, 338 with 2 and 6).  The grid is then
+// as many blocks as are resident, registers capped to that: one block more is a
+// second pass over the tiles of its own.  But one tile a block with 16 channels,
+// where the stores are four times the loads and the next tile need not wait for
+// them (16 -> 64: 316 us with 4, 243 with 2, 197 so; its input gradient 240, 247, 181).
+template <int NB, int KC, int ST>
+__host__ __device__ constexpr int gemm_bytes() { return ST * (kRows + NB) * gemm_pitch(KC); }
+template <int NB, int KC, int ST>
+__host__ __device__ constexpr int gemm_blocks() {  // an SM
+    return ST == 2 ? (KC == 64 ? 6 : (KC == 32 ? 7 : 8))
+                   : (220 * 1024 / gemm_bytes<NB, KC, ST>() < 8 ? 220 * 1024 / gemm_bytes<NB, KC, ST>() : 8);
+}
+template <int MODE, int NB, int KC, int ST>
+__global__ void __launch_bounds__(128, ST == 2 ? gemm_blocks<NB, KC, ST>() : 0) k_conv_gemm(const bf16* __restrict__ src, const bf16* __restrict__ B,
                                                    const float* __restrict__ bias, bf16* __restrict__ out,
                                                    float* __restrict__ out_f32, Conv g, int64_t rows, int64_t ntiles,
                                                    int co, int relu) {
@@ -166,11 +179,11 @@ __global__ void __launch_bounds__(128) k_conv_gemm(const bf16* __restrict__ src,
             }
             if (++ltap == taps) { ltap = 0; lt += gridDim.x; locate(); }
         }
-        if (++slot == kGemmStages) slot = 0;
+        if (++slot == ST) slot = 0;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     locate();
-    for (int k = 0; k < kGemmStages - 1; ++k) copy();
+    for (int k = 0; k < ST - 1; ++k) copy();
 
     float acc[NB / 8][4];
     int at = 0;
@@ -180,7 +193,7 @@ __global__ void __launch_bounds__(128) k_conv_gemm(const bf16* __restrict__ src,
 #pragma unroll
         for (int j = 0; j < NB / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
         for (int t = 0; t < taps; ++t) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kGemmStages - 2) : "memory");
+            asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
             __syncthreads();  // the step's copies are seen, and the slot the next copy takes is read
             copy();
 #pragma unroll
@@ -195,7 +208,7 @@ __global__ void __launch_bounds__(128) k_conv_gemm(const bf16* __restrict__ src,
                     mma_bf16(acc[2 * j + 1], a, b[2], b[3]);
                 }
             }
-            if (++at == kGemmStages) at = 0;
+            if (++at == ST) at = 0;
         }
         // epilogue: bias, ReLU, BF16 (and optionally FP32) store
 #pragma unroll
@@ -892,28 +905,28 @@ Conv make_conv(const int dims_in[3], int ci, int co, int ks, int stride) {
     return g;
 }
 
-template <int MODE, int NB, int KC>
+template <int MODE, int NB, int KC, int ST>
 cudaError_t launch_gemm_kc(const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32, const Conv& g,
                            int64_t rows, int co, int relu, cudaStream_t st) {
-    constexpr int bytes = kGemmStages * (kRows + NB) * gemm_pitch(KC);
+    constexpr int bytes = gemm_bytes<NB, KC, ST>();
     if constexpr (bytes > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_conv_gemm<MODE, NB, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        const cudaError_t e = cudaFuncSetAttribute(k_conv_gemm<MODE, NB, KC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
     }
-    constexpr int64_t fit = 220 * 1024 / bytes, most = 152 * (fit < 8 ? fit : 8);
+    constexpr int64_t most = ST == 2 && KC == 16 ? 0x7fffffff : 152 * gemm_blocks<NB, KC, ST>();
     const int64_t tiles = lbm::ceil_div(rows, kRows);
-    k_conv_gemm<MODE, NB, KC><<<dim3((unsigned)(tiles < most ? tiles : most), (unsigned)(co / NB)), 128, bytes, st>>>(
+    k_conv_gemm<MODE, NB, KC, ST><<<dim3((unsigned)(tiles < most ? tiles : most), (unsigned)(co / NB)), 128, bytes, st>>>(
         src, B, bias, out, out_f32, g, rows, tiles, co, relu);
     return cudaGetLastError();
 }
 
-template <int MODE, int NB>
+template <int MODE, int NB, int ST>
 cudaError_t launch_gemm_nb(const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32, const Conv& g,
                            int64_t rows, int kc, int co, int relu, cudaStream_t st) {
     switch (kc) {
-        case 16: return launch_gemm_kc<MODE, NB, 16>(src, B, bias, out, out_f32, g, rows, co, relu, st);
-        case 32: return launch_gemm_kc<MODE, NB, 32>(src, B, bias, out, out_f32, g, rows, co, relu, st);
-        default: return launch_gemm_kc<MODE, NB, 64>(src, B, bias, out, out_f32, g, rows, co, relu, st);
+        case 16: return launch_gemm_kc<MODE, NB, 16, ST>(src, B, bias, out, out_f32, g, rows, co, relu, st);
+        case 32: return launch_gemm_kc<MODE, NB, 32, ST>(src, B, bias, out, out_f32, g, rows, co, relu, st);
+        default: return launch_gemm_kc<MODE, NB, 64, ST>(src, B, bias, out, out_f32, g, rows, co, relu, st);
     }
 }
 
@@ -924,10 +937,12 @@ template <int MODE>
 cudaError_t launch_gemm(int co, const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32,
                         const Conv& g, int64_t rows, int kc, int relu, cudaStream_t st) {
     if (co > 16 && rows >= (int64_t)kRows * 152) {
-        if (co == 32) return launch_gemm_nb<MODE, 32>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
-        if (co == 64) return launch_gemm_nb<MODE, 64>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
+        if (co == 32) return launch_gemm_nb<MODE, 32, 4>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
+        if (co == 64)
+            return g.ks == 1 ? launch_gemm_nb<MODE, 64, 2>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st)
+                             : launch_gemm_nb<MODE, 64, 4>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
     }
-    return launch_gemm_nb<MODE, 16>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
+    return launch_gemm_nb<MODE, 16, 4>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
 }
 
 template <int CO>
