@@ -103,17 +103,18 @@ __host__ __device__ constexpr int gemm_pitch(int kc) { return kc * 2 + 16; }
 // gradient; memory alone 76 and 38).  The order of the sums is the one it
 // always had: networks' values do not change.
 // ST: 4; 2 for the 64 columns of a 1x1 layer, where a block has hardly any sums
-// to hide its stores behind and more blocks an SM do it instead (64 -> 64 on 256 x
-// 128 x 128: 535 us with 4 and 3 blocks an SM, 338 with 2 and 6).  The grid is then
-// as many blocks as are resident, registers capped to that: one block more is a
-// second pass over the tiles of its own.  But one tile a block with 16 channels,
-// where the stores are four times the loads and the next tile need not wait for
-// them (16 -> 64: 316 us with 4, 243 with 2, 197 so; its input gradient 240, 247, 181).
+// to hide its stores behind and more blocks and registers do it instead (64 -> 64
+// on 256 x 128 x 128: 535 us with 4 stages, 3 blocks an SM and 72 registers, 338 with
+// 2, 4 and 122; 363 with 2, 6 and 72).  The grid is then as many blocks as are
+// resident: one more is a second pass over the tiles of its own.  But one tile a
+// block with 16 channels, where the stores are four times the loads and the next
+// tile need not wait for them (16 -> 64: 316 us with 4 stages, 243 with 2, 197 so;
+// its input gradient 240, 247, 181).
 template <int NB, int KC, int ST>
 __host__ __device__ constexpr int gemm_bytes() { return ST * (kRows + NB) * gemm_pitch(KC); }
 template <int NB, int KC, int ST>
 __host__ __device__ constexpr int gemm_blocks() {  // an SM
-    return ST == 2 ? (KC == 64 ? 6 : (KC == 32 ? 7 : 8))
+    return ST == 2 ? (KC == 16 ? 8 : 4)
                    : (220 * 1024 / gemm_bytes<NB, KC, ST>() < 8 ? 220 * 1024 / gemm_bytes<NB, KC, ST>() : 8);
 }
 template <int MODE, int NB, int KC, int ST>
