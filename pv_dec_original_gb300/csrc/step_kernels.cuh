@@ -1955,16 +1955,23 @@ cudaError_t launch_compact(const StepParams& p, cudaStream_t st) {
 //   D3Q19 from 32 MB a buffer on: the populations come from memory, more
 //   loads in flight pay: FP32 550k (128,8) 11.71, (128,10) 11.56; 900k 19.31,
 //   18.74; 16-bit 1.6M (128,8) 29.23, (128,10) 28.28, (128,12) 28.17; 3.2M 62.5,
-//   57.9, 56.5.
+//   57.9, 56.5;
+//   D3Q19 from 300 MB a buffer on, nothing of it left in L2 from step to step: in 16
+//   bits the flat (128,10) (FP16 compact (128,12) / flat (128,10) 4.8M 94.3 / 100.4,
+//   6.5M 149.5 / 150.3, 9.3M 204.0 / 199.7, 11.9M 264.2 / 255.6, 20.3M 447.6 /
+//   428.7, BF16 alike), in FP32 the compact (128,12) (3.2M, 6.2M and 12M within 0.2%
+//   of (128,10); 12M in narrow tubes 335.6, (128,10) 346.4, the flat (128,12) 344).
 // The flat (128,12) that every such handle started on: 4.41 us at 20k nodes,
 // 8.29 at 250k (compact (128,8) 6.6), D3Q27 13.6 (8.3), FP32 1.4M 40.8 (35.5).
-constexpr int64_t kLatencyNodes = 12000, kMemoryBytes = 32000000;
+constexpr int64_t kLatencyNodes = 12000, kMemoryBytes = 32000000, kLargeBytes = 300000000;
 template <int Q, typename S, int MODE>
 int default_variant(const StepParams& p) {
     if (!Store<S>::offset) return 4;
     if (MODE != MODE_PHYSICS) return 0;
+    const int64_t bytes = (int64_t)Q * p.stride * (int64_t)sizeof(S);
+    if (Q == 19 && bytes >= kLargeBytes) return sizeof(S) == 4 ? 7 : 1;
     if (p.nact <= kLatencyNodes) return 3;
-    if (Q == 27 || (int64_t)Q * p.stride * (int64_t)sizeof(S) < kMemoryBytes) return 4;
+    if (Q == 27 || bytes < kMemoryBytes) return 4;
     return sizeof(S) == 4 ? 6 : 7;
 }
 
