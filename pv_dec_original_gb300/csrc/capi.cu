@@ -14,6 +14,7 @@
 // previous step's populations -- and applies the boundary rules again, or
 // reads buf[0] directly if no step ran since the start.
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -89,9 +90,15 @@ struct lbm_handle {
     int graph_steps = 0;
     int persist = 0;             // steps per persistent launch (0: one launch per step)
     unsigned* bar = nullptr;     // grid barrier of persistent launches: arrivals, extra arrivals (tests)
-    cudaGraphExec_t gexec = nullptr;
-    int gexec_parity = -1;
-    int gexec_cur = -1;
+    struct Captured {  // graph_steps launches from one (step parity, cur)
+        cudaGraphExec_t exec = nullptr;
+        int parity = -1, cur = -1;
+    } captured[2];              // [crowded]
+    int64_t l2_bytes = 0;       // one population buffer
+    bool crowded = false;       // l2_crowded at the last lbm_step_async
+    bool in_flight = false;     // counted in stepping_bytes
+    int64_t beside = 0;         // others' stepping_bytes when its last steps were waited for
+    int64_t step_calls = 0, outputs_at = -1;  // lbm_step_async calls, and their number at the last asynchronous read-out
     int variant = -1;           // launch shape of the step kernel (lbm_autotune); -1: default_variant's
     size_t geo_bytes = 0;
     lbm_counts counts{};
@@ -155,9 +162,37 @@ cudaError_t dalloc(lbm_handle* h, T** p, size_t bytes) {
 }
 
 void drop_graph(lbm_handle* h) {
-    if (h->gexec) cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
-    h->gexec_parity = -1;
+    for (auto& c : h->captured) {
+        if (c.exec) cudaGraphExecDestroy(c.exec);
+        c = {};
+    }
+}
+
+// Bytes of one population buffer of every lattice whose steps were issued and
+// not waited for since, per device: what shares its L2.  It steers launch
+// shapes only, whose results are the same bit for bit.
+constexpr int kStepDevices = 64;
+std::atomic<int64_t> stepping_bytes[kStepDevices];
+
+void steps_done(lbm_handle* h) {
+    if (h->in_flight) h->beside = (stepping_bytes[h->d.device] -= h->l2_bytes);
+    h->in_flight = false;
+}
+
+void steps_issued(lbm_handle* h) {
+    ++h->step_calls;
+    if (h->d.device < 0 || h->d.device >= kStepDevices) return;
+    if (!h->in_flight) stepping_bytes[h->d.device] += h->l2_bytes;
+    h->in_flight = true;
+    // those beside it now, or still at the end of its last steps: of lattices
+    // issued one after another and waited for in turn, the first see none yet
+    h->crowded = l2_crowded(h->l2_bytes, std::max(stepping_bytes[h->d.device].load() - h->l2_bytes, h->beside));
+}
+
+cudaError_t drain(lbm_handle* h) {
+    const cudaError_t e = cudaStreamSynchronize(h->st);
+    if (e == cudaSuccess) steps_done(h);
+    return e;
 }
 
 // Concatenate the host waveforms into the device table; unset waveforms
@@ -191,7 +226,7 @@ int upload_waves(lbm_handle* h) {
         CK(h, cudaEventRecord(h->ev_table, h->st));
         return LBM_OK;
     }
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     if (total > h->amp_cap) {
         drop_graph(h);  // the table pointer is baked into captured launches
         if (h->amp) cudaFree(h->amp);
@@ -206,7 +241,7 @@ int upload_waves(lbm_handle* h) {
                                   cudaMemcpyHostToDevice, h->st));
     CK(h, cudaMemcpyAsync(h->wave_off, off.data(), sizeof(int64_t) * LBM_MAX_WAVES, cudaMemcpyHostToDevice, h->st));
     CK(h, cudaMemcpyAsync(h->wave_len, len.data(), sizeof(int64_t) * LBM_MAX_WAVES, cudaMemcpyHostToDevice, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     h->wave_off_h = off;
     h->wave_len_h = len;
     return LBM_OK;
@@ -233,6 +268,8 @@ int wait_staging(lbm_handle* h, int which) {
 }
 
 void free_geometry(lbm_handle* h) {
+    steps_done(h);
+    h->l2_bytes = 0;
     if (h->cst) cudaStreamSynchronize(h->cst);  // copies still reading staging buffers
     GeometryLists& g = h->g;
     void* ptrs[] = {g.cls, g.sp_pt, g.sp_miss, g.sp_cls, g.sp_nw, g.sp_bc, g.bcidx, g.sp_prof, g.nw_pt, g.act_word,
@@ -279,6 +316,7 @@ StepParams make_params(lbm_handle* h, int kind) {
         p.direct = h->since_start == 0 ? 1 : 0;
     }
     p.odd = h->cur;
+    p.crowded = h->crowded ? 1 : 0;
     p.stride = h->stride;
     p.seg_delta = h->seg_delta;
     p.seg_abs = h->seg_abs;
@@ -365,7 +403,7 @@ int start_state(lbm_handle* h, bool reset) {
     h->cur = 1;
     h->since_start = 0;
     drop_graph(h);  // the graph's buffer roles depend on cur
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     h->has_state = true;
     return LBM_OK;
 }
@@ -376,19 +414,19 @@ static_assert(LBM_NUM_VARIANTS == kNumVariants, "variant count");
 int check_flags(lbm_handle* h) {
     unsigned f = 0;
     CK(h, cudaMemcpyAsync(&f, h->flags, sizeof(unsigned), cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     if (f & FLAG_TIMEOUT) {
         // a bounded wait gave up; clear the flag and a barrier left half-arrived
         CK(h, cudaMemsetAsync(h->flags, 0, sizeof(unsigned), h->st));
         if (h->bar) CK(h, cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned), h->st));
-        CK(h, cudaStreamSynchronize(h->st));
+        CK(h, drain(h));
         return fail(h, LBM_ERR_CUDA,
                     "a step kernel's bounded wait gave up (a tiled step's bulk copy or a persistent launch's grid "
                     "barrier)");
     }
     if (f & FLAG_BOUNDS) {
         CK(h, cudaMemsetAsync(h->flags, 0, sizeof(unsigned), h->st));
-        CK(h, cudaStreamSynchronize(h->st));
+        CK(h, drain(h));
         return fail(h, LBM_ERR_CUDA,
                     "a step kernel's index fell outside its array (bounds-checked build; the access was skipped)");
     }
@@ -439,7 +477,6 @@ bool persist_ok(const lbm_handle* h) { return (int64_t)h->d.Q * h->stride < ((in
 
 // Capture graph_steps (even) launches starting at the current parity.
 int build_graph(lbm_handle* h) {
-    drop_graph(h);
     const int64_t steps0 = h->steps, since0 = h->since_start, launches0 = h->launches;
     const int cur0 = h->cur;
     cudaGraph_t graph = nullptr;
@@ -477,15 +514,16 @@ int build_graph(lbm_handle* h) {
         ++k;
     }
     CK(h, cudaStreamEndCapture(h->st, &graph));
-    cudaError_t e = cudaGraphInstantiate(&h->gexec, graph, 0);
+    auto& captured = h->captured[h->crowded];
+    cudaError_t e = cudaGraphInstantiate(&captured.exec, graph, 0);
     cudaGraphDestroy(graph);
     h->steps = steps0;
     h->since_start = since0;
     h->cur = cur0;
     h->launches = launches0;
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    h->gexec_parity = (int)(steps0 & 1);
-    h->gexec_cur = cur0;
+    captured.parity = (int)(steps0 & 1);
+    captured.cur = cur0;
     return LBM_OK;
 }
 
@@ -768,7 +806,7 @@ lbm_status lbm_set_geometry(lbm_handle* h, const uint8_t* mask, const int dims[3
         REQUIRE(h, bc[b].wave >= 0 && bc[b].wave < LBM_MAX_WAVES, LBM_ERR_ARG, "waveform index out of range");
     }
     CK(h, cudaSetDevice(h->d.device));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     free_geometry(h);
     h->nx = dims[0]; h->ny = dims[1]; h->nz = dims[2];
     h->npts = npts;
@@ -812,6 +850,7 @@ lbm_status lbm_set_geometry(lbm_handle* h, const uint8_t* mask, const int dims[3
     CK(h, dalloc(h, &h->buf[1], es * Q * h->stride));
     CK(h, cudaMemsetAsync(h->buf[0], 0, es * Q * h->stride, h->st));
     CK(h, cudaMemsetAsync(h->buf[1], 0, es * Q * h->stride, h->st));
+    h->l2_bytes = (int64_t)es * Q * h->stride;
     if (h->d.mode == LBM_PARITY) {
         for (void*& b : h->stale) CK(h, dalloc(h, &b, rs * Q * (h->g.nsp + 1)));
         CK(h, dalloc(h, &h->nw_prev, rs * 4 * (h->g.nnw + 1)));
@@ -848,7 +887,7 @@ lbm_status lbm_set_geometry(lbm_handle* h, const uint8_t* mask, const int dims[3
         CK(h, cudaMemcpyAsync(h->sp_bc.data(), h->g.sp_bc, sizeof(int32_t) * h->g.nsp, cudaMemcpyDeviceToHost,
                               h->st));
     }
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     lbm_counts c{};
     c.points = h->npts;
     c.active = h->g.nact;
@@ -898,7 +937,7 @@ lbm_status lbm_set_normals_from_surface(lbm_handle* h, const double* tri12, int6
     if (e == cudaSuccess)
         e = surface_normals(d_tri, ntri, h->g.nw_pt, h->g.nnw, h->nx, h->ny, h->d.origin, h->d.spacing, h->nw_n, h->st);
     if (e == cudaSuccess) e = normals_to_float(h->nw_n, h->g.nnw, h->nw_stride, h->nw_nf, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    if (e == cudaSuccess) e = drain(h);
     cudaFree(d_tri);
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("normals: ") + cudaGetErrorString(e));
     return LBM_OK;
@@ -915,7 +954,7 @@ lbm_status lbm_set_normals_from_surface_box(lbm_handle* h, const double* tri12, 
     // next-to-wall points inside the box
     std::vector<int64_t> pt(nn), sel_idx, sel_pt;
     CK(h, cudaMemcpyAsync(pt.data(), h->g.nw_pt, sizeof(int64_t) * nn, cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     const int64_t nxy = (int64_t)h->nx * h->ny;
     for (int64_t p = 0; p < nn; ++p) {
         const int64_t n = pt[p];
@@ -946,7 +985,7 @@ lbm_status lbm_set_normals_from_surface_box(lbm_handle* h, const double* tri12, 
     if (e == cudaSuccess) e = surface_normals(d_tri, ntri, d_pt, m, h->nx, h->ny, h->d.origin, h->d.spacing, d_out, h->st);
     if (e == cudaSuccess) e = scatter_normals(d_out, d_pt + m, m, nn, h->nw_n, h->st);
     if (e == cudaSuccess) e = normals_to_float(h->nw_n, nn, h->nw_stride, h->nw_nf, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    if (e == cudaSuccess) e = drain(h);
     cudaFree(d_tri);
     cudaFree(d_pt);
     cudaFree(d_out);
@@ -960,7 +999,7 @@ lbm_status lbm_set_wall_distances(lbm_handle* h, const double* tri12, int64_t nt
     REQUIRE(h, h->d.mode == LBM_PHYSICS, LBM_ERR_ARG, "interpolated bounce-back is a physics-mode rule");
     REQUIRE(h, ntri >= 0 && (ntri == 0 || tri12), LBM_ERR_ARG, "null triangles");
     CK(h, cudaSetDevice(h->d.device));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     drop_graph(h);  // the table pointer is baked into captured launches
     if (ntri == 0) {
         if (h->sp_q) cudaFree(h->sp_q);
@@ -973,7 +1012,7 @@ lbm_status lbm_set_wall_distances(lbm_handle* h, const double* tri12, int64_t nt
     cudaError_t e = cudaMemcpyAsync(d_tri, tri12, sizeof(double) * 12 * ntri, cudaMemcpyHostToDevice, h->st);
     if (e == cudaSuccess)
         e = wall_distances(h->d.Q, d_tri, ntri, h->g, h->nx, h->ny, h->d.origin, h->d.spacing, h->sp_q, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    if (e == cudaSuccess) e = drain(h);
     cudaFree(d_tri);
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("wall distances: ") + cudaGetErrorString(e));
     return LBM_OK;
@@ -989,7 +1028,7 @@ lbm_status lbm_get_wall_distances(lbm_handle* h, int64_t* pt, float* q) {
     std::vector<float> planes((size_t)Q * n, 0.5f);
     if (q && n && h->sp_q)
         CK(h, cudaMemcpyAsync(planes.data(), h->sp_q, sizeof(float) * Q * n, cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     if (q)
         for (int64_t e = 0; e < n; ++e)
             for (int k = 0; k < Q; ++k) q[e * Q + k] = planes[(size_t)k * n + e];
@@ -1068,7 +1107,7 @@ lbm_status lbm_init_from_macro(lbm_handle* h, const float* rho, const float* u, 
                          regularized, h->out_f, h->st);
     if (e == cudaSuccess)
         e = init_state(h->d.precision, h->d.Q, 1, h->buf[0], h->stride, h->out_f, na, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    if (e == cudaSuccess) e = drain(h);
     cudaFree(d_rho);
     if (d_u) cudaFree(d_u);
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("init_from_macro: ") + cudaGetErrorString(e));
@@ -1092,7 +1131,10 @@ lbm_status lbm_step_async(lbm_handle* h, int nsteps) {
     REQUIRE(h, h->has_state, LBM_ERR_STATE, "no state: set the geometry first");
     REQUIRE(h, nsteps >= 0, LBM_ERR_ARG, "negative step count");
     CK(h, cudaSetDevice(h->d.device));
-    if (nsteps > 0) h->wss_from_ckpt = false;
+    if (nsteps > 0) {
+        h->wss_from_ckpt = false;
+        steps_issued(h);
+    }
     REQUIRE(h, h->persist == 0 || persist_ok(h), LBM_ERR_UNSUPPORTED,
             "persistent steps need 32-bit population offsets (Q * stride < 2^31)");
     int left = nsteps;
@@ -1101,17 +1143,18 @@ lbm_status lbm_step_async(lbm_handle* h, int nsteps) {
     // one (cur, parity) is valid whenever that pair recurs -- one direct step
     // re-aligns otherwise.
     while (h->graph_steps > 0 && left >= h->graph_steps) {
-        if (h->gexec && (h->gexec_parity != (int)(h->steps & 1) || h->gexec_cur != h->cur)) {
+        const auto& graph = h->captured[h->crowded];
+        if (graph.exec && (graph.parity != (int)(h->steps & 1) || graph.cur != h->cur)) {
             int rc = one_step(h);
             if (rc) return rc;
             --left;
             continue;
         }
-        if (!h->gexec) {
+        if (!graph.exec) {
             int rc = build_graph(h);
             if (rc) return rc;
         }
-        CK(h, cudaGraphLaunch(h->gexec, h->st));
+        CK(h, cudaGraphLaunch(graph.exec, h->st));
         h->launches += h->persist > 0 ? h->graph_steps / h->persist : h->graph_steps;
         h->steps += h->graph_steps;
         h->since_start += h->graph_steps;
@@ -1131,7 +1174,7 @@ lbm_status lbm_step_async(lbm_handle* h, int nsteps) {
 
 lbm_status lbm_sync(lbm_handle* h) {
     if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1166,7 +1209,7 @@ lbm_status lbm_preset_barrier(lbm_handle* h, unsigned extra_arrivals) {
     REQUIRE(h, h->bar, LBM_ERR_STATE, "no persistent barrier: call lbm_set_persistent first");
     CK(h, cudaSetDevice(h->d.device));
     CK(h, cudaMemcpyAsync(h->bar + 1, &extra_arrivals, sizeof(unsigned), cudaMemcpyHostToDevice, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1177,7 +1220,7 @@ lbm_status lbm_preset_flags(lbm_handle* h, unsigned flags) {
             "only LBM_FLAG_NONFINITE and LBM_FLAG_BOUNDS can be preset");
     CK(h, cudaSetDevice(h->d.device));
     CK(h, cudaMemcpyAsync(h->flags, &flags, sizeof(unsigned), cudaMemcpyHostToDevice, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1193,7 +1236,7 @@ lbm_status lbm_get_classes(lbm_handle* h, uint8_t* cls) {
     if (!h || !cls) return fail(h, LBM_ERR_ARG, "null handle or output");
     REQUIRE(h, h->has_geo, LBM_ERR_STATE, "set the geometry first");
     CK(h, cudaMemcpyAsync(cls, h->g.cls, h->npts, cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1203,7 +1246,7 @@ lbm_status lbm_get_distributions(lbm_handle* h, double* f) {
     int rc = readout(h, true);
     if (rc) return rc;
     CK(h, cudaMemcpyAsync(f, h->out_f, sizeof(double) * h->g.nact * h->d.Q, cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1245,7 +1288,7 @@ lbm_status lbm_get_macro(lbm_handle* h, double* rho, double* u3) {
     int rc = macro_to_staging(h);
     if (!rc) rc = macro_copies(h, rho, u3, h->st);
     if (rc) return rc;
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1260,6 +1303,7 @@ lbm_status lbm_get_macro_async(lbm_handle* h, double* rho, double* u3) {
     rc = macro_copies(h, rho, u3, h->cst);
     if (rc) return rc;
     CK(h, cudaEventRecord(h->ev_copied[0], h->cst));
+    h->outputs_at = h->step_calls;
     return LBM_OK;
 }
 
@@ -1267,6 +1311,7 @@ lbm_status lbm_wait_outputs(lbm_handle* h) {
     if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
     CK(h, cudaSetDevice(h->d.device));
     if (h->cst) CK(h, cudaStreamSynchronize(h->cst));
+    if (h->cst && h->outputs_at == h->step_calls) steps_done(h);  // the read-outs waited for came after every step issued
     return LBM_OK;
 }
 
@@ -1297,7 +1342,7 @@ int read_accumulators(lbm_handle* h, std::vector<double>& w, std::vector<double>
         CK(h, cudaMemcpyAsync(w.data(), h->nw_wss, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
         CK(h, cudaMemcpyAsync(a.data(), h->nw_acc, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->st));
         CK(h, cudaMemcpyAsync(am.data(), h->nw_accm, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
-        CK(h, cudaStreamSynchronize(h->st));
+        CK(h, drain(h));
         return LBM_OK;
     }
     int first, pending, last;
@@ -1308,7 +1353,7 @@ int read_accumulators(lbm_handle* h, std::vector<double>& w, std::vector<double>
     CK(h, cudaMemcpyAsync(w.data(), h->nw_out, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
     CK(h, cudaMemcpyAsync(a.data(), h->nw_out + n, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->st));
     CK(h, cudaMemcpyAsync(am.data(), h->nw_out + 4 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1320,7 +1365,7 @@ int write_accumulators(lbm_handle* h, const std::vector<double>& w, const std::v
         CK(h, cudaMemcpyAsync(h->nw_wss, w.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
         CK(h, cudaMemcpyAsync(h->nw_acc, a.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->st));
         CK(h, cudaMemcpyAsync(h->nw_accm, am.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
-        CK(h, cudaStreamSynchronize(h->st));
+        CK(h, drain(h));
         return LBM_OK;
     }
     std::vector<float> wf(n);
@@ -1336,7 +1381,7 @@ int write_accumulators(lbm_handle* h, const std::vector<double>& w, const std::v
     // the accumulators hold every step so far: no ring slot is pending
     CK(h, cudaMemsetAsync(h->nw_ring, 0, sizeof(float) * kRingSlots * 4 * (n + 1), h->st));
     h->wss_from_ckpt = true;
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1400,7 +1445,7 @@ lbm_status lbm_get_wss(lbm_handle* h, int64_t* pt, double* normal3, double* wss,
     int rc = wss_to_staging(h);
     if (!rc) rc = wss_copies(h, pt, normal3, wss, acc3, acc_mag, osi, tawss, h->st);
     if (rc) return rc;
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     return LBM_OK;
 }
 
@@ -1418,6 +1463,7 @@ lbm_status lbm_get_wss_async(lbm_handle* h, int64_t* pt, double* normal3, double
     rc = wss_copies(h, pt, normal3, wss, acc3, acc_mag, osi, tawss, h->cst);
     if (rc) return rc;
     CK(h, cudaEventRecord(h->ev_copied[1], h->cst));
+    h->outputs_at = h->step_calls;
     return LBM_OK;
 }
 
@@ -1441,7 +1487,7 @@ lbm_status lbm_nearest_next_to_wall(lbm_handle* h, const double* xyz, int64_t nv
     if (e == cudaSuccess) e = cudaMemcpyAsync(nw_index, d_idx, sizeof(int64_t) * nv, cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess && distance)
         e = cudaMemcpyAsync(distance, d_dist, sizeof(double) * nv, cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    if (e == cudaSuccess) e = drain(h);
     cudaFree(d_xyz);
     if (d_idx) cudaFree(d_idx);
     if (d_dist) cudaFree(d_dist);
@@ -1456,7 +1502,7 @@ lbm_status lbm_get_conservation(lbm_handle* h, double* mass, double* mom3, doubl
     if (rc) return rc;
     double s[kPartialStride];
     CK(h, cudaMemcpyAsync(s, h->sums, sizeof(s), cudaMemcpyDeviceToHost, h->st));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     if (mass) *mass = (double)h->g.nact + s[0];  // the kernel sums rho - 1
     if (mom3) { mom3[0] = s[1]; mom3[1] = s[2]; mom3[2] = s[3]; }
     if (flux) {
@@ -1464,7 +1510,7 @@ lbm_status lbm_get_conservation(lbm_handle* h, double* mass, double* mom3, doubl
         std::vector<double> fx(h->g.nsp);
         if (h->g.nsp) CK(h, cudaMemcpyAsync(fx.data(), h->sp_flux, sizeof(double) * h->g.nsp,
                                             cudaMemcpyDeviceToHost, h->st));
-        CK(h, cudaStreamSynchronize(h->st));
+        CK(h, drain(h));
         for (int b = 0; b < h->nbc; ++b) flux[b] = 0.0;
         for (int64_t e = 0; e < h->g.nsp; ++e)
             if (h->sp_bc[e] >= 0 && h->sp_bc[e] < h->nbc) flux[h->sp_bc[e]] += fx[e];
@@ -1562,7 +1608,7 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* best, float* ms_per
     REQUIRE(h, h->has_state, LBM_ERR_STATE, "no state: set the geometry first");
     REQUIRE(h, trial_steps > 0, LBM_ERR_ARG, "trial_steps must be > 0");
     CK(h, cudaSetDevice(h->d.device));
-    CK(h, cudaStreamSynchronize(h->st));
+    CK(h, drain(h));
     // snapshot of everything a step writes, restored after every trial
     const size_t fbytes = (size_t)elem_size(h->d.precision) * h->d.Q * h->stride;
     const size_t rs = real_size(h->d.precision);
@@ -1593,6 +1639,7 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* best, float* ms_per
     }
     const int64_t steps0 = h->steps, since0 = h->since_start, launches0 = h->launches;
     const int cur0 = h->cur, v0 = h->variant;
+    h->crowded = false;  // until lbm_step_async sees otherwise
     auto restore = [&]() -> cudaError_t {
         for (Item& it : items) {
             cudaError_t e = cudaMemcpyAsync(it.live, it.copy, it.bytes, cudaMemcpyDeviceToDevice, h->st);

@@ -121,7 +121,8 @@ struct StepParams {
     int64_t fold_blocks;      // leading blocks of a step launch that fold the ring, or (FP64) compute the
                               // next-to-wall stress (set by the launcher)
     int odd;                  // which of the two buffers fin is
-    int stream, reverse;      // compact step kernel, set by its launcher: evict-first loads, blocks in the other order
+    int crowded;              // l2_crowded
+    int reverse;              // compact step kernel, set by its launcher: blocks in the other order
     int pdl_early;            // step launch: let the next launch begin at block start (else at block end)
     float2* nw_accf;          // [4][nnw]
     void* nw_prev;            // parity: rho, ux, uy, uz of the previous collision, [4][nnw]
@@ -160,6 +161,11 @@ struct StepParams {
 
 constexpr int kPartialStride = 4;
 constexpr int kStepThreads = 256;
+
+// Whether a lattice of `own` bytes a population buffer shares the L2 (129 MB)
+// with others stepping on its device, `others` bytes of theirs, so that their
+// buffers (two each) do not all fit: it does not step as if the L2 were its own then.
+inline bool l2_crowded(int64_t own, int64_t others) { return others > 0 && own + others > 64000000; }
 
 // Launchers (one per translation unit family).  kind: 0 step, 1 prologue
 // (collide the initial state), 2 materialize (post-boundary f + sums), 3 rho and u.

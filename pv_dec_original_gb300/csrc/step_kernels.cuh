@@ -1327,7 +1327,7 @@ __global__ void __launch_bounds__(BT, MINB) step_kernel(const StepParams P) {
 //
 // What bounds it is the populations' traffic, and how much of it L2 keeps from
 // one step to the next: a step reads the buffer that the step before wrote.
-// P.stream loads the populations evict-first: a line read is dead (the next
+// STREAM loads the populations evict-first: a line read is dead (the next
 // step overwrites it), and leaving it early keeps what this step writes for the
 // next one's reads.  P.reverse runs the blocks in the other order on every
 // second step: what the step before wrote last is read first.  The rule for
@@ -1348,7 +1348,7 @@ __device__ __forceinline__ S load_hinted(const S* p, uint64_t policy) {
     }
 }
 
-template <int Q, typename S, int BT, int MINB>
+template <int Q, typename S, int BT, int MINB, bool STREAM>
 __global__ void __launch_bounds__(BT, MINB) step_compact_kernel(const StepParams P) {
     using R = typename Store<S>::real;
     constexpr int DR = kDeltaRow<Q>, WB = kWarpBlockWords;
@@ -1411,19 +1411,17 @@ __global__ void __launch_bounds__(BT, MINB) step_compact_kernel(const StepParams
     if (a < (uint32_t)P.nact) {
         const S* __restrict__ fin = static_cast<const S*>(P.fin);
         const uint32_t st = (uint32_t)P.stride;
-        uint64_t keep, policy;
-        asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(keep));
-        asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-        if (!P.stream) policy = keep;
+        uint64_t policy = 0;
+        if constexpr (STREAM) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
         R g[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             uint32_t idx = a + (uint32_t)row[q];
             if (q != Lat<Q>::REST && (miss & (1u << Lat<Q>::opp(q)))) idx = a + (uint32_t)Lat<Q>::opp(q) * st;
-            if (in_bounds(idx, (int64_t)Q * st, P.flags))
-                g[q] = Store<S>::template decode<Q>(load_hinted(fin + idx, policy), q);  // w_opp(q) == w_q: the same decode
-            else
-                g[q] = R(0);
+            // (w_opp(q) == w_q: the same decode)
+            if (!in_bounds(idx, (int64_t)Q * st, P.flags)) g[q] = R(0);
+            else if constexpr (STREAM) g[q] = Store<S>::template decode<Q>(load_hinted(fin + idx, policy), q);
+            else g[q] = Store<S>::template load<Q>(fin + idx, q);
         }
         const int slot = nw ? (int)(*P.step_base & (kRingSlots - 1)) : 0;
         node_finish<Q, S, MODE_PHYSICS, KIND_STEP, false>(P, a, 0, s, nw || bc,
@@ -1924,7 +1922,10 @@ cudaError_t launch_tile(const StepParams& p, cudaStream_t st) {
 //   FP16  38 MB 18.74 / 18.43 / 19.46 / 18.89   61 MB 30.96 / 28.17 / 29.88 / 28.89
 //         87 MB 42.75 / 41.05 / 42.20 / 40.99  122 MB 57.90 / 59.65 / 57.28 / 56.47
 //   D3Q27 FP32 76 MB 25.75 / 21.24 / 24.12 / 21.73   130 MB 42.55 / 46.82 / 40.72 / 40.76
-// Below 38 MB both buffers stay in L2 either way (equal within 0.5%).
+// Below 38 MB both buffers stay in L2 either way (equal within 0.5%).  Not beside
+// other lattices' steps (P.crowded, l2_crowded): they share the L2, and evict-first
+// loads of each as if it were alone cost them (11.8M nodes FP32 in 16 lattices,
+// (128,12): 354.5 us a step of all with, 327.0 without).
 constexpr int64_t kStreamBytes = 138000000, kReverseBytes = 86000000;
 template <int Q, typename S, int MODE, int BT, int MB, int FB>
 cudaError_t launch_compact(const StepParams& p, cudaStream_t st) {
@@ -1932,12 +1933,13 @@ cudaError_t launch_compact(const StepParams& p, cudaStream_t st) {
         if (p.warp_block && p.seg_abs && !p.sp_q && (int64_t)Q * p.stride < ((int64_t)1 << 31)) {
             StepParams q = p;
             const int64_t bytes = (int64_t)Q * p.stride * (int64_t)sizeof(S);
-            q.stream = bytes <= kStreamBytes ? 1 : 0;
             q.reverse = bytes >= kReverseBytes ? p.odd : 0;
             q.fold_blocks = ceil_div(p.nnw, (int64_t)BT * kFoldNodes);
             const int64_t nb = ceil_div(p.nact, BT);
             if (nb <= 0) return cudaSuccess;
-            return launch_dependent(step_compact_kernel<Q, S, BT, MB>, q.fold_blocks + nb, BT, MB, q, st);
+            const bool stream = bytes <= kStreamBytes && !p.crowded;
+            return launch_dependent(stream ? step_compact_kernel<Q, S, BT, MB, true> : step_compact_kernel<Q, S, BT, MB, false>,
+                                    q.fold_blocks + nb, BT, MB, q, st);
         }
         return launch_step_variant<Q, S, MODE, 0>(p, st);
     }
@@ -1960,7 +1962,11 @@ cudaError_t launch_compact(const StepParams& p, cudaStream_t st) {
 //   bits the flat (128,10) (FP16 compact (128,12) / flat (128,10) 4.8M 94.3 / 100.4,
 //   6.5M 149.5 / 150.3, 9.3M 204.0 / 199.7, 11.9M 264.2 / 255.6, 20.3M 447.6 /
 //   428.7, BF16 alike), in FP32 the compact (128,12) (3.2M, 6.2M and 12M within 0.2%
-//   of (128,10); 12M in narrow tubes 335.6, (128,10) 346.4, the flat (128,12) 344).
+//   of (128,10); 12M in narrow tubes 335.6, (128,10) 346.4, the flat (128,12) 344);
+//   beside other lattices' steps (P.crowded) the SMs are full whatever a lattice's
+//   size, and warps count: 11.8M nodes in 16 lattices FP32 (128,12) 330.6, (128,10)
+//   351.7, (128,8) 393.4, the flat (128,12) 336; FP16 286.4, 300.6, 333.1, 288; 1.3M in
+//   8, FP32 37.1, 39.1, 43.7, 38.0; D3Q27 5.9M in 32 FP32 253.2, 236.2, 249.0, 262.7.
 // The flat (128,12) that every such handle started on: 4.41 us at 20k nodes,
 // 8.29 at 250k (compact (128,8) 6.6), D3Q27 13.6 (8.3), FP32 1.4M 40.8 (35.5).
 constexpr int64_t kLatencyNodes = 12000, kMemoryBytes = 32000000, kLargeBytes = 300000000;
@@ -1970,6 +1976,7 @@ int default_variant(const StepParams& p) {
     if (MODE != MODE_PHYSICS) return 0;
     const int64_t bytes = (int64_t)Q * p.stride * (int64_t)sizeof(S);
     if (Q == 19 && bytes >= kLargeBytes) return sizeof(S) == 4 ? 7 : 1;
+    if (p.crowded) return Q == 19 ? 7 : 6;
     if (p.nact <= kLatencyNodes) return 3;
     if (Q == 27 || bytes < kMemoryBytes) return 4;
     return sizeof(S) == 4 ? 6 : 7;
