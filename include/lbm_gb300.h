@@ -339,10 +339,13 @@ lbm_status lbm_preset_flags(lbm_handle* h, unsigned flags);
  * (256,3), 4 (256,1) or in FP64 (64,8), 6 and 7 variant 0.  5: the tiled kernel
  * (bulk copies stage each 256-node tile's sources in shared memory; physics mode,
  * FP32 / FP16 / BF16; elsewhere variant 0, or 4 for FP64).  A handle on which
- * none was set takes one by its lattice, precision and number of nodes.
+ * none was set takes one by its lattice, precision and number of nodes, and by
+ * whether other lattices' steps are in flight on its device (the L2 and the SMs
+ * are shared then); results are the same bit for bit.
  * lbm_autotune times each variant for
  * trial_steps steps on a snapshot of the current state, restores the
- * state, keeps the fastest and reports it (and, if ms_per_step is not NULL,
+ * state, keeps the fastest for this lattice by itself (beside other lattices'
+ * steps it takes the shape it would take untuned) and reports it (and, if ms_per_step is not NULL,
  * the time of every variant: LBM_NUM_VARIANTS floats).  No reference
  * counterpart (the reference has a single serial loop). */
 #define LBM_NUM_VARIANTS 8

@@ -23,7 +23,8 @@ def _state(s):
 
 @pytest.mark.parametrize("Q,prec", [(19, "f32"), (19, "f16"), (27, "f32"), (19, "f64")])
 @pytest.mark.parametrize("graph", [0, 4])
-def test_gpu_step_beside_other_lattices(gpu_lib, Q, prec, graph):
+@pytest.mark.parametrize("tune", [False, True])
+def test_gpu_step_beside_other_lattices(gpu_lib, Q, prec, graph, tune):
     box = (40, 33, 31)
     alone = _solver(gpu_lib, box, Q, prec)
     alone.set_graph_steps(graph)
@@ -31,6 +32,8 @@ def test_gpu_step_beside_other_lattices(gpu_lib, Q, prec, graph):
     ref = _state(alone)
     alone.close()
     s = _solver(gpu_lib, box, Q, prec)
+    if tune:
+        s.autotune(2)
     s.set_graph_steps(graph)
     s.step(11)
     other = _solver(gpu_lib, (140, 128, 109))  # 148 MB a buffer: both together beyond the L2
