@@ -1143,7 +1143,7 @@ cudaError_t launch_wgrad(const bf16* x, const bf16* dy, float* dw, int Di, int H
     const int64_t tiles = lbm::ceil_div(Do, G::TZ) * lbm::ceil_div(Ho, G::TY) * lbm::ceil_div(Wo, G::TX);
     const int roles = co / G::COB * (ci / 16);
     // one CTA an SM over all channel blocks, each with about the same number of tiles
-    const int64_t want = 152 / roles > 1 ? 152 / roles : 1;
+    const int64_t want = lbm::sm_count() / roles > 1 ? lbm::sm_count() / roles : 1;
     const int64_t per = lbm::ceil_div(tiles, want);
     kern<<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)roles), G::THREADS, G::SMEM, st>>>(
         xm, ym, dw, Do, Ho, Wo, ci, (int)tiles, (uint32_t)(G::XBYTES / G::XD * xd + G::YBYTES / G::TZ * tz));
@@ -1195,7 +1195,7 @@ cudaError_t launch_pipe(const bf16* x, const bf16* w, const float* bias, bf16* y
     cudaError_t e = cudaFuncSetAttribute(k_conv3_pipe<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     const int parts = co / CO;
-    const int64_t per = lbm::ceil_div(tiles, 152 / parts);
+    const int64_t per = lbm::ceil_div(tiles, lbm::sm_count() / parts > 1 ? lbm::sm_count() / parts : 1);
     k_conv3_pipe<CO><<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)parts), kPipeThreads, p.bytes, st>>>(
         x, w, bias, y, y32, D, H, W, ci, co, relu, (int)tiles, p.stages);
     return cudaGetLastError();
@@ -1210,7 +1210,7 @@ cudaError_t launch_dx2(const bf16* dy, const bf16* wt, bf16* dx, int D, int H, i
     cudaError_t e = cudaFuncSetAttribute(k_conv3_dx2<CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     const int parts = ci / CI;
-    const int64_t per = lbm::ceil_div(tiles, 152 / parts);
+    const int64_t per = lbm::ceil_div(tiles, lbm::sm_count() / parts > 1 ? lbm::sm_count() / parts : 1);
     k_conv3_dx2<CI><<<dim3((unsigned)lbm::ceil_div(tiles, per), (unsigned)parts), kPipeThreads, p.bytes, st>>>(
         dy, wt, dx, D, H, W, ci, Do, Ho, Wo, co, (int)tiles, p.stages);
     return cudaGetLastError();

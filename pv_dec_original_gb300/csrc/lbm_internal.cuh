@@ -1,5 +1,6 @@
 // Internal device structures shared by the library's translation units.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <cuda_runtime.h>
@@ -241,6 +242,21 @@ cudaError_t scatter_normals(const double* part, const int64_t* idx, int64_t m, i
 cudaError_t normals_to_float(const double* n, int64_t nn, int64_t stride, float* out, cudaStream_t s);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// SMs of the current device (asked for once per device; 1 where that fails, as
+// the launch that follows then does): grids of resident blocks.
+inline int sm_count() {
+    constexpr int kDevs = 64;
+    static std::atomic<int> known[kDevs];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 1;
+    int n = dev < kDevs ? known[dev].load(std::memory_order_acquire) : 0;
+    if (n <= 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 1;
+        if (dev < kDevs) known[dev].store(n, std::memory_order_release);
+    }
+    return n;
+}
 
 // Entries per pull-segment row of the delta table: Q offsets padded to a
 // multiple of 4 (one 16-byte load per 4 offsets).

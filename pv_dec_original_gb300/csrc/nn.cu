@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(const bf16* __restrict__ x, 
 // Blocks of a reduction over n items of 256-thread blocks: a few resident
 // waves, so that every block ends with one atomic per output.
 unsigned reduce_blocks(int64_t n) {
-    const int64_t need = lbm::ceil_div(n, 256), most = 152 * 4;
+    const int64_t need = lbm::ceil_div(n, 256), most = lbm::sm_count() * 4;
     return (unsigned)(need < 1 ? 1 : (need < most ? need : most));
 }
 
@@ -914,7 +914,7 @@ cudaError_t launch_gemm_kc(const bf16* src, const bf16* B, const float* bias, bf
         const cudaError_t e = cudaFuncSetAttribute(k_conv_gemm<MODE, NB, KC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
     }
-    constexpr int64_t most = ST == 2 && KC == 16 ? 0x7fffffff : 152 * gemm_blocks<NB, KC, ST>();
+    const int64_t most = ST == 2 && KC == 16 ? 0x7fffffff : lbm::sm_count() * gemm_blocks<NB, KC, ST>();
     const int64_t tiles = lbm::ceil_div(rows, kRows);
     k_conv_gemm<MODE, NB, KC, ST><<<dim3((unsigned)(tiles < most ? tiles : most), (unsigned)(co / NB)), 128, bytes, st>>>(
         src, B, bias, out, out_f32, g, rows, tiles, co, relu);
@@ -937,7 +937,7 @@ cudaError_t launch_gemm_nb(const bf16* src, const bf16* B, const float* bias, bf
 template <int MODE>
 cudaError_t launch_gemm(int co, const bf16* src, const bf16* B, const float* bias, bf16* out, float* out_f32,
                         const Conv& g, int64_t rows, int kc, int relu, cudaStream_t st) {
-    if (co > 16 && rows >= (int64_t)kRows * 152) {
+    if (co > 16 && rows >= (int64_t)kRows * lbm::sm_count()) {
         if (co == 32) return launch_gemm_nb<MODE, 32, 4>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st);
         if (co == 64)
             return g.ks == 1 ? launch_gemm_nb<MODE, 64, 2>(src, B, bias, out, out_f32, g, rows, kc, co, relu, st)

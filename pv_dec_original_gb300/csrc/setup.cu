@@ -647,7 +647,7 @@ cudaError_t surface_normals(const double* d_tri, int64_t ntri, const int64_t* d_
     if (ntri > 0) k_tri_weights<<<blocks(ntri), 256, 0, st>>>(d_tri, ntri, tw);
     // about 8 blocks an SM, at least a tile of triangles each
     const int64_t nb = ceil_div(npts, kNormThreads);
-    int64_t parts = std::min(ceil_div(8 * 152, nb), ceil_div(ntri > 0 ? ntri : 1, kNormTile));
+    int64_t parts = std::min(ceil_div(8 * sm_count(), nb), ceil_div(ntri > 0 ? ntri : 1, kNormTile));
     const int64_t per = ceil_div(ceil_div(ntri > 0 ? ntri : 1, parts), 4) * 4;
     parts = ceil_div(ntri > 0 ? ntri : 1, per);
     double* sums = nullptr;

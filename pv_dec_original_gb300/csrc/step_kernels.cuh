@@ -1454,22 +1454,8 @@ constexpr Variant variant_shape() {
 // pdl_trigger / pdl_wait); minb: the kernel's minimum resident blocks per SM.
 inline cudaError_t launch_dependent(void (*kern)(const StepParams), int64_t nblocks, int bt, int minb,
                                     const StepParams& p0, cudaStream_t st) {
-    // SM count per device ordinal (handles on different devices may step
-    // from different threads)
-    constexpr int kDevs = 64;
-    static std::atomic<int> sms_of[kDevs];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kDevs) return cudaErrorInvalidDevice;
-    int sms = sms_of[dev].load(std::memory_order_acquire);
-    if (sms <= 0) {
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        sms_of[dev].store(sms, std::memory_order_release);
-    }
     StepParams p = p0;
-    p.pdl_early = nblocks > (int64_t)minb * sms ? 1 : 0;
+    p.pdl_early = nblocks > (int64_t)minb * sm_count() ? 1 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)nblocks);
     cfg.blockDim = dim3(bt);
