@@ -973,7 +973,7 @@ def run_ours(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
                          "bytes_per_lu": bpl, "peak_source": peak_kind,
-                         "kernel": (f"lbm::step_compact_kernel<{args.Q}, {args.precision}>" if tuned[0] in (6, 7)
+                         "kernel": (f"lbm::step_compact_kernel<{args.Q}, {args.precision}>" if tuned[0] in (3, 4, 6, 7)
                                     else f"lbm::step_kernel<{args.Q}, {args.precision}, physics, step>"),
                          "launch_variant": tuned[0]},
             "cpu_baseline": cpu,
