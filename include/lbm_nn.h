@@ -28,10 +28,12 @@ lbm_status lbm_nn_conv3d_fwd(const void* x, const int dims_in[3], int ci, const 
 
 /* Convolution engine.  LBM_NN_ENGINE_AUTO (default): 3x3x3 convolutions
  * run on the tcgen05 tensor cores with tensor-memory accumulators
- * (conv_tc.cu) -- the forward pass at stride 1 and the input gradients on
- * any grid, the forward pass at stride 2 on even grids whose output has
- * H % 16 and W % 8 == 0; the others run on mma.sync, the weight gradients (kernel size 3
- * and 1, any grid) on the staged-tile kernel of conv_tc.cu.
+ * (conv_tc.cu) -- the forward pass and the input gradient at stride 1 on grids
+ * of H >= 16 (lower ones keep the order of summation of the mma.sync kernel),
+ * the forward pass at stride 2 on even grids whose output has H % 16 and W % 8
+ * == 0, the input gradient at stride 2 where an output plane has more than 8
+ * voxels; the others run on mma.sync.  The weight gradients (kernel size 3 and
+ * 1) run on the staged-tile kernel of conv_tc.cu but for a few voxels.
  * LBM_NN_ENGINE_MMA_SYNC: the plain mma.sync kernels everywhere (the
  * comparison path).
  * Process-wide. */

@@ -330,7 +330,8 @@ __global__ void __launch_bounds__(kThreads) k_conv3_s2_tc(const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------
-// Stride 1 (forward, and the input gradient with flipped weights), any grid.
+// Stride 1 (forward, and the input gradient with flipped weights): any grid,
+// of which conv3_tc_applies gives it those of 16 rows or more.
 // The same block (8 x 16 x 4 outputs), staged layout and MMAs as described
 // at the top, in one persistent CTA an SM whose warps each do one thing:
 //   warps 0-3  epilogue: tensor memory -> bias, ReLU -> global memory
@@ -581,7 +582,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_conv3_pipe(const bf16* __re
 }
 
 // ---------------------------------------------------------------------------
-// Input gradient at stride 2, any grid: dx[i] = sum over taps t of
+// Input gradient at stride 2, any grid (conv3_dx2_applies: planes of more than 8
+// output voxels): dx[i] = sum over taps t of
 // dY[(i + 1 - t) / 2] W[t] where i + 1 - t is even (per axis).  With i =
 // 2 j + p, an even i (p = 0) has one tap, t = 1 at dY[j]; an odd one two,
 // t = 2 at dY[j] and t = 0 at dY[j + 1].  So the 8 parity classes of an 8 x
@@ -1226,7 +1228,8 @@ bool conv3_tc_applies(int D, int H, int W, int ci, int co, int stride) {
     // Lower than a block's 16 rows, as a network's lowest level is: the mma.sync
     // kernel, whose order of summation such levels have always had (a network's
     // gradients move by 4e-4 with the order here; 16 x 8 x 8, 64 -> 64 channels
-    // take 12 us there, 9 here).
+    // take 12 us there, 9 here).  A line drawn for values: the kernel here takes
+    // such grids too.
     if (stride == 1) return H >= TY && ceil_div(D, kPipeZ) * ceil_div(H, TY) * ceil_div(W, TX) <= 0x7fffffffLL;
     if (stride == 2) return D % 2 == 0 && H % (2 * TY) == 0 && W % (2 * TX) == 0;
     return false;

@@ -270,22 +270,21 @@ cudaError_t nw_readout_f32(const float2* accf, const float* ring, int64_t nnw, i
                            const float* wss_ckpt, double* out, cudaStream_t st);
 
 // 3x3x3 convolutions of the warm-start network on tcgen05 tensor cores
-// (conv_tc.cu): the shapes they take (channels 16 / 32 / 64; input grid D x
-// H x W any at stride 1, at stride 2 with even dimensions and H / 2 % 16,
-// W / 2 % 8 == 0), the forward convolution, the
-// flipped-transposed weights that turn a stride-1 input gradient into a
+// (conv_tc.cu): the shapes they are given (channels 16 / 32 / 64; input grid D x
+// H x W with H >= 16 at stride 1, at stride 2 with even dimensions and H / 2 %
+// 16, W / 2 % 8 == 0), the forward convolution, the flipped-transposed weights that turn a stride-1 input gradient into a
 // forward convolution, and the flag of a bounded wait that gave up (read
 // and cleared).
 bool conv3_tc_applies(int D, int H, int W, int ci, int co, int stride);
 cudaError_t conv3_tc(const void* x, int D, int H, int W, int ci, const void* w, const float* bias, int co, int relu,
                      void* y, float* y32, int stride, cudaStream_t st);
 cudaError_t conv3_flip_transpose(const void* w, void* wt, int co, int ci, cudaStream_t st);
-// Input gradient of a 3x3x3 stride-2 convolution (input grid D x H x W, any)
-// on tcgen05; wt: the weights as [ci][27][co].
+// Input gradient of a 3x3x3 stride-2 convolution (input grid D x H x W, of
+// more than 8 output voxels a plane) on tcgen05; wt: the weights as [ci][27][co].
 bool conv3_dx2_applies(int D, int H, int W, int ci, int co);
 cudaError_t conv3_dx2(const void* dy, const void* wt, void* dx, int D, int H, int W, int ci, int co, cudaStream_t st);
 // Weight gradient dw += dL/dw of a 3x3x3 (stride 1 or 2) or 1x1x1
-// convolution from staged tiles (conv_tc.cu), any grid.
+// convolution from staged tiles (conv_tc.cu), any grid but of a few voxels.
 bool conv_wgrad_tiles_applies(int D, int H, int W, int ci, int co, int ks, int stride);
 cudaError_t conv_wgrad_tiles(const void* x, int D, int H, int W, int ci, const void* dy, int co, int ks, int stride,
                              float* dw, cudaStream_t st);

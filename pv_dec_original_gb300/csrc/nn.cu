@@ -516,8 +516,9 @@ __global__ void k_add(const bf16* __restrict__ a, const bf16* __restrict__ b, bf
 // Bound by the additions to the one loss word, one a warp (1.5 ns each):
 // a warp whose values are all zero (outside the mask, 60% of the voxels of a
 // vessel's box) adds nothing, 3.14 -> 1.23 ms at 4.2M voxels.  (Partial sums
-// per block would take 75 us, but end further than 2e-5 from the loss that
-// this chain of 0.8M FP32 additions gives.)
+// per block would take 75 us and come nearer the exact sum, which this chain of
+// 0.8M FP32 additions misses by 1e-5 to 3e-5; they would also change every loss
+// value that a run reports.)
 __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ target,
                       const uint8_t* __restrict__ mask, int64_t nvox, int c, int nc, float inv_norm,
                       bf16* __restrict__ dpred, float* __restrict__ loss) {

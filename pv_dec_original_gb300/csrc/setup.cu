@@ -13,8 +13,9 @@
 // here a node is one class byte in a dense box and the boundary/next-to-wall
 // nodes form one compact, index-sorted list built by a scan.
 //
-// Compiled with --fmad=false: the normals keep the reference's rounding
-// (pow(d, 2) is evaluated as d*d).
+// Compiled with --fmad=false: a triangle's normal, area and centroid are rounded
+// as the reference rounds them.  The sums over the triangles are not: they use
+// fused multiply-adds, one reciprocal for four distances and parts (k_normals).
 #include <algorithm>
 
 #include "lbm_internal.cuh"

@@ -1950,9 +1950,9 @@ cudaError_t launch_compact(const StepParams& p, cudaStream_t st) {
 //   428.7, BF16 alike), in FP32 the compact (128,12) (3.2M, 6.2M and 12M within 0.2%
 //   of (128,10); 12M in narrow tubes 335.6, (128,10) 346.4, the flat (128,12) 344);
 //   beside other lattices' steps (P.crowded) the SMs are full whatever a lattice's
-//   size, and warps count: 11.8M nodes in 16 lattices FP32 (128,12) 330.6, (128,10)
-//   351.7, (128,8) 393.4, the flat (128,12) 336; FP16 286.4, 300.6, 333.1, 288; 1.3M in
-//   8, FP32 37.1, 39.1, 43.7, 38.0; D3Q27 5.9M in 32 FP32 253.2, 236.2, 249.0, 262.7.
+//   size, and warps count: 11.8M nodes in 16 lattices FP32 (128,12) 325.6, (128,10)
+//   347.9, (128,8) 390.9, the flat (128,12) 334.9; FP16 284.4, 296.1, 328.0, 286.4; 1.3M
+//   in 8, FP32 36.6, 39.0, 43.3, 37.9; D3Q27 5.9M in 32 FP32 247.9, 231.7, 243.9, 261.5.
 // The flat (128,12) that every such handle started on: 4.41 us at 20k nodes,
 // 8.29 at 250k (compact (128,8) 6.6), D3Q27 13.6 (8.3), FP32 1.4M 40.8 (35.5).
 constexpr int64_t kLatencyNodes = 12000, kMemoryBytes = 32000000, kLargeBytes = 300000000;

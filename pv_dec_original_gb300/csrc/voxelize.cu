@@ -11,14 +11,14 @@
 //   parity -> Fluid        ComplexGeometry.cpp:1041-1048
 //
 // GB300 design: the reference tests every point against every triangle
-// (O(N*T)).  Here a triangle meets only the lattice columns its xy extent,
-// widened by a per-triangle margin, contains: a triangle outside that
-// widened extent provably fails the point-in-triangle test for every point
-// of the column (the margin is ~1e8 times the worst-case rounding of that
-// test), so dropping it changes no count.  Triangles that can never pass
-// (zero area, or a computed normal with |n_z| < 1e-16, which the reference
-// rejects outright) are dropped; ill-conditioned ones go to a global list
-// tested by every point.
+// (O(N*T)).  Here a triangle meets only the lattice columns within its xy extent
+// widened by 4 L E (tri_extent): L its longest edge at vertex 1, E a bound of
+// the rounding of the reference's barycentric coordinates (barycentric_bound),
+// beyond which the point-in-triangle test fails for every point of the column,
+// so that leaving the triangle out changes no count.  Triangles that can never
+// pass (zero area, a computed normal with |n_z| < 1e-16 or a file normal whose z
+// the plane test rejects) have no columns; those too ill-conditioned for any
+// bound (cull_margin) go to a global list tested by every point.
 // All points of a column share the ray's x and y, so a (column, triangle)
 // pair is decided once for the whole column: whether the line lies inside
 // the triangle does not depend on k but for rounding, and the crossing
@@ -115,7 +115,10 @@ __device__ __forceinline__ int ray_hits(const Ray& r, const double* __restrict__
     return 0;
 }
 
-// Conservative xy margin (see file comment); -1 never counts, 1e30 never cull.
+// A margin of the xy extent about 1e8 times the rounding of the point-in-triangle
+// test; -1: the triangle never counts, 1e30: no margin holds it.  It sorts the
+// triangles, bounds the columns where tri_extent's own bound is larger, and gives
+// the number of candidate tests that a call reports.
 __device__ double cull_margin(const double* T, double zspan) {
     double uX = T[3] - T[0], uY = T[4] - T[1], uZ = T[5] - T[2];
     double vX = T[6] - T[0], vY = T[7] - T[1], vZ = T[8] - T[2];

@@ -166,7 +166,7 @@ class GroupedEnsemble:
     One packed lattice advances step by step: every launch waits for the
     whole previous step, so each step ends in a drain where the last blocks
     run alone.  Independent lattices on their own streams fill each other's
-    drains (64 seeded stenosed tubes, FP16: 4 or 8 groups ran 1.04-1.05x
+    drains (64 seeded stenosed tubes, FP16: 4 or 8 groups ran 1.02-1.05x
     one packed lattice).  Advancing the groups one after another instead, so
     that a group's populations could stay in L2 across its steps, gained
     nothing (groups of 2 to 16 members: 0.91-1.01x one packed lattice).
