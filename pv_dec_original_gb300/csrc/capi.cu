@@ -377,8 +377,8 @@ cudaError_t launch(lbm_handle* h, int kind, const StepParams& p) {
     h->launches++;
     // lbm_autotune's choice is the fastest of a lattice that steps alone (11.8M nodes
     // FP32 in 16 lattices, each tuned: 374 us a step of all with it, 325 without)
-    const bool alone = h->tuned && h->crowded && h->d.mode == LBM_PHYSICS;
-    const int v = alone ? -1 : h->variant;
+    const bool untuned = h->tuned && h->crowded && h->d.mode == LBM_PHYSICS;
+    const int v = untuned ? -1 : h->variant;
     switch (h->d.precision) {
         case LBM_F64: return launch_step_f64(h->d.Q, h->d.mode, kind, h->variant, p, h->st);
         case LBM_F32: return launch_step_f32(h->d.Q, h->d.mode, kind, v, p, h->st);
@@ -1136,12 +1136,10 @@ lbm_status lbm_step_async(lbm_handle* h, int nsteps) {
     REQUIRE(h, h->has_state, LBM_ERR_STATE, "no state: set the geometry first");
     REQUIRE(h, nsteps >= 0, LBM_ERR_ARG, "negative step count");
     CK(h, cudaSetDevice(h->d.device));
-    if (nsteps > 0) {
-        h->wss_from_ckpt = false;
-        steps_issued(h);
-    }
+    if (nsteps > 0) h->wss_from_ckpt = false;
     REQUIRE(h, h->persist == 0 || persist_ok(h), LBM_ERR_UNSUPPORTED,
             "persistent steps need 32-bit population offsets (Q * stride < 2^31)");
+    if (nsteps > 0) steps_issued(h);
     int left = nsteps;
     // Graph replay: a captured graph bakes the buffer roles (cur) and the
     // counter slot (step parity); both flip every step, so a graph built at
